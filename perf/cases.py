@@ -225,18 +225,16 @@ def prepare(case: dict, seed: int) -> dict:
     read = case.get("read", "ldr")
     s["buffer"] = _pinned(h, w, 4, dtype=torch.uint8 if read == "ldr" else torch.float32)
     if kind == "animate":
-        # eight poses of the moved spheres (instances 7.. of the seeded scene), column-major object to world
+        # eight poses of the moved spheres (instances 7.. of the seeded scene, column-major object to world): each
+        # circles its built place by about its own radius, as an animation moves an object between frames
         g = np.random.default_rng(seed)
         n = case["moved"]
         s["ids"] = np.arange(7, 7 + n, dtype=np.uint32)
-        t = np.zeros((8, n, 16), np.float32)
-        radius = g.uniform(0.05, 0.15, (1, n))
-        for k in (0, 5, 10):
-            t[:, :, k] = 2.0 * radius
-        t[:, :, 12] = g.uniform(-0.85, 0.85, (8, n))
-        t[:, :, 13] = -1.0 + radius + g.uniform(0.0, 1.2, (8, n))
-        t[:, :, 14] = g.uniform(-0.85, 0.85, (8, n))
-        t[:, :, 15] = 1.0
+        a = b.arrays()
+        t = np.array([list(a.instances[int(i)].transform) for i in s["ids"]], np.float32)[None].repeat(8, axis=0)
+        angle = 2.0 * math.pi * (np.arange(8)[:, None] / 8.0 + g.uniform(0.0, 1.0, (1, n)))
+        t[:, :, 12] += 0.5 * t[:, :, 0] * np.cos(angle)
+        t[:, :, 14] += 0.5 * t[:, :, 0] * np.sin(angle)
         s["poses"] = t
     return s
 
@@ -283,6 +281,8 @@ def run(s: dict):
         return image
     if kind == "rays":
         hits = s["scene"].trace(s["rays"], any_hit=case["any_hit"])
+        if case["any_hit"]:
+            return {"prim": hits["prim"]}  # occluded or not: which of the hits was found first is not defined
         return {"t": hits["t"], "prim": hits["prim"], "u": hits["u"], "v": hits["v"]}
     status = srt.lib().srt_photon_grid_build_noalloc(
         C.c_void_p(torch.cuda.current_stream().cuda_stream), C.c_void_p(s["photons"].data_ptr()), case["photons"],
