@@ -681,6 +681,33 @@ __global__ void k_refit8(Node8* __restrict__ nodes, const TriSlot* __restrict__ 
     nodes[i] = nd;
 }
 
+// Scatter masks of one level's nodes, from the deeper level's masks or the leaf triangles' materials.
+__global__ void k_scatter_mask(const Node8* __restrict__ nodes, const TriSlot* __restrict__ tris,
+                               const uint32_t* __restrict__ tri_inst, const InstDev* __restrict__ inst,
+                               const float4* __restrict__ materials, uint32_t begin, uint32_t end,
+                               uint8_t* __restrict__ mask) {
+    const uint32_t i = begin + blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= end) return;
+    const uint32_t imask = nodes[i].a.w >> 24;
+    const uint4 b = nodes[i].b;
+    uint32_t out = 0u;
+    for (uint32_t s = 0; s < 8u; ++s) {
+        const uint32_t m = ((s < 4u ? b.z : b.w) >> (8u * (s & 3u))) & 0xFFu;
+        if (m == 0u) continue;
+        bool any = false;
+        if ((imask >> s) & 1u) {
+            any = mask[b.x + __popc(imask & ((1u << s) - 1u))] != 0u;
+        } else {
+            for (uint32_t k = 0; k < (m >> 5); ++k) {
+                const uint32_t tri = __float_as_uint(tris[b.y + (m & 31u) + k].v0.w);
+                any = any || scatters_photons(materials[2 * inst[tri_inst[tri]].mat_id + 1]);
+            }
+        }
+        if (any) out |= 1u << s;
+    }
+    mask[i] = (uint8_t)out;
+}
+
 // Leaf slots of moved instances, re-transformed from object space.
 __global__ void k_update_slots(TriSlot* __restrict__ tris, uint32_t n_tris, const uint32_t* __restrict__ tri_inst,
                                const uint8_t* __restrict__ moved, const float4* __restrict__ vtx,
@@ -1059,6 +1086,19 @@ int launch_expand_lights(const LightInst* li, uint32_t n_li, const uint8_t* move
     if (n_li == 0) return 0;
     k_expand_lights<<<n_li, 128, 0, st>>>(li, moved, vtx, indices, mesh_infos, inst, fwd, lights);
     return 1;
+}
+
+int launch_scatter_masks(const BvhOutputs& bvh, const InstDev* inst, const float4* materials, uint8_t* mask,
+                         cudaStream_t st) {
+    int n = 0;
+    for (int L = (int)bvh.depth - 1; L >= 0; --L) {
+        const uint32_t b = bvh.level_start[L], e = bvh.level_start[L + 1];
+        if (e <= b) continue;
+        k_scatter_mask<<<(e - b + 127) / 128, 128, 0, st>>>(bvh.nodes, bvh.tris, bvh.tri_inst, inst, materials, b, e,
+                                                            mask);
+        ++n;
+    }
+    return n;
 }
 
 int refit_bvh8(Node8* nodes, const TriSlot* tris, const BvhOutputs& lv, float4* aux, uint32_t* err,

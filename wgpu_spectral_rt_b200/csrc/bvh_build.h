@@ -59,6 +59,12 @@ struct BvhOutputs {
 // owned by the caller afterwards (cudaFree).
 cudaError_t build_bvh8(const BvhInputs& in, cudaStream_t st, BvhOutputs* out, std::string* msg);
 
+// Per node, the child slots whose subtree holds a triangle of a material that
+// scatters photons (scatters_photons): mask[n_nodes], level by level from the
+// deepest.  Depends on the topology and the materials only, so a refit keeps it.
+int launch_scatter_masks(const BvhOutputs& bvh, const InstDev* inst, const float4* materials, uint8_t* mask,
+                         cudaStream_t st);
+
 // Scene updates (moved instances), all on `st`:
 // re-transform the leaf slots of instances with moved[inst] != 0,
 int launch_update_slots(TriSlot* tris, uint32_t n_tris, const uint32_t* tri_inst, const uint8_t* moved,

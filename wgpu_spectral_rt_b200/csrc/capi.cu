@@ -313,6 +313,7 @@ struct srt_scene {
     InstDev* inst = nullptr;
     InstFwd* fwd = nullptr;
     BvhOutputs bvh{};
+    uint8_t* scatter = nullptr;  // scatter masks of bvh's nodes (launch_scatter_masks)
     DevScene dev{};
     uint64_t n_tris = 0;
     uint32_t n_lights = 0;
@@ -350,6 +351,7 @@ struct srt_scene {
         cudaFree(bvh.nodes);
         cudaFree(bvh.tris);
         cudaFree(bvh.tri_inst);
+        cudaFree(scatter);
     }
 };
 
@@ -458,6 +460,9 @@ srt_status scene_build_impl(srt_ctx* c, const srt_scene_arrays* a,
     if (e != cudaSuccess) return fail(c, e == cudaErrorMemoryAllocation ? SRT_ERR_OOM : SRT_ERR_CUDA, "BVH build: " + msg);
     if (s->bvh.depth > (uint32_t)TRAV_STACK)
         return fail(c, SRT_ERR_UNSUPPORTED, "BVH deeper than the traversal stack");
+    CUDA_TRY(c, dev_alloc(&s->scatter, s->bvh.n_nodes));
+    launch_scatter_masks(s->bvh, s->inst, s->materials, s->scatter, st);
+    CUDA_TRY(c, cudaGetLastError());
     CUDA_TRY(c, cudaStreamSynchronize(st));
     s->n_tris = total;
     s->n_lights = a->n_lights;
@@ -472,6 +477,7 @@ srt_status scene_build_impl(srt_ctx* c, const srt_scene_arrays* a,
     d.tri_inst = s->bvh.tri_inst;
     d.nodes = s->bvh.nodes;
     d.tris = s->bvh.tris;
+    d.scatter = s->scatter;
     d.n_nodes = s->bvh.n_nodes;
     d.n_tris = (uint32_t)total;
     d.depth = s->bvh.depth;
@@ -652,16 +658,26 @@ extern "C" srt_status srt_scene_rebuild_bvh(srt_scene* s, uint32_t width) {
         e = cudaErrorInvalidValue;
         msg = "BVH deeper than the traversal stack";
     }
+    uint8_t* scatter = nullptr;
+    if (e == cudaSuccess) e = dev_alloc(&scatter, nb.n_nodes);
+    if (e == cudaSuccess) {
+        launch_scatter_masks(nb, s->inst, s->materials, scatter, st);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         cudaFree(nb.nodes);
         cudaFree(nb.tris);
         cudaFree(nb.tri_inst);
+        cudaFree(scatter);
         return fail(c, e == cudaErrorMemoryAllocation ? SRT_ERR_OOM : SRT_ERR_CUDA, "BVH rebuild: " + msg);
     }
     cudaFree(s->bvh.nodes);
     cudaFree(s->bvh.tris);
     cudaFree(s->bvh.tri_inst);
+    cudaFree(s->scatter);
     s->bvh = nb;
+    s->scatter = scatter;
     // refit scratch is sized by the node count: allocated again on the next update
     cudaFree(s->moved);
     cudaFree(s->refit_aux);
@@ -674,6 +690,7 @@ extern "C" srt_status srt_scene_rebuild_bvh(srt_scene* s, uint32_t width) {
     d.tri_inst = s->bvh.tri_inst;
     d.nodes = s->bvh.nodes;
     d.tris = s->bvh.tris;
+    d.scatter = s->scatter;
     d.n_nodes = s->bvh.n_nodes;
     d.depth = s->bvh.depth;
     s->gen += 1;

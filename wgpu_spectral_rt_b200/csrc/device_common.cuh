@@ -67,6 +67,7 @@ struct DevScene {
     const uint32_t* tri_inst;   // flattened triangle -> instance
     const Node8* nodes;
     const TriSlot* tris;
+    const uint8_t* scatter;     // per node: child slots whose subtree holds a scattering triangle (k_scatter_mask)
     uint32_t n_nodes;
     uint32_t n_tris;
     uint32_t depth;  // 8-wide levels: a traversal stack needs at least this many entries
@@ -492,14 +493,6 @@ SRT_DEV float2 fma2(float2 a, float2 b, float2 c) {
 #endif
 }
 
-// Child bookkeeping of a node visit in one pass after the slab tests
-// (SRT_TRAV_LEAN, the default: a hit mask from the child loop, then the octant
-// order of the internal children and the leaves' triangle bits once per node)
-// instead of per child (config-2 closest-hit 3.35 vs 3.43 ms per frame).
-#ifndef SRT_TRAV_LEAN
-#define SRT_TRAV_LEAN 1
-#endif
-
 struct TravCounters {
     unsigned long long* nodes;
     unsigned long long* tris;
@@ -523,13 +516,12 @@ SRT_DEV void fetch_node_async(const DevScene& S, uint32_t idx, uint4* nbuf, int 
 }
 
 // Child slab tests of one node (words w0..w4) for a ray with inverse
-// direction idir and octant oct: the node's hit internal children (bits
-// 24..31, ordered by octant) | imask, and its hit triangle bits.
-SRT_DEV void node_children(uint4 w0, uint4 w1, uint4 w2, uint4 w3, uint4 w4, float3 o, float3 idir, uint32_t oct,
-                           float tmin, float tbest, uint2& g, uint2& tg) {
+// direction idir and octant oct: the slots whose box the ray meets within
+// [tmin, tbest].
+SRT_DEV uint32_t node_hits(uint4 w0, uint4 w1, uint4 w2, uint4 w3, uint4 w4, float3 o, float3 idir, uint32_t oct,
+                           float tmin, float tbest) {
     float sx = __uint_as_float((w0.w & 0xFFu) << 23), sy = __uint_as_float(((w0.w >> 8) & 0xFFu) << 23),
           sz = __uint_as_float(((w0.w >> 16) & 0xFFu) << 23);
-    uint32_t imask = w0.w >> 24;
     float ax = sx * idir.x, ay = sy * idir.y, az = sz * idir.z;
     float bx = unbias(ax, (__uint_as_float(w0.x) - o.x) * idir.x), by = unbias(ay, (__uint_as_float(w0.y) - o.y) * idir.y),
           bz = unbias(az, (__uint_as_float(w0.z) - o.z) * idir.z);
@@ -540,9 +532,6 @@ SRT_DEV void node_children(uint4 w0, uint4 w1, uint4 w2, uint4 w3, uint4 w4, flo
     uint32_t nz0 = (oct & 4u) ? w4.z : w3.x, nz1 = (oct & 4u) ? w4.w : w3.y;
     uint32_t fz0 = (oct & 4u) ? w3.x : w4.z, fz1 = (oct & 4u) ? w3.y : w4.w;
     const float robust = 1.0000004f;
-#if SRT_TRAV_LEAN
-    // the child loop only collects which slots are hit; the octant order of
-    // the internal children and the leaves' triangle bits follow once per node
     uint32_t hitmask = 0u;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -558,6 +547,18 @@ SRT_DEV void node_children(uint4 w0, uint4 w1, uint4 w2, uint4 w3, uint4 w4, flo
         const float tf = fminf(fminf(tx.y, ty.y), fminf(tz.y, tbest)) * robust;
         hitmask |= (m != 0u && tn <= tf) ? (1u << i) : 0u;
     }
+    return hitmask;
+}
+
+// One node visit: the node's hit internal children (bits 24..31, ordered by
+// octant) | imask, and its hit triangle bits.  The child loop (node_hits) only
+// collects which slots are hit; the octant order of the internal children and
+// the leaves' triangle bits follow once per node (config-2 closest-hit 3.35
+// vs 3.43 ms per frame with both per child).
+SRT_DEV void node_children(uint4 w0, uint4 w1, uint4 w2, uint4 w3, uint4 w4, float3 o, float3 idir, uint32_t oct,
+                           float tmin, float tbest, uint2& g, uint2& tg) {
+    const uint32_t imask = w0.w >> 24;
+    const uint32_t hitmask = node_hits(w0, w1, w2, w3, w4, o, idir, oct, tmin, tbest);
     // internal children: slot i -> bit i ^ (oct ^ 7) (three conditional swaps)
     uint32_t ib = hitmask & imask;
     const uint32_t x = oct ^ 7u;
@@ -574,29 +575,62 @@ SRT_DEV void node_children(uint4 w0, uint4 w1, uint4 w2, uint4 w3, uint4 w4, flo
     }
     g = make_uint2(w1.x, (ib << 24) | imask);
     tg = make_uint2(w1.y, tris);
-#else
-    uint32_t hits = 0u;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const uint32_t k = (uint32_t)(i & 3);
-        uint32_t m = byte_of(i < 4 ? w1.z : w1.w, k);
-        const float2 tx = fma2(make_float2(qbyte(i < 4 ? nx0 : nx1, k), qbyte(i < 4 ? fx0 : fx1, k)),
-                               make_float2(ax, ax), make_float2(bx, bx));
-        const float2 ty = fma2(make_float2(qbyte(i < 4 ? ny0 : ny1, k), qbyte(i < 4 ? fy0 : fy1, k)),
-                               make_float2(ay, ay), make_float2(by, by));
-        const float2 tz = fma2(make_float2(qbyte(i < 4 ? nz0 : nz1, k), qbyte(i < 4 ? fz0 : fz1, k)),
-                               make_float2(az, az), make_float2(bz, bz));
-        float tn = fmaxf(fmaxf(tx.x, ty.x), fmaxf(tz.x, tmin));
-        float tf = fminf(fminf(tx.y, ty.y), fminf(tz.y, tbest)) * robust;
-        if (m != 0u && tn <= tf) {
-            uint32_t c = m >> 5;
-            if (c == 7u) hits |= 1u << (24 + ((uint32_t)i ^ (oct ^ 7u)));
-            else hits |= ((1u << c) - 1u) << (m & 31u);
+}
+
+// Materials a photon path goes on from: types 1, 2, 4 and 5.  At any other
+// surface a path ends, and its first surface stores nothing either (only
+// diffuse surfaces reached after a refraction or a film store photons).
+SRT_DEV bool scatters_photons(float4 extra) {
+    const uint32_t type = (uint32_t)extra.x;
+    return type == 1u || type == 2u || type == 4u || type == 5u;
+}
+
+// Whether the ray meets the box of a leaf that holds a scattering triangle
+// (S.scatter), on a walk of such subtrees only.  Conservative: the closest-hit
+// traversal reaches a triangle through boxes that pass the same slab test with
+// a t_max no larger than `tmax`, so a ray refused here has no scattering
+// triangle as its closest hit.  `stack`: STACK entries of this thread, stride
+// `stride` (one entry per level at most).
+template <int STACK>
+SRT_DEV bool may_scatter(const DevScene& S, float3 o, float3 d, float tmin, float tmax, uint2* stack, int stride,
+                         uint32_t* err) {
+    if (S.n_nodes == 0u || !(d.x != 0.0f || d.y != 0.0f || d.z != 0.0f)) return false;
+    const float eps = 1e-12f;
+    const float3 idir = f3(1.0f / (fabsf(d.x) > eps ? d.x : copysignf(eps, d.x)),
+                           1.0f / (fabsf(d.y) > eps ? d.y : copysignf(eps, d.y)),
+                           1.0f / (fabsf(d.z) > eps ? d.z : copysignf(eps, d.z)));
+    const uint32_t oct = (d.x < 0.f ? 1u : 0u) | (d.y < 0.f ? 2u : 0u) | (d.z < 0.f ? 4u : 0u);
+    uint2 g = make_uint2(0u, 0x101u);  // child base; child slots left (bits 8..15) | imask; the root as slot 0
+    int sp = 0;
+    while (true) {
+        if ((g.y & 0xFF00u) == 0u) {
+            if (sp == 0) return false;
+            --sp;
+            g = stack[sp * stride];
         }
+        const uint32_t slot = (uint32_t)__ffs(g.y >> 8) - 1u;
+        g.y &= ~(0x100u << slot);
+        const uint32_t idx = g.x + __popc(g.y & ((1u << slot) - 1u) & 0xFFu);
+        if (g.y & 0xFF00u) {
+            if (sp >= STACK) {
+                atomicOr(err, ERR_STACK_OVERFLOW);
+                return false;
+            }
+            stack[sp * stride] = g;
+            ++sp;
+        }
+        if (idx >= S.n_nodes) {
+            atomicOr(err, ERR_BAD_INDEX);
+            return false;
+        }
+        const uint32_t scatter = __ldg(S.scatter + idx);
+        const uint4* np = reinterpret_cast<const uint4*>(S.nodes + idx);
+        const uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
+        const uint32_t hits = node_hits(w0, w1, w2, w3, w4, o, idir, oct, tmin, tmax) & scatter;
+        const uint32_t imask = w0.w >> 24;
+        if (hits & ~imask) return true;
+        g = make_uint2(w1.x, (hits << 8) | imask);
     }
-    g = make_uint2(w1.x, (hits & 0xFF000000u) | imask);
-    tg = make_uint2(w1.y, hits & 0x00FFFFFFu);
-#endif
 }
 
 // Stack-based traversal of the compressed BVH8.  A node group holds the

@@ -1,14 +1,16 @@
 // render_kernels.cu — per-frame kernels of the spectral path tracer.
 //
 // One frame = one sample per pixel (src/renderer/mod.rs:168-207):
-//   photon pass   photon_emit.wgsl:154-331 as a wavefront (emit, direction
-//                 sort, per bounce trace + shade, emitter-ordered compaction
+//   photon pass   photon_emit.wgsl:154-331 as a wavefront (emit and
+//                 cull, per bounce trace + shade, emitter-ordered compaction
 //                 of the stored photons) and the grid (build_grid.wgsl:25-73)
 //                 as cell keys + radix sort + ranges
 //   camera paths  shader.wgsl:708-823 as a wavefront: raygen, then per
 //                 bounce trace_closest -> shade -> trace_shadow over SoA
 //                 queues compacted with warp ballots; finalize converts the
 //                 hero tuple to sRGB, accumulates and tonemaps.
+#include <algorithm>
+
 #include "radix_sort.cuh"
 #include "render_kernels.h"
 
@@ -77,15 +79,13 @@ SRT_DEV float4 gather(const GatherArgs& g, uint32_t frame, float3 hit_pos, float
 // flagged; an emitter-ordered compaction afterwards reproduces the order a
 // sequential run of the reference's atomicAdd gives.
 //
-// SRT_PHOTON_DIR_SORT sorts the emitted rays by an octahedral direction key
-// first, so that a warp traces rays of similar direction.  It paid while
-// photon rays were traced one per thread; with the persistent warps (refill,
-// warp-synchronous node visits) it no longer does: config-2 photon pass 2.25
-// ms unsorted vs 2.45 ms sorted on 24 bits (2.36 on 16, 2.29 on 8), the same
-// photons.
-#ifndef SRT_PHOTON_DIR_SORT
-#define SRT_PHOTON_DIR_SORT 0
-#endif
+// Emission culls first: a photon path whose first surface does not scatter
+// (diffuse, emitter) ends there without storing anything, so an emitted ray
+// that meets no leaf box with a scattering triangle (may_scatter: a walk of
+// the scene's tree restricted to those subtrees) needs no closest hit, and
+// none of its state is written.  Config 2 (4.2M emitted, 31k scatter): photon pass 2.12 -> 1.59 ms alone (closest hits of bounce 0
+// 1.42 -> 0.50 ms, emission 0.09 -> 0.66 ms), frame 8.87 -> 8.35 ms; eight
+// seeded scenes in a batch 17.1 -> 15.6 ms for two iterations.
 
 // Octahedral 12+12-bit direction code, Morton-interleaved (24 bits).
 SRT_DEV uint32_t dir_key(float3 d) {
@@ -122,131 +122,140 @@ SRT_DEV uint32_t ray_sort_key(float3 o, float3 d, float4 bmin, float4 binv) {
 
 constexpr uint32_t PH_CAUSTIC = 0x1u;
 
-// Emission: photon_emit.wgsl:159-214.
-__global__ void k_photon_emit(FrameArgs a) {
-    uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= a.photons_per_frame) return;
+// Emission (photon_emit.wgsl:159-214), one thread per emitter id: the light
+// point and direction, the cull, and for the rays that may scatter the
+// wavelength, energy and state; they are queued for bounce 0 (any order: a
+// path's results go to its emitter's slot).
+template <int STACK>
+__global__ void __launch_bounds__(TRACE_BLOCK, SRT_SHADE_MIN_BLOCKS) k_photon_emit(FrameArgs a) {
+    extern __shared__ uint2 stack_smem[];
+    const uint32_t e = blockIdx.x * TRACE_BLOCK + threadIdx.x;
     const DevScene& S = a.scene;
-    uint32_t frame = a.cam->frame_count;
-    uint32_t s = pcg_hash(e + frame * 927163u + a.seed);
-    uint32_t nl = S.n_lights;  // > 0: the pass is skipped without lights
-    uint32_t li = min(__float2uint_rz(rng_next(s) * (float)nl), nl - 1u);
-    float4 L0 = S.lights[4 * li], L1 = S.lights[4 * li + 1], L2 = S.lights[4 * li + 2], LP = S.lights[4 * li + 3];
-    float3 v0 = xyz(L0), v1 = xyz(L1), v2 = xyz(L2);
-    float3 c = cross(v1 - v0, v2 - v0);
-    float3 normal = normalize(c);
-    float area = length(c) * 0.5f;
-    float r1 = rng_next(s);
-    float r2 = rng_next(s);
-    float sr1 = sqrtf(r1);
-    float u = 1.0f - sr1, v = r2 * sr1, w = 1.0f - u - v;
-    float3 emit_pos = v0 * u + v1 * v + v2 * w;
-    float3 emit_dir = normalize(normal + random_unit_vector(s));
-    float cmin = cauchy_cdf(LAMBDA_MIN), cmax = cauchy_cdf(LAMBDA_MAX), crange = cmax - cmin;
-    float lambda =
-        clampf(555.0f + 40.0f * tanf(PI * ((cmin + rng_next(s) * crange) - 0.5f)), LAMBDA_MIN, LAMBDA_MAX);
-    float dw = (lambda - 555.0f) / 40.0f;
-    float pdf = (1.0f / (crange * PI * 40.0f)) / (1.0f + dw * dw);
-    float energy = (blackbody(lambda, LP.y) / pdf) * area * PI * LP.z;
-    float3 pos = emit_pos + emit_dir * 0.001f;
-    a.ph.ray_o[e] = f4(pos.x, pos.y, pos.z, 0.0001f);
-    a.ph.ray_d[e] = f4(emit_dir.x, emit_dir.y, emit_dir.z, 100.0f);
-    a.ph.state[e] = f4(lambda, energy, __uint_as_float(s), __uint_as_float(0u));
-    a.ph.flags[e] = 0u;
-    if (SRT_PHOTON_DIR_SORT) {
-        a.ph.keys[e] = dir_key(emit_dir);
-        a.ph.vals[e] = e;
+    bool live = e < a.photons_per_frame;
+    if (live) {
+        uint32_t frame = a.cam->frame_count;
+        uint32_t s = pcg_hash(e + frame * 927163u + a.seed);
+        uint32_t nl = S.n_lights;  // > 0: the pass is skipped without lights
+        uint32_t li = min(__float2uint_rz(rng_next(s) * (float)nl), nl - 1u);
+        float4 L0 = S.lights[4 * li], L1 = S.lights[4 * li + 1], L2 = S.lights[4 * li + 2];
+        float3 v0 = xyz(L0), v1 = xyz(L1), v2 = xyz(L2);
+        float3 c = cross(v1 - v0, v2 - v0);
+        float3 normal = normalize(c);
+        float r1 = rng_next(s);
+        float r2 = rng_next(s);
+        float sr1 = sqrtf(r1);
+        float u = 1.0f - sr1, v = r2 * sr1, w = 1.0f - u - v;
+        float3 emit_pos = v0 * u + v1 * v + v2 * w;
+        float3 emit_dir = normalize(normal + random_unit_vector(s));
+        float3 pos = emit_pos + emit_dir * 0.001f;
+        live = may_scatter<STACK>(S, pos, emit_dir, 0.0001f, 100.0f, stack_smem + threadIdx.x, TRACE_BLOCK, a.err);
+        if (live) {
+            float4 LP = S.lights[4 * li + 3];
+            float area = length(c) * 0.5f;
+            float cmin = cauchy_cdf(LAMBDA_MIN), cmax = cauchy_cdf(LAMBDA_MAX), crange = cmax - cmin;
+            float lambda =
+                clampf(555.0f + 40.0f * tanf(PI * ((cmin + rng_next(s) * crange) - 0.5f)), LAMBDA_MIN, LAMBDA_MAX);
+            float dw = (lambda - 555.0f) / 40.0f;
+            float pdf = (1.0f / (crange * PI * 40.0f)) / (1.0f + dw * dw);
+            float energy = (blackbody(lambda, LP.y) / pdf) * area * PI * LP.z;
+            a.ph.ray_o[e] = f4(pos.x, pos.y, pos.z, 0.0001f);
+            a.ph.ray_d[e] = f4(emit_dir.x, emit_dir.y, emit_dir.z, 100.0f);
+            a.ph.state[e] = f4(lambda, energy, __uint_as_float(s), __uint_as_float(0u));
+        }
     }
-    if (e == 0) a.counters->photon_paths[0] = a.photons_per_frame;
+    const uint32_t slot = warp_push(live, &a.counters->photon_paths[0]);
+    if (live) a.ph.queue[0][slot] = e;
+    if (e == 0) a.counters->photons_emitted = a.photons_per_frame;
 }
 
 // One bounce of the photon loop after its closest-hit query
 // (photon_emit.wgsl:227-330).  Material type 5 (no reference counterpart)
 // reflects with the probability of the film's Airy reflectance, else absorbs.
 __global__ void __launch_bounds__(TRACE_BLOCK, SRT_SHADE_MIN_BLOCKS) k_photon_shade(FrameArgs a, uint32_t bounce) {
-    uint32_t n = a.counters->photon_paths[bounce];
-    if (blockIdx.x * blockDim.x >= n) return;
-    uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t n = a.counters->photon_paths[bounce];
     const DevScene& S = a.scene;
-    const uint32_t* qin = bounce == 0 ? a.ph.sorted_vals : a.ph.queue[bounce & 1];
-    bool alive = false;
-    uint32_t e = q < n ? (qin ? qin[q] : q) : 0u;
-    if (q < n) {
-        float4 h = a.ph.hit[e];
-        uint32_t prim = __float_as_uint(h.y);
-        if (prim != MISS) {
-            float4 o4 = a.ph.ray_o[e], d4 = a.ph.ray_d[e], st = a.ph.state[e];
-            float3 pos = xyz(o4), dir = xyz(d4);
-            float lambda = st.x, energy = st.y;
-            uint32_t s = __float_as_uint(st.z), fl = __float_as_uint(st.w);
-            Surface sf = surface_at(S, prim, h.z, h.w, dir);
-            float4 extra = S.materials[2 * sf.mat + 1];
-            float3 ffn = sf.front ? sf.wn : -sf.wn;
-            uint32_t type = (uint32_t)extra.x;
-            float3 hp = pos + dir * h.x;
-            bool caustic = (fl & PH_CAUSTIC) != 0u;
-            if (type == 0u) {
-                if (caustic) {
-                    a.ph.staging[2 * e] = f4(hp.x, hp.y, hp.z, lambda);
-                    a.ph.staging[2 * e + 1] = f4(-dir.x, -dir.y, -dir.z, energy);
-                    a.ph.flags[e] = 1u;
-                }
-            } else if (type == 1u) {
-                dir = reflect(normalize(dir), ffn);
-                pos = hp + ffn * 0.001f;
-                alive = true;
-            } else if (type == 2u) {
-                float lum = lambda / 1000.0f;
-                float ir = extra.z + (extra.w / (lum * lum));
-                float ratio = sf.front ? 1.0f / ir : ir;
-                float3 ud = normalize(dir);
-                float ct = fminf(dot(-ud, ffn), 1.0f);
-                float stn = sqrtf(1.0f - ct * ct);
-                if (ratio * stn > 1.0f || schlick(ct, ratio) > rng_next(s)) {
-                    dir = reflect(ud, ffn);
-                } else {
-                    caustic = true;
-                    dir = refract(ud, ffn, ratio);
-                }
-                pos = hp + (dot(dir, ffn) > 0.0f ? ffn : -ffn) * 0.001f;
-                alive = true;
-            } else if (type == 4u) {
-                float3 ud = normalize(dir);
-                float ct = fminf(dot(-ud, ffn), 1.0f);
-                // select(n1 / n3, n3 / n1, is_front_face) with n1 = 1
-                float ratio = sf.front ? extra.w / 1.0f : 1.0f / extra.w;
-                float stt = ratio * ratio * (1.0f - ct * ct);
-                if (stt > 1.0f) {
-                    dir = reflect(ud, ffn);
-                } else {
+    const uint32_t* qin = a.ph.queue[bounce & 1];
+    for (uint32_t base = blockIdx.x * TRACE_BLOCK; base < n; base += gridDim.x * TRACE_BLOCK) {
+        const uint32_t q = base + threadIdx.x;
+        bool alive = false;
+        uint32_t e = q < n ? qin[q] : 0u;
+        if (q < n) {
+            float4 h = a.ph.hit[e];
+            uint32_t prim = __float_as_uint(h.y);
+            if (prim != MISS) {
+                float4 o4 = a.ph.ray_o[e], d4 = a.ph.ray_d[e], st = a.ph.state[e];
+                float3 pos = xyz(o4), dir = xyz(d4);
+                float lambda = st.x, energy = st.y;
+                uint32_t s = __float_as_uint(st.z), fl = __float_as_uint(st.w);
+                Surface sf = surface_at(S, prim, h.z, h.w, dir);
+                float4 extra = S.materials[2 * sf.mat + 1];
+                float3 ffn = sf.front ? sf.wn : -sf.wn;
+                uint32_t type = (uint32_t)extra.x;
+                float3 hp = pos + dir * h.x;
+                bool caustic = (fl & PH_CAUSTIC) != 0u;
+                if (type == 0u) {
+                    if (caustic) {
+                        a.ph.staging[2 * e] = f4(hp.x, hp.y, hp.z, lambda);
+                        a.ph.staging[2 * e + 1] = f4(-dir.x, -dir.y, -dir.z, energy);
+                        a.ph.flags[e] = 1u;
+                    }
+                } else if (type == 1u) {
+                    dir = reflect(normalize(dir), ffn);
+                    pos = hp + ffn * 0.001f;
+                    alive = true;
+                } else if (type == 2u) {
+                    float lum = lambda / 1000.0f;
+                    float ir = extra.z + (extra.w / (lum * lum));
+                    float ratio = sf.front ? 1.0f / ir : ir;
+                    float3 ud = normalize(dir);
+                    float ct = fminf(dot(-ud, ffn), 1.0f);
+                    float stn = sqrtf(1.0f - ct * ct);
+                    if (ratio * stn > 1.0f || schlick(ct, ratio) > rng_next(s)) {
+                        dir = reflect(ud, ffn);
+                    } else {
+                        caustic = true;
+                        dir = refract(ud, ffn, ratio);
+                    }
+                    pos = hp + (dot(dir, ffn) > 0.0f ? ffn : -ffn) * 0.001f;
+                    alive = true;
+                } else if (type == 4u) {
+                    float3 ud = normalize(dir);
+                    float ct = fminf(dot(-ud, ffn), 1.0f);
+                    // select(n1 / n3, n3 / n1, is_front_face) with n1 = 1
+                    float ratio = sf.front ? extra.w / 1.0f : 1.0f / extra.w;
+                    float stt = ratio * ratio * (1.0f - ct * ct);
+                    if (stt > 1.0f) {
+                        dir = reflect(ud, ffn);
+                    } else {
+                        bool tir;
+                        float F = thin_film1(ct, 1.0f, extra.z, extra.w, fmaxf(extra.y, 50.0f), lambda, tir);
+                        dir = rng_next(s) < F ? reflect(ud, ffn) : refract(ud, ffn, ratio);
+                    }
+                    caustic = true;  // the position is not advanced (photon_emit.wgsl:291-326)
+                    alive = true;
+                } else if (type == 5u) {
+                    float3 ud = normalize(dir);
+                    float ct = fminf(dot(-ud, ffn), 1.0f);
                     bool tir;
                     float F = thin_film1(ct, 1.0f, extra.z, extra.w, fmaxf(extra.y, 50.0f), lambda, tir);
-                    dir = rng_next(s) < F ? reflect(ud, ffn) : refract(ud, ffn, ratio);
+                    if (rng_next(s) < F) {
+                        dir = reflect(ud, ffn);
+                        pos = hp + ffn * 0.001f;
+                        caustic = true;
+                        alive = true;
+                    }
                 }
-                caustic = true;  // the position is not advanced (photon_emit.wgsl:291-326)
-                alive = true;
-            } else if (type == 5u) {
-                float3 ud = normalize(dir);
-                float ct = fminf(dot(-ud, ffn), 1.0f);
-                bool tir;
-                float F = thin_film1(ct, 1.0f, extra.z, extra.w, fmaxf(extra.y, 50.0f), lambda, tir);
-                if (rng_next(s) < F) {
-                    dir = reflect(ud, ffn);
-                    pos = hp + ffn * 0.001f;
-                    caustic = true;
-                    alive = true;
+                if (bounce + 1u >= a.photon_max_bounces) alive = false;
+                if (alive) {
+                    a.ph.ray_o[e] = f4(pos.x, pos.y, pos.z, 0.0001f);
+                    a.ph.ray_d[e] = f4(dir.x, dir.y, dir.z, 100.0f);
+                    a.ph.state[e] = f4(lambda, energy, __uint_as_float(s), __uint_as_float(caustic ? PH_CAUSTIC : 0u));
                 }
-            }
-            if (bounce + 1u >= a.photon_max_bounces) alive = false;
-            if (alive) {
-                a.ph.ray_o[e] = f4(pos.x, pos.y, pos.z, 0.0001f);
-                a.ph.ray_d[e] = f4(dir.x, dir.y, dir.z, 100.0f);
-                a.ph.state[e] = f4(lambda, energy, __uint_as_float(s), __uint_as_float(caustic ? PH_CAUSTIC : 0u));
             }
         }
+        uint32_t slot = warp_push(alive, &a.counters->photon_paths[bounce + 1]);
+        if (alive) a.ph.queue[(bounce + 1) & 1][slot] = e;
     }
-    uint32_t slot = warp_push(alive, &a.counters->photon_paths[bounce + 1]);
-    if (alive) a.ph.queue[(bounce + 1) & 1][slot] = e;
 }
 
 // Emitter-ordered compaction of the stored photons: per-block counts, an
@@ -703,8 +712,10 @@ __global__ void k_frame_stats(FrameArgs a) {
     unsigned long long pr = 0;
     if (a.photons_per_frame > 0u)
         for (uint32_t i = 0; i < a.photon_max_bounces; ++i) {
-            pr += a.ph_counters->photon_paths[i];
-            a.stats->rays_bounce[TRAV_PHOTON][i] += a.ph_counters->photon_paths[i];
+            // bounce 0: every emitted ray, also those the cull answered
+            const uint32_t k = i == 0u ? a.ph_counters->photons_emitted : a.ph_counters->photon_paths[i];
+            pr += k;
+            a.stats->rays_bounce[TRAV_PHOTON][i] += k;
         }
     a.stats->photon_rays += pr;
 }
@@ -808,21 +819,18 @@ inline uint32_t blocks_for(uint64_t n, uint32_t b) { return (uint32_t)((n + b - 
 int launch_photon_pass(FrameArgs& a, cudaStream_t st) {
     int launches = 0;
     const uint32_t n = a.photons_per_frame;
-    // emit (with SRT_PHOTON_DIR_SORT, then order the emitted rays by direction)
-    k_photon_emit<<<blocks_for(n, 256), 256, 0, st>>>(a);
+    cudaMemsetAsync(a.ph.flags, 0, n, st);
+    const uint32_t blocks = blocks_for(n, TRACE_BLOCK);
+    if (a.scene.depth <= (uint32_t)TRAV_STACK_SMALL)
+        k_photon_emit<TRAV_STACK_SMALL><<<blocks, TRACE_BLOCK, sizeof(uint2) * TRAV_STACK_SMALL * TRACE_BLOCK, st>>>(a);
+    else k_photon_emit<TRAV_STACK><<<blocks, TRACE_BLOCK, sizeof(uint2) * TRAV_STACK * TRACE_BLOCK, st>>>(a);
     ++launches;
-    uint32_t* order = nullptr;  // bounce-0 queue: emitter order
-    if (SRT_PHOTON_DIR_SORT) {
-        uint32_t* dir_keys;
-        launches += sort_pairs(a.ph.keys, a.ph.vals, a.ph.keys2, a.ph.vals2, n, nullptr, 0, 24, a.ph.sort_scratch,
-                               st, &dir_keys, &order);
-    }
-    a.ph.sorted_vals = order;  // bounce-0 queue (read by k_photon_shade at bounce 0)
+    const uint32_t shade_grid = std::min(blocks, (uint32_t)(a.sm_count > 0 ? a.sm_count : 148) * SRT_SHADE_MIN_BLOCKS);
     for (uint32_t b = 0; b < a.photon_max_bounces; ++b) {
-        launches += launch_trace_queue(a.scene, b, b == 0 ? order : a.ph.queue[b & 1], &a.counters->photon_paths[b],
+        launches += launch_trace_queue(a.scene, b, a.ph.queue[b & 1], &a.counters->photon_paths[b],
                                        &a.counters->fetch[TRAV_PHOTON][b], n, a.ph.ray_o, a.ph.ray_d, a.ph.hit,
                                        TRAV_PHOTON, a.count_visits, a.err, a.stats, a.sm_count, st);
-        k_photon_shade<<<blocks_for(n, TRACE_BLOCK), TRACE_BLOCK, 0, st>>>(a, b);
+        k_photon_shade<<<shade_grid, TRACE_BLOCK, 0, st>>>(a, b);
         ++launches;
     }
     // stored photons in emitter order

@@ -20,7 +20,8 @@ struct FrameCounters {
     uint32_t photon_paths[MAX_PHOTON_BOUNCES + 1];  // live photon paths entering bounce i
     uint32_t fetch[3][MAX_BOUNCES + 1];  // persistent traversal: next queue position, by TRAV_* kind and bounce
     uint32_t photons_stored;
-    uint32_t pad[2];
+    uint32_t photons_emitted;  // emitted by this photon pass (photon_paths[0] holds those that may scatter)
+    uint32_t pad;
 };
 
 // Device statistics accumulated over frames (64-bit).
@@ -54,7 +55,7 @@ struct PhotonBuffers {
     float4* state;          // per emitter: wavelength, energy, rng (bits), flags (bits)
     float4* hit;            // per emitter: closest hit (t, triangle, u, v)
     uint8_t* flags;         // per emitter: 1 if a photon was stored
-    uint32_t* queue[2];     // live emitter ids after bounce 0
+    uint32_t* queue[2];     // live emitter ids, by bounce parity
     float4* staging;        // per emitter: the stored photon, 2 float4
     uint32_t* block_counts; // per block of PHOTON_BLOCK emitters; scanned in place into offsets
     float4* photons;        // emission order, 2 per photon

@@ -438,9 +438,7 @@ int launch_trace_queue(const DevScene& s, uint32_t bounce, const uint32_t* queue
                        uint32_t* fetch, uint32_t max_n, const float4* ro, const float4* rd, float4* hit, int kind,
                        int count_visits, uint32_t* err, DevStats* stats, int sm_count, cudaStream_t st) {
     if (max_n == 0) return 0;
-    // photon rays in emitter order (direction-sorted with
-    // SRT_PHOTON_DIR_SORT); persistent warps take them in that order
-    // (SRT_PHOTON_PERSISTENT)
+    // persistent warps (SRT_PHOTON_PERSISTENT)
     TraceLaunch L{s, queue, count, SRT_PHOTON_PERSISTENT ? fetch : nullptr, max_n, ro, rd, hit, nullptr, nullptr,
                   nullptr, err, stats, kind, sm_count, (int)bounce};
     launch_kind<false>(L, count_visits, st);
