@@ -411,7 +411,7 @@ srt_status srt_renderer_get_bounce_stats(srt_renderer* r, srt_bounce_stats* out)
  * SRT_TAIL_AUTO (the default): the renderer reads back the path counts of
  * its first frame without waiting for them and, once they are there, starts
  * the tail at the first bounce >= 1 whose live paths fit in one wave of the
- * tail kernel's resident threads (a batch: the scenes' paths summed), for a
+ * tail kernel, eight threads per path (a batch: the scenes' paths summed), for a
  * guiding renderer not before the end of its guided bounces; frames before
  * that run bounce by bounce.  0 = bounce by bounce.  Not used with
  * SRT_FLAG_RAY_SORT, nor where a set number of guided bounces reaches it

@@ -706,13 +706,15 @@ extern "C" srt_status srt_scene_bvh_width(const srt_scene* s, uint32_t* width) {
 
 // ====================================================================== renderer
 // The tail kernel (launch_tail) follows each remaining path through its
-// last bounces in one launch, one thread per path at a time: it pays once
-// the live paths fit in about one wave of it, and costs where many long paths
-// remain (1080p: config 2 from bounce 5, 118k paths, 10.76 vs 11.04 ms per
-// frame; the caustic-slab scene from bounce 5, 202k paths, 7.05 vs 5.93 ms,
-// from bounce 7, 69k paths, 5.92 ms).  SRT_TAIL_AUTO (the default) starts it
-// at the first bounce whose live paths in the renderer's first frame number
-// at most SRT_TAIL_WAVES waves of the tail kernel's resident threads.
+// last bounces in one launch, eight lanes per path: it pays once the live
+// paths fit in about one wave of it (9,472 paths), where the bounce-by-bounce
+// launches cost their latency, and costs where more remain.  Frames by first
+// tail bounce (paths entering it): config 2 at 1080p none 8.02, 5 (59k) 8.37,
+// 7 (15k) 7.96, 8 (7.7k) 7.96 ms; Cornell 640x480 none 2.33, 7 (17k) 2.40, 8
+// (10k) 2.31; config 1 none 0.92, 4 (40k) 0.99, 5 (7.5k) 0.86; the caustic slab
+// at 1080p none 5.11, 9 (24k) 5.25; prism 96x64 none 0.42, 1 (5.8k) 0.28.  SRT_TAIL_AUTO
+// (the default) starts it at the first bounce whose live paths in the
+// renderer's first frame number at most SRT_TAIL_WAVES waves of it.
 #ifndef SRT_TAIL_WAVES
 #define SRT_TAIL_WAVES 1.0
 #endif
@@ -967,7 +969,7 @@ struct srt_renderer {
         if (tail_first != SRT_TAIL_AUTO || counts_state != 1) return;
         if (cudaEventQuery(counts_ev) != cudaSuccess) return;
         counts_state = 2;
-        const uint32_t t = choose_tail(counts_host, p.max_depth, (double)tail_threads(args));
+        const uint32_t t = choose_tail(counts_host, p.max_depth, (double)tail_paths(args));
         if (t != tail_auto) {
             tail_auto = t;
             drop_graph();
@@ -2550,7 +2552,7 @@ struct srt_batch {
             for (int b = 0; b <= MAX_BOUNCES; ++b) sum[b] += r[i]->counts_host[b];
         }
         if (first < 0) return;
-        const uint32_t t = srt_renderer::choose_tail(sum.data(), depth, (double)tail_threads(r[first]->args));
+        const uint32_t t = srt_renderer::choose_tail(sum.data(), depth, (double)tail_paths(r[first]->args));
         for (srt_renderer* x : r) {
             if (x->tail_first != SRT_TAIL_AUTO || x->tail_auto == t) continue;
             x->tail_auto = t;

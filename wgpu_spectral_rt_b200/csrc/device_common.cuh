@@ -1126,6 +1126,211 @@ SRT_DEV bool trav_step(const DevScene& S, TravState& T, uint2* stack, int stride
     return false;
 }
 
+// ------------------------------------------------------------------ one ray on eight lanes
+// The same traversal with a ray on a group of 8 lanes (4 rays per warp): lane
+// c of the group tests child c of a node and the triangles of that child's
+// leaf, so a node visit is one slab test deep instead of eight and a node's
+// leaves are tested at once.  Per ray it issues about as many warp
+// instructions as the one-lane form at its usual occupancy of lanes, but the
+// chain of a single ray is several times shorter, and rays of a warp do not
+// diverge (the groups step together).  It serves the launches that last as
+// long as their longest rays: few rays (k_trace_pt) and the tail.
+// Every function here is called by all 32 lanes of a warp at once.
+constexpr uint32_t GROUP = 8;
+constexpr uint32_t GROUP_LEADERS = 0x01010101u;  // lane 0 of each group
+
+template <int STACK>
+struct GroupTrav {
+    float3 o, idir;
+    float tmin, tbest;  // tbest: the group's closest t so far
+    float sx, sy, sz;
+    uint32_t axes;      // kx | ky << 2 | kz << 4 | oct << 8
+    uint2 g;
+    uint2 st[STACK / 8];  // the group's stack: entry e in slot e / 8 of lane e % 8
+    int sp;
+    float t, u, v;      // this lane's closest hit
+    uint32_t id;        // MISS: none
+};
+
+// Returns false when the ray cannot hit anything.  The same values in all
+// lanes of a group.
+template <int STACK>
+SRT_DEV bool group_init(GroupTrav<STACK>& T, const DevScene& S, float3 o, float3 d, float tmin, float tmax) {
+    T.id = MISS;
+    T.t = __int_as_float(0x7F800000);
+    T.u = T.v = 0.f;
+    T.tbest = tmax;
+    T.tmin = tmin;
+    T.sp = 0;
+    T.o = o;
+    T.g = make_uint2(0u, 0u);
+    if (S.n_nodes == 0u || !(d.x != 0.0f || d.y != 0.0f || d.z != 0.0f) || !(tmin <= tmax)) return false;
+    const RayShear sh = make_shear(d);
+    T.sx = sh.sx;
+    T.sy = sh.sy;
+    T.sz = sh.sz;
+    const float eps = 1e-12f;
+    T.idir = f3(1.0f / (fabsf(d.x) > eps ? d.x : copysignf(eps, d.x)),
+                1.0f / (fabsf(d.y) > eps ? d.y : copysignf(eps, d.y)),
+                1.0f / (fabsf(d.z) > eps ? d.z : copysignf(eps, d.z)));
+    const uint32_t oct = (d.x < 0.f ? 1u : 0u) | (d.y < 0.f ? 2u : 0u) | (d.z < 0.f ? 4u : 0u);
+    T.axes = (uint32_t)sh.kx | ((uint32_t)sh.ky << 2) | ((uint32_t)sh.kz << 4) | (oct << 8);
+    T.g = make_uint2(0u, (1u << (24 + (0u ^ (oct ^ 7u)))) | 1u);
+    return true;
+}
+
+// One node visit and its triangles for the groups with `active` set; true
+// when the group's ray is finished (ANY: at its first hit).
+template <bool ANY, int STACK>
+SRT_DEV bool group_step(const DevScene& S, GroupTrav<STACK>& T, bool active, uint32_t* err, uint32_t& n_nodes,
+                        uint32_t& n_tris) {
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u, c = lane & 7u, shift = lane & 24u;
+    const uint32_t oct = (T.axes >> 8) & 7u;
+    bool fin = false;
+    const bool empty = active && (T.g.y & 0xFF000000u) == 0u;
+    if (__any_sync(FULL, empty)) {
+        const int top = T.sp - 1;
+        uint2 e = T.st[0];
+#pragma unroll
+        for (int k = 1; k < STACK / 8; ++k)
+            if ((top >> 3) == k) e = T.st[k];
+        const uint32_t px = __shfl_sync(FULL, e.x, (int)(shift | ((uint32_t)top & 7u)));
+        const uint32_t py = __shfl_sync(FULL, e.y, (int)(shift | ((uint32_t)top & 7u)));
+        if (empty) {
+            if (top < 0) fin = true;
+            else {
+                T.g = make_uint2(px, py);
+                T.sp = top;
+            }
+        }
+    }
+    bool go = active && !fin;
+    bool hit = false;
+    uint32_t cnt = 0u, first = 0u, imask = 0u, child = 0u;
+    if (go) {
+        const int bit = 31 - __clz(T.g.y & 0xFF000000u);
+        T.g.y &= ~(1u << bit);
+        const uint32_t slot = (uint32_t)(bit - 24) ^ (oct ^ 7u);
+        const uint32_t idx = T.g.x + __popc(T.g.y & ((1u << slot) - 1u) & 0xFFu);
+        if (T.g.y & 0xFF000000u) {
+            if (T.sp >= STACK) {
+                atomicOr(err, ERR_STACK_OVERFLOW);
+                go = false;
+            } else {
+#pragma unroll
+                for (int k = 0; k < STACK / 8; ++k)
+                    if (T.sp == (int)(8u * k + c)) T.st[k] = T.g;
+                ++T.sp;
+            }
+        }
+        if (go && idx >= S.n_nodes) {
+            atomicOr(err, ERR_BAD_INDEX);
+            go = false;
+        }
+        if (go) {
+            // header by every lane (one broadcast), child c's bytes by lane c
+            const uint8_t* nb = reinterpret_cast<const uint8_t*>(S.nodes + idx);
+            const uint4 w0 = __ldg(reinterpret_cast<const uint4*>(nb));
+            const uint2 w1 = __ldg(reinterpret_cast<const uint2*>(nb + 16));
+            const uint32_t m = __ldg(nb + 24 + c);
+            const uint32_t lx = __ldg(nb + 32 + c), ly = __ldg(nb + 40 + c), lz = __ldg(nb + 48 + c);
+            const uint32_t hx = __ldg(nb + 56 + c), hy = __ldg(nb + 64 + c), hz = __ldg(nb + 72 + c);
+            if (c == 0u) ++n_nodes;
+            const float ax = __uint_as_float((w0.w & 0xFFu) << 23) * T.idir.x,
+                        ay = __uint_as_float(((w0.w >> 8) & 0xFFu) << 23) * T.idir.y,
+                        az = __uint_as_float(((w0.w >> 16) & 0xFFu) << 23) * T.idir.z;
+            const float bx = unbias(ax, (__uint_as_float(w0.x) - T.o.x) * T.idir.x),
+                        by = unbias(ay, (__uint_as_float(w0.y) - T.o.y) * T.idir.y),
+                        bz = unbias(az, (__uint_as_float(w0.z) - T.o.z) * T.idir.z);
+            // the slab test of node_hits for one child: 2^23 + byte as a float
+            const uint32_t B = 0x4B000000u;
+            const float nx = fmaf(__uint_as_float(B | ((oct & 1u) ? hx : lx)), ax, bx),
+                        fx = fmaf(__uint_as_float(B | ((oct & 1u) ? lx : hx)), ax, bx),
+                        ny = fmaf(__uint_as_float(B | ((oct & 2u) ? hy : ly)), ay, by),
+                        fy = fmaf(__uint_as_float(B | ((oct & 2u) ? ly : hy)), ay, by),
+                        nz = fmaf(__uint_as_float(B | ((oct & 4u) ? hz : lz)), az, bz),
+                        fz = fmaf(__uint_as_float(B | ((oct & 4u) ? lz : hz)), az, bz);
+            const float tn = fmaxf(fmaxf(nx, ny), fmaxf(nz, T.tmin));
+            const float tf = fminf(fminf(fx, fy), fminf(fz, T.tbest)) * 1.0000004f;
+            hit = m != 0u && tn <= tf;
+            imask = w0.w >> 24;
+            child = w1.x;
+            if (hit && !((imask >> c) & 1u)) {
+                cnt = m >> 5;
+                first = w1.y + (m & 31u);
+            }
+        } else {
+            fin = true;
+        }
+    }
+    uint32_t ib = ((__ballot_sync(FULL, hit) >> shift) & 0xFFu) & imask;
+    if (go) {
+        const uint32_t x = oct ^ 7u;
+        ib = (x & 1u) ? (((ib & 0x55u) << 1) | ((ib >> 1) & 0x55u)) : ib;
+        ib = (x & 2u) ? (((ib & 0x33u) << 2) | ((ib >> 2) & 0x33u)) : ib;
+        ib = (x & 4u) ? (((ib & 0x0Fu) << 4) | ((ib >> 4) & 0x0Fu)) : ib;
+        T.g = make_uint2(child, (ib << 24) | imask);
+    }
+    if (!__any_sync(FULL, cnt != 0u)) return fin;
+    // the hit leaves' triangles, each lane its own leaf's
+    for (uint32_t k = 0; __any_sync(FULL, k < cnt); ++k) {
+        if (k < cnt) {
+            const TriSlot* ts = S.tris + first + k;
+            const float4 a0 = __ldg(&ts->v0), a1 = __ldg(&ts->v1), a2 = __ldg(&ts->v2);
+            ++n_tris;
+            float t, u, v;
+            if (tri_test(xyz(a0), xyz(a1), xyz(a2), T.o, T.axes & 3u, (T.axes >> 2) & 3u, (T.axes >> 4) & 3u, T.sx, T.sy,
+                         T.sz, T.tmin, T.tbest, t, u, v)) {
+                const uint32_t id = __float_as_uint(a0.w);
+                if (t < T.t || (t == T.t && id < T.id)) {
+                    T.t = t;
+                    T.id = id;
+                    T.u = u;
+                    T.v = v;
+                }
+            }
+        }
+    }
+    if (ANY) {
+        if ((__ballot_sync(FULL, active && T.id != MISS) >> shift) & 0xFFu) fin = true;
+    } else {
+        float t = fminf(T.t, T.tbest);
+        t = fminf(t, __shfl_xor_sync(FULL, t, 1));
+        t = fminf(t, __shfl_xor_sync(FULL, t, 2));
+        t = fminf(t, __shfl_xor_sync(FULL, t, 4));
+        if (active) T.tbest = t;
+    }
+    return fin;
+}
+
+// The closest hit of each group's finished ray, in all its lanes: the
+// lexicographic minimum of (t, id) over the lanes; prim MISS without a hit.
+template <int STACK>
+SRT_DEV void group_closest(const GroupTrav<STACK>& T, float& t, uint32_t& prim, float& u, float& v) {
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    t = T.t;
+    prim = T.id;
+    uint32_t own = threadIdx.x & 31u;
+#pragma unroll
+    for (uint32_t d = 1; d < GROUP; d <<= 1) {
+        const float ot = __shfl_xor_sync(FULL, t, d);
+        const uint32_t oi = __shfl_xor_sync(FULL, prim, d), oo = __shfl_xor_sync(FULL, own, d);
+        if (ot < t || (ot == t && oi < prim)) {
+            t = ot;
+            prim = oi;
+            own = oo;
+        }
+    }
+    u = __shfl_sync(FULL, T.u, (int)own);
+    v = __shfl_sync(FULL, T.v, (int)own);
+}
+// Whether an any-hit ray's group found a hit.
+template <int STACK>
+SRT_DEV bool group_occluded(const GroupTrav<STACK>& T) {
+    return ((__ballot_sync(0xFFFFFFFFu, T.id != MISS) >> (threadIdx.x & 24u)) & 0xFFu) != 0u;
+}
+
 // ------------------------------------------------------------------ surface data at a hit
 struct Surface {
     uint32_t inst, mat;

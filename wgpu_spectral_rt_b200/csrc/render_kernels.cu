@@ -592,50 +592,105 @@ __global__ void __launch_bounds__(TRACE_BLOCK, SRT_SHADE_MIN_BLOCKS)
 #define SRT_TAIL_MIN_BLOCKS 4
 #endif
 
-// The last bounces of the live paths in one persistent launch: each thread
-// takes a path entering bounce `first` and follows it to its end (closest
-// hit, shade_vertex, its shadow ray), then takes the next path.  Per path
-// the operations and the order of its radiance updates are those of the
-// bounce-by-bounce wavefront (the traversal rounds alike in every kernel), so
-// the image is bit-identical; where few paths remain, one launch replaces a
-// chain of launches that each last as long as their slowest ray.
+// The last bounces of the live paths in one persistent launch: a group of
+// eight lanes takes a path entering bounce `first` and follows it to its end
+// (closest hit on the group's lanes, shade_vertex on its first, its shadow ray
+// on all again), then takes the next path.  Per path the operations and the
+// order of its radiance updates are those of the bounce-by-bounce wavefront
+// (a ray is answered alike by every kernel), so the image is bit-identical;
+// where few paths remain, one launch replaces a chain of launches that each
+// last as long as their slowest ray.  What bounds it is the chain of one path
+// (closest hit, shading, shadow ray, next bounce): with a thread per path and
+// lanes of a warp at different stages it took 0.89 ms on config 2 (bounces 5-11
+// of 59k paths) and 0.73 ms on config 1 (bounces 1-7 of 65k); the lanes of a
+// group share a ray's node visits and the groups of a warp keep in step, and
+// with the launches before it (trace_groups) config 2 8.35 -> 8.17 ms per frame,
+// config 1 15.6 -> 14.6 ms per 16 frames, prism 96x64 0.445 -> 0.330 ms.
 template <bool GUIDE, bool COUNT, int STACK>
 __global__ void __launch_bounds__(TRACE_BLOCK, SRT_TAIL_MIN_BLOCKS) k_tail(FrameArgs a, uint32_t first) {
-    extern __shared__ uint2 stack_smem[];
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
     __shared__ uint32_t n_closest[MAX_BOUNCES + 1], n_shadow[MAX_BOUNCES + 1];
     for (uint32_t i = threadIdx.x; i <= (uint32_t)MAX_BOUNCES; i += blockDim.x) n_closest[i] = n_shadow[i] = 0u;
     __syncthreads();
-    uint2* stack = stack_smem + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u, c = lane & 7u, shift = lane & 24u;
     const uint32_t n = a.counters->paths[first];
     uint32_t* fetch = &a.counters->fetch[TRAV_CLOSEST][first];
     const uint32_t* queue = a.pb.queue[first & 1];
+    GroupTrav<STACK> T;
+    T.sp = 0;
+    T.axes = 0u;
+    bool live = false, exhausted = false;
+    uint32_t id = 0u, b = first;
     while (true) {
-        const uint32_t q = atomicAdd(fetch, 1u);
-        if (q >= n) break;
-        const uint32_t id = queue[q];
-        for (uint32_t b = first; b < a.max_depth; ++b) {
-            if (b > first) atomicAdd(&n_closest[b], 1u);  // paths[first] was counted by the last shading step
+        const uint32_t idle = __ballot_sync(FULL, !live) & GROUP_LEADERS;
+        if (!exhausted && idle) {
+            uint32_t base = 0u;
+            if (lane == 0u) base = atomicAdd(fetch, (uint32_t)__popc(idle));
+            base = __shfl_sync(FULL, base, 0);
+            if (base + (uint32_t)__popc(idle) >= n) exhausted = true;
+            const uint32_t q = base + __popc(idle & ((1u << shift) - 1u));
+            if (!live && q < n) {
+                id = queue[q];
+                b = first;
+                live = true;
+            }
+        }
+        if (__ballot_sync(FULL, live) == 0u) break;  // exhausted: a fetch that gave no path was past the end
+        // closest hits
+        uint32_t nodes = 0u, tris = 0u;
+        T.id = MISS;
+        bool act = false;
+        if (live) {
+            if (b > first && c == 0u) atomicAdd(&n_closest[b], 1u);  // paths[first] was counted by the last shading step
             const float4 o = a.pb.ray_o[id], d = a.pb.ray_d[id];
-            float t = 0.f, u = 0.f, v = 0.f;
-            uint32_t prim;
-            TravCounters tc{&a.stats->nodes_bounce[TRAV_CLOSEST][b], &a.stats->tris_bounce[TRAV_CLOSEST][b]};
-            const bool h = traverse<false, COUNT, STACK>(a.scene, Ray{xyz(o), xyz(d), o.w, d.w}, stack, TRACE_BLOCK, t,
-                                                         prim, u, v, a.err, tc);
-            a.pb.hit[id] = h ? make_float4(t, __uint_as_float(prim), u, v) : make_float4(0.f, __uint_as_float(MISS), 0.f, 0.f);
-            const VertexOut vo = shade_vertex<GUIDE>(a, id, b);
-            if (vo.shadow) {
+            act = group_init(T, a.scene, xyz(o), xyz(d), o.w, d.w);
+        }
+        while (__any_sync(FULL, act))
+            if (group_step<false>(a.scene, T, act, a.err, nodes, tris)) act = false;
+        float t, u, v;
+        uint32_t prim;
+        group_closest(T, t, prim, u, v);
+        if (COUNT && live) {
+            atomicAdd(&a.stats->nodes_bounce[TRAV_CLOSEST][b], (unsigned long long)nodes);
+            atomicAdd(&a.stats->tris_bounce[TRAV_CLOSEST][b], (unsigned long long)tris);
+        }
+        // shading
+        VertexOut vo;
+        if (live && c == 0u) {
+            a.pb.hit[id] = prim != MISS ? make_float4(t, __uint_as_float(prim), u, v)
+                                        : make_float4(0.f, __uint_as_float(MISS), 0.f, 0.f);
+            vo = shade_vertex<GUIDE>(a, id, b);
+        }
+        __syncwarp();  // the path's next ray, written by the group's first lane, is read by all
+        const uint32_t alive = __ballot_sync(FULL, vo.alive), shadow = __ballot_sync(FULL, vo.shadow);
+        if (shadow) {
+            const float3 so = f3(__shfl_sync(FULL, vo.sh_o.x, (int)shift), __shfl_sync(FULL, vo.sh_o.y, (int)shift),
+                                 __shfl_sync(FULL, vo.sh_o.z, (int)shift));
+            const float3 sd = f3(__shfl_sync(FULL, vo.sh_d.x, (int)shift), __shfl_sync(FULL, vo.sh_d.y, (int)shift),
+                                 __shfl_sync(FULL, vo.sh_d.z, (int)shift));
+            const float smax = __shfl_sync(FULL, vo.sh_tmax, (int)shift);
+            const bool has = ((shadow >> shift) & 1u) != 0u;
+            nodes = tris = 0u;
+            T.id = MISS;
+            act = has && group_init(T, a.scene, so, sd, 0.001f, smax);
+            while (__any_sync(FULL, act))
+                if (group_step<true>(a.scene, T, act, a.err, nodes, tris)) act = false;
+            const bool occluded = group_occluded(T);
+            if (has && c == 0u) {
                 atomicAdd(&n_shadow[b], 1u);
-                TravCounters ts{&a.stats->nodes_bounce[TRAV_SHADOW][b], &a.stats->tris_bounce[TRAV_SHADOW][b]};
-                const bool occluded = traverse<true, COUNT, STACK>(a.scene, Ray{vo.sh_o, vo.sh_d, 0.001f, vo.sh_tmax},
-                                                                   stack, TRACE_BLOCK, t, prim, u, v, a.err, ts);
                 if (!occluded) {  // as the shadow-ray kernel adds it (shader.wgsl:659-669)
-                    const float4 r = a.pb.rad[id], c = vo.sh_c;
-                    a.pb.rad[id] = make_float4(__fadd_rn(r.x, c.x), __fadd_rn(r.y, c.y), __fadd_rn(r.z, c.z),
-                                               __fadd_rn(r.w, c.w));
+                    const float4 r = a.pb.rad[id], k = vo.sh_c;
+                    a.pb.rad[id] = make_float4(__fadd_rn(r.x, k.x), __fadd_rn(r.y, k.y), __fadd_rn(r.z, k.z),
+                                               __fadd_rn(r.w, k.w));
                 }
             }
-            if (!vo.alive) break;
+            if (COUNT && has) {
+                atomicAdd(&a.stats->nodes_bounce[TRAV_SHADOW][b], (unsigned long long)nodes);
+                atomicAdd(&a.stats->tris_bounce[TRAV_SHADOW][b], (unsigned long long)tris);
+            }
         }
+        live = live && ((alive >> shift) & 1u) != 0u;
+        ++b;
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i <= (uint32_t)MAX_BOUNCES; i += blockDim.x) {
@@ -650,8 +705,8 @@ int tail_per_sm() {
     static int per_sm = 0;
     if (per_sm == 0) {
         int x = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&x, k_tail<GUIDE, COUNT, STACK>, TRACE_BLOCK,
-                                                          sizeof(uint2) * STACK * TRACE_BLOCK) != cudaSuccess ||
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&x, k_tail<GUIDE, COUNT, STACK>, TRACE_BLOCK, 0) !=
+                cudaSuccess ||
             x < 1)
             x = 1;
         per_sm = x;
@@ -661,9 +716,8 @@ int tail_per_sm() {
 
 template <bool GUIDE, bool COUNT, int STACK>
 int launch_tail_t(const FrameArgs& a, uint32_t first, cudaStream_t st) {
-    const size_t smem = sizeof(uint2) * STACK * TRACE_BLOCK;
     const uint32_t grid = (uint32_t)(a.sm_count > 0 ? a.sm_count : 148) * (uint32_t)tail_per_sm<GUIDE, COUNT, STACK>();
-    k_tail<GUIDE, COUNT, STACK><<<grid, TRACE_BLOCK, smem, st>>>(a, first);
+    k_tail<GUIDE, COUNT, STACK><<<grid, TRACE_BLOCK, 0, st>>>(a, first);
     return 1;
 }
 
@@ -911,7 +965,7 @@ int launch_frame_stats(const FrameArgs& a, cudaStream_t st) {
     return 1;
 }
 
-uint32_t tail_threads(const FrameArgs& a) {
+uint32_t tail_paths(const FrameArgs& a) {
     const bool small = a.scene.depth <= (uint32_t)TRAV_STACK_SMALL;
     const bool g = a.guiding != 0, c = a.count_visits != 0;
     int per_sm;
@@ -919,7 +973,7 @@ uint32_t tail_threads(const FrameArgs& a) {
                       : (small ? tail_per_sm<false, true, TRAV_STACK_SMALL>() : tail_per_sm<false, true, TRAV_STACK>());
     else per_sm = g ? (small ? tail_per_sm<true, false, TRAV_STACK_SMALL>() : tail_per_sm<true, false, TRAV_STACK>())
                     : (small ? tail_per_sm<false, false, TRAV_STACK_SMALL>() : tail_per_sm<false, false, TRAV_STACK>());
-    return (uint32_t)(a.sm_count > 0 ? a.sm_count : 148) * (uint32_t)per_sm * TRACE_BLOCK;
+    return (uint32_t)(a.sm_count > 0 ? a.sm_count : 148) * (uint32_t)per_sm * (TRACE_BLOCK / GROUP);
 }
 
 int launch_tail(const FrameArgs& a, uint32_t first, cudaStream_t st) {

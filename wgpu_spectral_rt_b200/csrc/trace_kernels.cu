@@ -45,6 +45,18 @@
 #ifndef SRT_TRACE_REFILL_ANY
 #define SRT_TRACE_REFILL_ANY 12
 #endif
+// k_trace_pt traces a ray on eight lanes (trace_groups) when the launch has at
+// most this many rays per group of its resident warps (2: 42,624 rays).  Such a
+// launch lasts as long as its longest rays: one ray per lane took 53 us for 44
+// photon rays and 0.13-0.16 ms for 1k-59k camera rays of config 2.  Frames
+// without the tail kernel, at 0 / 1 / 2 / 4 / 8 / 16 rays per group: prism
+// 96x64 0.606 / 0.411 / 0.416 / 0.415 / 0.417 / 0.415 ms, Cornell 640x480 2.569
+// / 2.322 / 2.293 / 2.327 / 2.596 / 3.123, a seeded scene of 812k triangles at
+// 512x384 2.890 / 2.361 / 2.312 / 2.415 / 2.647 / 2.808, config 1 1.072 / 0.945
+// / 0.929 / 0.917 / 0.912 / 0.915.
+#ifndef SRT_TRACE_GROUP_WAVES
+#define SRT_TRACE_GROUP_WAVES 2
+#endif
 #ifndef SRT_TRACE_PERSISTENT
 #define SRT_TRACE_PERSISTENT 1
 #endif
@@ -124,17 +136,83 @@ __global__ void __launch_bounds__(TRACE_BLOCK, SRT_TRACE_MIN_BLOCKS)
     }
 }
 
+// Few rays: a ray on eight lanes (group_step), the groups of a warp stepping
+// together and taking the next rays from *fetch as they finish.
+template <bool ANY, bool COUNT, int STACK>
+SRT_DEV void trace_groups(const DevScene& S, const uint32_t* queue, uint32_t n, uint32_t* fetch, const float4* ro,
+                          const float4* rd, float4* hit, const uint32_t* sh_id, const float4* sh_c, float4* rad,
+                          uint32_t* err, DevStats* stats, int kind, int bounce) {
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u, c = lane & 7u, shift = lane & 24u;
+    GroupTrav<STACK> T;
+    T.sp = 0;
+    T.axes = 0u;
+    T.id = MISS;
+    bool active = false, exhausted = false;
+    uint32_t q = 0, id = 0, n_nodes = 0, n_tris = 0;
+    while (true) {
+        const uint32_t idle = __ballot_sync(FULL, !active) & GROUP_LEADERS;
+        bool fin = false;
+        if (!exhausted && idle) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(fetch, (uint32_t)__popc(idle));
+            base = __shfl_sync(FULL, base, 0);
+            if (base + (uint32_t)__popc(idle) >= n) exhausted = true;
+            const uint32_t my = base + __popc(idle & ((1u << shift) - 1u));
+            if (!active && my < n) {
+                q = my;
+                id = queue ? queue[q] : q;
+                const float4 o = ro[ANY ? q : id], d = rd[ANY ? q : id];
+                active = true;
+                fin = !group_init(T, S, xyz(o), xyz(d), o.w, d.w);  // degenerate: finished without a hit
+            }
+        }
+        if (__ballot_sync(FULL, active) == 0u) {
+            if (exhausted) break;
+            continue;
+        }
+        fin = group_step<ANY>(S, T, active && !fin, err, n_nodes, n_tris) || fin;
+        if (__any_sync(FULL, fin)) {
+            if (ANY) {
+                const bool occluded = group_occluded(T);
+                if (fin && !occluded && c == 0u) {
+                    const uint32_t pid = sh_id[q];
+                    const float4 k = sh_c[q], r = rad[pid];
+                    rad[pid] = make_float4(__fadd_rn(r.x, k.x), __fadd_rn(r.y, k.y), __fadd_rn(r.z, k.z),
+                                           __fadd_rn(r.w, k.w));
+                }
+            } else {
+                float t, u, v;
+                uint32_t prim;
+                group_closest(T, t, prim, u, v);
+                if (fin && c == 0u)
+                    hit[id] = prim != MISS ? make_float4(t, __uint_as_float(prim), u, v)
+                                           : make_float4(0.f, __uint_as_float(MISS), 0.f, 0.f);
+            }
+            if (fin) active = false;
+        }
+    }
+    if (COUNT) {
+        atomicAdd(&stats->nodes_bounce[kind][bounce], (unsigned long long)n_nodes);
+        atomicAdd(&stats->tris_bounce[kind][bounce], (unsigned long long)n_tris);
+    }
+}
+
 // Persistent form: same inputs and outputs, queue positions from *fetch.
 template <bool ANY, bool COUNT, int STACK>
 __global__ void __launch_bounds__(TRACE_BLOCK, SRT_TRACE_PT_BLOCKS)
     k_trace_pt(DevScene S, const uint32_t* __restrict__ queue, const uint32_t* __restrict__ count,
                uint32_t* __restrict__ fetch, const float4* __restrict__ ro, const float4* __restrict__ rd,
                float4* __restrict__ hit, const uint32_t* __restrict__ sh_id, const float4* __restrict__ sh_c,
-               float4* __restrict__ rad, uint32_t* err, DevStats* stats, int kind, int bounce) {
+               float4* __restrict__ rad, uint32_t* err, DevStats* stats, int kind, int bounce, uint32_t group_max) {
     extern __shared__ uint2 stack_smem[];
     uint2* stack = stack_smem + threadIdx.x;
     const uint32_t n = *count;
     if (n == 0u) return;
+    if (n <= group_max) {
+        trace_groups<ANY, COUNT, STACK>(S, queue, n, fetch, ro, rd, hit, sh_id, sh_c, rad, err, stats, kind, bounce);
+        return;
+    }
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt = (1u << lane) - 1u;
     TravState T;
@@ -387,10 +465,11 @@ void launch_one(const TraceLaunch& L, cudaStream_t st) {
     size_t smem = trace_smem<STACK>();
     if (SRT_TRACE_PERSISTENT && L.fetch) {
         uint32_t grid = (uint32_t)(L.sm_count > 0 ? L.sm_count : 148) * SRT_TRACE_PT_BLOCKS;
-        grid = std::min(grid, std::max(1u, blocks_for(L.max_n, TRACE_BLOCK)));
+        const uint32_t group_max = grid * (TRACE_BLOCK / GROUP) * SRT_TRACE_GROUP_WAVES;
+        grid = std::min(grid, std::max(1u, blocks_for(L.max_n, TRACE_BLOCK / GROUP)));
         k_trace_pt<ANY, COUNT, STACK><<<grid, TRACE_BLOCK, smem, st>>>(L.s, L.queue, L.count, L.fetch, L.ro, L.rd,
                                                                       L.hit, L.sh_id, L.sh_c, L.rad, L.err, L.stats,
-                                                                      L.kind, L.bounce);
+                                                                      L.kind, L.bounce, group_max);
     } else {
         k_trace<ANY, COUNT, STACK><<<blocks_for(L.max_n, TRACE_BLOCK), TRACE_BLOCK, smem, st>>>(
             L.s, L.queue, L.count, L.ro, L.rd, L.hit, L.sh_id, L.sh_c, L.rad, L.err, L.stats, L.kind, L.bounce);
