@@ -833,7 +833,8 @@ struct srt_renderer {
         a.ph.photons = pipe[s].photons;
         a.ph.sorted = pipe[s].sorted;
         a.ph.ranges = pipe[s].ranges;
-        a.gather.photons = pipe[s].sorted;
+        a.gather.pos = pipe[s].sorted;
+        a.gather.dir = pipe[s].sorted + ph.capacity;
         a.gather.ranges = pipe[s].ranges;
         return a;
     }
@@ -856,8 +857,8 @@ struct srt_renderer {
         pipe[0].ranges = ph.ranges;
         if ((e = dev_alloc(&pipe[1].photons, 2ull * cap)) != cudaSuccess) return e;
         if ((e = dev_alloc(&pipe[1].sorted, 2ull * cap)) != cudaSuccess) return e;
-        if ((e = dev_alloc(&pipe[1].ranges, (size_t)1 << p.hash_bits)) != cudaSuccess) return e;
-        if ((e = cudaMemset(pipe[1].ranges, 0, sizeof(uint2) << p.hash_bits)) != cudaSuccess) return e;
+        if ((e = dev_alloc(&pipe[1].ranges, range_entries(p.hash_bits))) != cudaSuccess) return e;
+        if ((e = cudaMemset(pipe[1].ranges, 0, sizeof(uint2) * range_entries(p.hash_bits))) != cudaSuccess) return e;
         for (auto& ps : pipe) {
             if ((e = dev_alloc(&ps.counters, 1)) != cudaSuccess) return e;
             if ((e = cudaMemset(ps.counters, 0, sizeof(FrameCounters))) != cudaSuccess) return e;
@@ -917,7 +918,7 @@ struct srt_renderer {
         cudaFree(counters);
         cudaFree(stats);
         cudaFree(err);
-        void* bufs[] = {pb.ray_o, pb.ray_d, pb.hit, pb.thr, pb.wl, pb.rad, pb.misc, pb.queue[0], pb.queue[1],
+        void* bufs[] = {pb.ga_p, pb.ga_n, pb.ga_f, pb.ga_start, pb.ray_o, pb.ray_d, pb.hit, pb.thr, pb.wl, pb.rad, pb.misc, pb.queue[0], pb.queue[1],
                         pb.sh_o, pb.sh_d, pb.sh_c, pb.sh_id, pb.sort_keys, pb.sort_keys_alt, pb.sort_vals_alt,
                         pb.sort_scratch, ph.ray_o, ph.ray_d, ph.state, ph.hit, ph.flags,
                         ph.queue[0], ph.queue[1], ph.staging, ph.block_counts, ph.photons, ph.sorted,
@@ -1013,6 +1014,7 @@ struct srt_renderer {
             n += launch_bounce(args, b, st, 1);
             mark(2, (int)b);
             n += launch_bounce(args, b, st, 2);
+            n += launch_gather(args, b, st);
             mark(3, (int)b);
             n += launch_bounce(args, b, st, 3);
             mark(4, (int)b);
@@ -1033,7 +1035,7 @@ struct srt_renderer {
     // fork from and join `st`): the camera rays and their first closest hits
     // beside the photon pass (neither reads the other's buffers; shading
     // joins them), and after each shading step the shadow rays of bounce b
-    // beside the closest hits of bounce b + 1 (the shadow rays add to the
+    // beside the closest hits of bounce b + 1 (the photon gathers, then the shadow rays add to the
     // path radiance, which the shading of b + 1 reads after the join; the
     // closest hits read and write only rays, queues and hits).  The results
     // are those of the serial order.
@@ -1091,16 +1093,19 @@ struct srt_renderer {
             n += launch_bounce(A, b, st, 2);
             if (b + 1 == tail) {
                 // the tail kernel shades paths whose radiance these shadow rays add to: after them
+                n += launch_gather(A, b, st);
                 n += launch_bounce(A, b, st, 3);
                 n += launch_tail(A, tail, st);
                 break;
             }
             if (b + 1 < p.max_depth) {
                 fork();
+                n += launch_gather(A, b, s2);
                 n += launch_bounce(A, b, s2, 3);
                 n += launch_bounce(A, b + 1, st, 1);
                 join();
             } else {
+                n += launch_gather(A, b, st);
                 n += launch_bounce(A, b, st, 3);
             }
         }
@@ -1131,7 +1136,10 @@ struct srt_renderer {
     // guide = false: the guided continuation and the training step are left
     // to the batch's grouped guide kernels
     int record_shade(uint32_t b, cudaStream_t st, bool guide) {
-        return b < p.max_depth ? launch_bounce(frame_args(), b, st, guide ? 2 : 4) : 0;
+        if (b >= p.max_depth) return 0;
+        const FrameArgs A = frame_args();
+        const int n = launch_bounce(A, b, st, guide ? 2 : 4);
+        return n + launch_gather(A, b, st);
     }
     int record_end(cudaStream_t st, bool guide) {
         const FrameArgs A = frame_args();
@@ -1225,6 +1233,12 @@ extern "C" srt_status srt_renderer_create(srt_ctx* c, srt_scene* s, uint32_t w, 
     CUDA_TRY(c, dev_alloc(&pb.sh_d, np));
     CUDA_TRY(c, dev_alloc(&pb.sh_c, np));
     CUDA_TRY(c, dev_alloc(&pb.sh_id, np));
+    if (p.photons_per_frame > 0) {
+        CUDA_TRY(c, dev_alloc(&pb.ga_p, np));
+        CUDA_TRY(c, dev_alloc(&pb.ga_n, np));
+        CUDA_TRY(c, dev_alloc(&pb.ga_f, np));
+        CUDA_TRY(c, dev_alloc(&pb.ga_start, np));
+    }
     if (p.flags & SRT_FLAG_RAY_SORT) {
         CUDA_TRY(c, dev_alloc(&pb.sort_keys, np));
         CUDA_TRY(c, dev_alloc(&pb.sort_keys_alt, np));
@@ -1262,8 +1276,8 @@ extern "C" srt_status srt_renderer_create(srt_ctx* c, srt_scene* s, uint32_t w, 
         CUDA_TRY(c, dev_alloc(&ph.keys2, cap));
         CUDA_TRY(c, dev_alloc(&ph.vals2, cap));
         CUDA_TRY(c, dev_alloc(&ph.sort_scratch, radix_scratch_words(cap)));
-        CUDA_TRY(c, dev_alloc(&ph.ranges, (size_t)1 << p.hash_bits));
-        CUDA_TRY(c, cudaMemset(ph.ranges, 0, sizeof(uint2) << p.hash_bits));
+        CUDA_TRY(c, dev_alloc(&ph.ranges, range_entries(p.hash_bits)));
+        CUDA_TRY(c, cudaMemset(ph.ranges, 0, sizeof(uint2) * range_entries(p.hash_bits)));
     }
     FrameArgs& a = r->args;
     a.scene = s->dev;
@@ -1280,7 +1294,8 @@ extern "C" srt_status srt_renderer_create(srt_ctx* c, srt_scene* s, uint32_t w, 
     a.err = r->err;
     a.pb = pb;
     a.ph = ph;
-    a.gather.photons = ph.sorted;
+    a.gather.pos = ph.sorted;
+    a.gather.dir = ph.sorted + cap;
     a.gather.ranges = ph.ranges;
     a.gather.hash_bits = p.hash_bits;
     a.gather.cap = p.gather_cap;
@@ -1670,7 +1685,7 @@ srt_status temp_grid(srt_ctx* c, const srt_photon* photons, uint32_t n, uint32_t
     CUDA_TRY(c, dev_alloc(&t.ph.keys2, n));
     CUDA_TRY(c, dev_alloc(&t.ph.vals2, n));
     CUDA_TRY(c, dev_alloc(&t.ph.sort_scratch, radix_scratch_words(n)));
-    CUDA_TRY(c, dev_alloc(&t.ph.ranges, (size_t)1 << bits));
+    CUDA_TRY(c, dev_alloc(&t.ph.ranges, range_entries(bits)));
     if (n) CUDA_TRY(c, cudaMemcpyAsync(t.src, photons, (size_t)n * 32, cudaMemcpyHostToDevice, c->stream));
     t.ph.capacity = n;
     launch_grid_build(t.src, n, frame, cell, bits, t.ph, c->stream);
@@ -1716,7 +1731,8 @@ extern "C" srt_status srt_photon_gather(srt_ctx* c, const srt_photon* photons, u
         return cuda_fail(c, e, "alloc");
     }
     GatherArgs g{};
-    g.photons = t.ph.sorted;
+    g.pos = t.ph.sorted;
+    g.dir = t.ph.sorted + n;
     g.ranges = t.ph.ranges;
     g.hash_bits = p->hash_bits;
     g.cap = p->gather_cap;
@@ -2207,16 +2223,6 @@ extern "C" srt_status srt_renderer_splat_photons(srt_renderer* r, const srt_came
 #ifndef SRT_BATCH_PHOTON_PIPELINE
 #define SRT_BATCH_PHOTON_PIPELINE 0
 #endif
-// 1: the batch shades all its scenes' vertices of a bounce in one launch
-// (k_shade_multi); 0 (the default): one shading launch per scene on its
-// graph branch, the branches running at once.  Measured on the 32-scene
-// batch (256^2..1024^2 viewports, all scenes active): 120.2 ms per iteration
-// with the branches, 123.5 ms with the single launch (it reads the frame
-// arguments from shared memory and spills more registers).
-#ifndef SRT_BATCH_SHADE_MULTI
-#define SRT_BATCH_SHADE_MULTI 0
-#endif
-
 struct srt_batch {
     srt_ctx* ctx = nullptr;
     std::vector<srt_renderer*> r;
@@ -2225,9 +2231,8 @@ struct srt_batch {
     cudaEvent_t up_ev[2] = {};
     int up_i = 0;
     MultiTraceItem* items_dev = nullptr;  // [2 kinds][MAX_BOUNCES][MAX_BATCH]
-    uint32_t* fetch_dev = nullptr;        // [4][MAX_BOUNCES]: closest-hit, shadow, guide, shading chunk counters
+    uint32_t* fetch_dev = nullptr;        // [3][MAX_BOUNCES]: closest-hit, shadow, guide chunk counters
     FrameArgs* guide_items_dev = nullptr; // [MAX_BATCH] frame arguments of the guided renderers
-    FrameArgs* shade_items_dev = nullptr; // [MAX_BATCH] frame arguments of the active renderers
     std::vector<uint32_t> graph_gen;      // the renderers' args_gen at capture
     std::vector<cudaStream_t> side;
     cudaStream_t cap = nullptr;
@@ -2284,7 +2289,6 @@ struct srt_batch {
         cudaFree(items_dev);
         cudaFree(fetch_dev);
         cudaFree(guide_items_dev);
-        cudaFree(shade_items_dev);
         for (srt_renderer* x : r) {
             if (x) {
                 x->batch_owned = false;
@@ -2351,7 +2355,7 @@ struct srt_batch {
             }
             for (int k = 0; k < na; ++k) cudaStreamWaitEvent(cap, join_ev[k], 0);
         };
-        cudaMemsetAsync(fetch_dev, 0, sizeof(uint32_t) * 4 * MAX_BOUNCES, cap);
+        cudaMemsetAsync(fetch_dev, 0, sizeof(uint32_t) * 3 * MAX_BOUNCES, cap);
         for (int k = 0; k < na; ++k) r[act[k]]->record_clear(cap);
         auto closest = [&](uint32_t b, cudaStream_t s) {
             return launch_trace_multi(items_dev + (size_t)b * MAX_BATCH, na, 0, small_stack, fetch_dev + b,
@@ -2393,10 +2397,7 @@ struct srt_batch {
         uint32_t tail = 0;
         for (int k = 0; k < na; ++k) tail = std::max(tail, r[act[k]]->tail_start());
         for (uint32_t b = 0; b < max_depth; ++b) {
-            if (SRT_BATCH_SHADE_MULTI)
-                n += launch_shade_multi(shade_items_dev, na, b, fetch_dev + 3 * MAX_BOUNCES + b, c->sm_count, cap);
-            else
-                fork_join([b](srt_renderer* x, cudaStream_t s) { return x->record_shade(b, s, false); });
+            fork_join([b](srt_renderer* x, cudaStream_t s) { return x->record_shade(b, s, false); });
             if (ng && b + 1 < guide_depth)
                 n += launch_guide_infer_multi(guide_items_dev, ng, b, fetch_dev + 2 * MAX_BOUNCES + b, c->sm_count,
                                               cap);
@@ -2423,13 +2424,6 @@ struct srt_batch {
             if (sets[act[k]] >= 0) cudaStreamWaitEvent(cap, ph_join[k], 0);
         cudaError_t e = cudaStreamEndCapture(cap, &g);
         CUDA_TRY(c, e);
-        {
-            std::vector<FrameArgs> sargs;
-            for (int k = 0; k < na; ++k) sargs.push_back(r[act[k]]->frame_args());
-            e = cudaMemcpy(shade_items_dev, sargs.data(), na * sizeof(FrameArgs), cudaMemcpyHostToDevice);
-            if (e != cudaSuccess) cudaGraphDestroy(g);
-            CUDA_TRY(c, e);
-        }
         if (ng) {
             std::vector<FrameArgs> gargs;
             for (srt_renderer* x : guided) gargs.push_back(x->frame_args());
@@ -2575,9 +2569,8 @@ extern "C" srt_status srt_batch_create(srt_ctx* c, uint32_t n, srt_scene* const*
     CUDA_TRY(c, cudaMemset(B->cams_dev, 0, n * sizeof(srt_camera_uniform)));
     for (auto& e : B->up_ev) CUDA_TRY(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CUDA_TRY(c, dev_alloc(&B->items_dev, (size_t)2 * MAX_BOUNCES * MAX_BATCH));
-    CUDA_TRY(c, dev_alloc(&B->fetch_dev, (size_t)4 * MAX_BOUNCES));
+    CUDA_TRY(c, dev_alloc(&B->fetch_dev, (size_t)3 * MAX_BOUNCES));
     CUDA_TRY(c, dev_alloc(&B->guide_items_dev, (size_t)MAX_BATCH));
-    CUDA_TRY(c, dev_alloc(&B->shade_items_dev, (size_t)MAX_BATCH));
     CUDA_TRY(c, cudaEventCreateWithFlags(&B->counts_ev, cudaEventDisableTiming));
     CUDA_TRY(c, cudaStreamCreateWithFlags(&B->cap, cudaStreamNonBlocking));
     CUDA_TRY(c, cudaEventCreateWithFlags(&B->fork_ev, cudaEventDisableTiming));

@@ -42,33 +42,124 @@ SRT_DEV uint32_t warp_push(bool pred, uint32_t* counter) {
     return base + __popc(mask & ((1u << lane) - 1u));
 }
 
-// gather_photons: shader.wgsl:297-342 over a sorted range; the walk goes
-// from the highest photon index down (the LIFO order of the reference's
-// linked list for in-order insertion), at most `cap` entries.
-SRT_DEV float4 gather(const GatherArgs& g, uint32_t frame, float3 hit_pos, float3 normal, float4 wl) {
-    float3 j = grid_jitter(frame, g.cell);
-    float r = g.r0 * powf((float)(frame + 1u), g.rexp);
-    float r2 = r * r;
-    uint32_t h = grid_hash(hit_pos, j, g.cell, g.hash_bits);
-    uint2 rg = __ldg(&g.ranges[h]);
-    float4 total = splat4(0.f);
-    uint32_t stop = rg.y - min(rg.y - rg.x, g.cap);
-    for (uint32_t i = rg.y; i > stop; --i) {
-        float4 pa = __ldg(&g.photons[2 * (i - 1)]);
-        float4 pb = __ldg(&g.photons[2 * (i - 1) + 1]);
-        float3 dd = hit_pos - xyz(pa);
-        float d2 = dot(dd, dd);
-        if (d2 < r2 && dot(normal, xyz(pb)) > 0.0f) {
-            float sw = 1.0f - (sqrtf(d2) / r);
-            float4 spw = f4(fmaxf(1.0f - fabsf(wl.x - pa.w) / g.spectral_radius, 0.f),
-                            fmaxf(1.0f - fabsf(wl.y - pa.w) / g.spectral_radius, 0.f),
-                            fmaxf(1.0f - fabsf(wl.z - pa.w) / g.spectral_radius, 0.f),
-                            fmaxf(1.0f - fabsf(wl.w - pa.w) / g.spectral_radius, 0.f));
-            total = total + spw * (pb.w * sw);
-        }
+SRT_DEV GatherConst gather_const(const GatherArgs& g, uint32_t frame) {
+    GatherConst k;
+    k.j = grid_jitter(frame, g.cell);
+    k.r = g.r0 * powf((float)(frame + 1u), g.rexp);
+    k.r2 = k.r * k.r;
+    k.density = (3.0f / (PI * k.r2)) * (1.0f / g.spectral_radius) * g.inv_norm_count;
+    return k;
+}
+
+// gather_photons: shader.wgsl:297-342 over a sorted range: a point's bucket,
+// walked from its highest photon index down (the LIFO order of the
+// reference's linked list for in-order insertion), at most `cap` photons.
+// gather_range is what the walk covers: [.x, .y).
+SRT_DEV uint2 gather_range(const GatherArgs& g, const GatherConst& k, float3 hit_pos) {
+    const uint2 rg = __ldg(&g.ranges[grid_hash(hit_pos, k.j, g.cell, g.hash_bits)]);
+    return make_uint2(rg.y - min(rg.y - rg.x, g.cap), rg.y);
+}
+
+// A photon adds zeros unless it lies within the radius and one of the path's
+// four wavelengths lies within spectral_radius of its own (two usually
+// cannot: they are 100 nm apart), and zeros are left out of the sum.  They are
+// zeros only if every energy is finite and the radius positive: a map with a
+// non-finite energy (ranges' last entry) weights every photon within the radius.
+SRT_DEV bool gather_all(const GatherArgs& g) {
+    return !(g.spectral_radius > 0.f) || __ldg(&g.ranges[(size_t)1 << g.hash_bits]).x != 0u;
+}
+SRT_DEV bool gather_near(float4 pa, float3 hit_pos, float4 wl, float r2, float sr, bool all) {
+    const float3 dd = hit_pos - xyz(pa);
+    const float a =
+        fminf(fminf(fabsf(wl.x - pa.w), fabsf(wl.y - pa.w)), fminf(fabsf(wl.z - pa.w), fabsf(wl.w - pa.w)));
+    return dot(dd, dd) < r2 && (a < sr || all);
+}
+// What a near photon (pa: position + wavelength, pb: direction + energy) adds.
+SRT_DEV float4 gather_weight(float4 pa, float4 pb, float3 hit_pos, float4 wl, float r, float sr, bool all) {
+    const float3 dd = hit_pos - xyz(pa);
+    const float sw = 1.0f - (sqrtf(dot(dd, dd)) / r);
+    const float e = pb.w * sw;
+    const float a0 = fabsf(wl.x - pa.w), a1 = fabsf(wl.y - pa.w), a2 = fabsf(wl.z - pa.w), a3 = fabsf(wl.w - pa.w);
+    if ((a0 < sr) + (a1 < sr) + (a2 < sr) + (a3 < sr) == 1 && !all) {
+        const float w = fmaxf(1.0f - fminf(fminf(a0, a1), fminf(a2, a3)) / sr, 0.f) * e;
+        return f4(a0 < sr ? w : 0.f, a1 < sr ? w : 0.f, a2 < sr ? w : 0.f, a3 < sr ? w : 0.f);
     }
-    float density = (3.0f / (PI * r2)) * (1.0f / g.spectral_radius) * g.inv_norm_count;
-    return total * density;
+    return f4(fmaxf(1.0f - a0 / sr, 0.f), fmaxf(1.0f - a1 / sr, 0.f), fmaxf(1.0f - a2 / sr, 0.f),
+              fmaxf(1.0f - a3 / sr, 0.f)) * e;
+}
+
+// One thread walks a range: which of 32 photons are near, GATHER_BATCH loads
+// at a time (the loads are independent, and every lane of the warp weighs its
+// near photons in one loop per 32), then their weights in order.  In the
+// shading kernel a loop per batch of 4 took 1.99 ms per slab frame, a loop per 32
+// 1.86 (batches of 2 / 8: 1.81 / 1.85), a plain walk 2.35.
+#ifndef SRT_GATHER_BATCH
+#define SRT_GATHER_BATCH 2
+#endif
+constexpr uint32_t GATHER_BATCH = SRT_GATHER_BATCH;
+SRT_DEV float4 gather(const GatherArgs& g, const GatherConst& k, uint2 range, float3 hit_pos, float3 normal, float4 wl) {
+    float4 total = splat4(0.f);
+    const float sr = g.spectral_radius;
+    const bool all = gather_all(g);
+    for (uint32_t i = range.y; i > range.x;) {
+        const uint32_t m = min(i - range.x, 32u);
+        uint32_t near = 0u;
+        for (uint32_t c = 0; c < m; c += GATHER_BATCH) {
+            float4 p[GATHER_BATCH];
+#pragma unroll
+            for (uint32_t b = 0; b < GATHER_BATCH; ++b) p[b] = __ldg(&g.pos[i - 1u - min(c + b, m - 1u)]);
+#pragma unroll
+            for (uint32_t b = 0; b < GATHER_BATCH; ++b)
+                if (gather_near(p[b], hit_pos, wl, k.r2, sr, all)) near |= 1u << (c + b);
+        }
+        near &= 0xFFFFFFFFu >> (32u - m);
+        while (near != 0u) {
+            const uint32_t at = i - (uint32_t)__ffs(near);
+            near &= near - 1u;
+            const float4 pb = __ldg(&g.dir[at]), pa = __ldg(&g.pos[at]);
+            if (dot(normal, xyz(pb)) > 0.0f) total = total + gather_weight(pa, pb, hit_pos, wl, k.r, sr, all);
+        }
+        i -= m;
+    }
+    return total * k.density;
+}
+
+// The same walk by a group of eight lanes (called by all 32 lanes of a warp;
+// the result in all lanes of the group): a lane weighs one photon, and the
+// weights of eight are added in order.
+SRT_DEV float4 gather_group(const GatherArgs& g, const GatherConst& k, bool active, uint2 range, float3 hit_pos,
+                            float3 normal, float4 wl) {
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    const uint32_t c = threadIdx.x & 7u, shift = threadIdx.x & 24u;
+    float4 total = splat4(0.f);
+    const float sr = g.spectral_radius;
+    const bool all = gather_all(g);
+    uint32_t i = range.y;
+    while (__any_sync(FULL, active && i > range.x)) {
+        float4 w = splat4(0.f);
+        bool near = active && i > range.x + c;
+        if (near) {
+            const float4 pa = __ldg(&g.pos[i - 1u - c]);
+            near = gather_near(pa, hit_pos, wl, k.r2, sr, all);
+            if (near) {
+                const float4 pb = __ldg(&g.dir[i - 1u - c]);
+                near = dot(normal, xyz(pb)) > 0.0f;
+                if (near) w = gather_weight(pa, pb, hit_pos, wl, k.r, sr, all);
+            }
+        }
+        // the lanes any group of the warp has to add (a lane without a weight adds zeros)
+        uint32_t add = __ballot_sync(FULL, near);
+        add |= add >> 16;
+        add = (add | (add >> 8)) & 0xFFu;
+        while (add != 0u) {
+            const int from = (int)(shift | ((uint32_t)__ffs(add) - 1u));
+            add &= add - 1u;
+            total = total + f4(__shfl_sync(FULL, w.x, from), __shfl_sync(FULL, w.y, from), __shfl_sync(FULL, w.z, from),
+                               __shfl_sync(FULL, w.w, from));
+        }
+        i = i > range.x + 8u ? i - 8u : range.x;
+    }
+    return total * k.density;
 }
 
 // ------------------------------------------------------------------ photon pass
@@ -308,14 +399,17 @@ __global__ void k_grid_keys(const float4* __restrict__ photons, const uint32_t* 
 
 __global__ void k_grid_ranges(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
                               const uint32_t* n_dev, uint32_t n_host, uint32_t hash_bits,
-                              const float4* __restrict__ photons, float4* __restrict__ sorted, uint2* __restrict__ ranges) {
+                              const float4* __restrict__ photons, float4* __restrict__ sorted, uint32_t capacity,
+                              uint2* __restrict__ ranges) {
     uint32_t n = n_dev ? *n_dev : n_host;
     uint32_t sentinel = 1u << hash_bits;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t h = keys[i];
         uint32_t v = vals[i];
-        sorted[2 * i] = photons[2 * v];
-        sorted[2 * i + 1] = photons[2 * v + 1];
+        const float4 dir = photons[2 * v + 1];
+        sorted[i] = photons[2 * v];
+        sorted[capacity + i] = dir;
+        if (!(fabsf(dir.w) < __int_as_float(0x7F800000))) ranges[sentinel].x = 1u;
         if (h >= sentinel) continue;
         if (i == 0 || keys[i - 1] != h) ranges[h].x = i;
         if (i + 1 == n || keys[i + 1] != h) ranges[h].y = i + 1;
@@ -366,7 +460,10 @@ __global__ void k_raygen(FrameArgs a) {
     a.pb.rad[p] = splat4(0.0f);
     a.pb.misc[p] = make_uint4(s, 0u, p, 0u);
     a.pb.queue[0][q] = p;
-    if (q == 0) a.counters->paths[0] = n;
+    if (q == 0) {
+        a.counters->paths[0] = n;
+        a.counters->gather = gather_const(a.gather, cam.frame_count);
+    }
 }
 
 struct LightSample {
@@ -413,16 +510,22 @@ struct VertexOut {
     float sh_tmax = 0.f;
     float4 sh_c = splat4(0.f);
     uint32_t key = 0u;
+    bool gather = false;                // TAIL only: photons to gather, over ga_range at ga_p
+    uint2 ga_range = make_uint2(0u, 0u);
+    float3 ga_p = f3(0.f, 0.f, 0.f), ga_n = f3(0.f, 0.f, 0.f);
+    float4 ga_f = splat4(0.f);
     float4 g_p = splat4(0.f), g_n = splat4(0.f), g_wo = splat4(0.f), g_spec = splat4(0.f);
 };
 
 // One iteration of ray_color's bounce loop after the closest-hit query
 // (shader.wgsl:568-700) for path `id`, whose hit is in a.pb.hit[id]: writes
-// the path's radiance and, when it continues, its next ray and state.
+// the path's radiance and, when it continues, its next ray and state.  The
+// photon gather of a diffuse vertex is left to launch_gather (queued here) or,
+// TAIL, to the caller; either adds it before the vertex's shadow ray.
 // GUIDE: Lambert continuations of bounces < guide_bounces are left to
 // k_guide_infer (guide.cu); every guided renderer records the radiance a
 // training record's next vertex sees.
-template <bool GUIDE>
+template <bool GUIDE, bool TAIL>
 SRT_DEV VertexOut shade_vertex(const FrameArgs& a, uint32_t id, uint32_t bounce) {
     VertexOut out;
     const DevScene& S = a.scene;
@@ -431,11 +534,11 @@ SRT_DEV VertexOut shade_vertex(const FrameArgs& a, uint32_t id, uint32_t bounce)
     if (prim == MISS) return out;
     float4 o4 = a.pb.ray_o[id], d4 = a.pb.ray_d[id];
     float3 o = xyz(o4), d = xyz(d4);
-    float4 thr = a.pb.thr[id], wl = a.pb.wl[id], rad = a.pb.rad[id];
+    float4 thr = a.pb.thr[id], wl = a.pb.wl[id];
     uint4 misc = a.pb.misc[id];
     uint32_t s = misc.x, flags = misc.y;
     // a training record of the previous vertex: radiance before this vertex
-    if (GUIDE && misc.w != 0u) a.guide.rec.rad[misc.w - 1u] = rad;
+    if (GUIDE && misc.w != 0u) a.guide.rec.rad[misc.w - 1u] = a.pb.rad[id];
     Surface sf = surface_at(S, prim, h.z, h.w, d);
     float4 color = S.materials[2 * sf.mat], extra = S.materials[2 * sf.mat + 1];
     float3 ffn = sf.front ? sf.wn : -sf.wn;
@@ -443,7 +546,7 @@ SRT_DEV VertexOut shade_vertex(const FrameArgs& a, uint32_t id, uint32_t bounce)
     if (type == 3u) {
         if (!(flags & FLAG_CAUSTIC) && (sf.front || extra.y > 0.0f)) {
             float4 em = blackbody4(wl, color.x) * color.y;
-            a.pb.rad[id] = rad + em * thr;
+            a.pb.rad[id] = a.pb.rad[id] + em * thr;
         }
         return out;
     }
@@ -453,8 +556,31 @@ SRT_DEV VertexOut shade_vertex(const FrameArgs& a, uint32_t id, uint32_t bounce)
         float4 spec = rgb_to_spectrum4(xyz(color), wl);
         float3 hp = o + d * h.x;
         if (a.gather.enabled) {
-            float4 gl = gather(a.gather, a.cam->frame_count, hp, ffn, wl);
-            rad = rad + thr * (spec / PI) * gl;
+            const GatherConst& k = a.counters->gather;
+            const uint2 rg = gather_range(a.gather, k, hp);
+            const float4 f = thr * (spec / PI);
+            const float inf = __int_as_float(0x7F800000);
+            // an empty range adds zeros (unless a factor is not finite)
+            if (rg.y > rg.x || !(max4(f) < inf) || !(fabsf(k.density) < inf)) {
+                if (TAIL) {
+                    out.gather = true;
+                    out.ga_range = rg;
+                    out.ga_p = hp;
+                    out.ga_n = ffn;
+                    out.ga_f = f;
+                } else {
+                    // a slot for each lane that is here (in any grouping)
+                    const uint32_t here = __activemask();
+                    const uint32_t lane = threadIdx.x & 31u, leader = (uint32_t)__ffs(here) - 1u;
+                    uint32_t slot = 0u;
+                    if (lane == leader) slot = atomicAdd(&a.counters->gathers[bounce], (uint32_t)__popc(here));
+                    slot = __shfl_sync(here, slot, (int)leader) + __popc(here & ((1u << lane) - 1u));
+                    a.pb.ga_p[slot] = f4(hp.x, hp.y, hp.z, __uint_as_float(id));
+                    a.pb.ga_n[slot] = f4(ffn.x, ffn.y, ffn.z, __uint_as_float(rg.y));
+                    a.pb.ga_f[slot] = f;
+                    a.pb.ga_start[slot] = rg.x;
+                }
+            }
         }
         LightSample ls = sample_light(S, hp, wl, s);
         if (ls.pdf > 0.0f) {
@@ -467,7 +593,6 @@ SRT_DEV VertexOut shade_vertex(const FrameArgs& a, uint32_t id, uint32_t bounce)
             out.sh_tmax = ls.dist - 0.001f;
             out.shadow = true;
         }
-        a.pb.rad[id] = rad;
         if (GUIDE && bounce + 1u < a.max_depth && bounce < a.guide_bounces) {
             out.guided = true;
             out.g_p = f4(hp.x, hp.y, hp.z, wl.x);
@@ -510,7 +635,7 @@ SRT_DEV void shade_slot(const FrameArgs& a, uint32_t bounce, uint32_t q, uint32_
     bool valid = q < n;
     uint32_t id = valid ? a.pb.queue[bounce & 1][q] : 0u;
     VertexOut v;
-    if (valid) v = shade_vertex<GUIDE>(a, id, bounce);
+    if (valid) v = shade_vertex<GUIDE, false>(a, id, bounce);
     uint32_t slot = warp_push(v.alive, &a.counters->paths[bounce + 1]);
     if (v.alive) {
         a.pb.queue[(bounce + 1) & 1][slot] = id;
@@ -542,47 +667,42 @@ __global__ void __launch_bounds__(TRACE_BLOCK, SRT_SHADE_MIN_BLOCKS) k_shade(Fra
     shade_slot<GUIDE>(a, bounce, blockIdx.x * blockDim.x + threadIdx.x, n);
 }
 
-// The shading of many scenes in one launch (the batched renderer): a virtual
-// queue concatenates the scenes' path queues of this bounce, each padded to
-// whole blocks, so a block's chunk belongs to one scene; blocks draw chunks
-// from *fetch and copy that scene's frame arguments into shared memory when
-// the scene changes.  Per vertex the work is k_shade's (guided scenes write
-// their Lambert vertices for the grouped guide inference).
-__global__ void __launch_bounds__(TRACE_BLOCK, SRT_SHADE_MIN_BLOCKS)
-    k_shade_multi(const FrameArgs* __restrict__ items, int n_items, uint32_t bounce, uint32_t* __restrict__ fetch) {
-    __shared__ FrameArgs sa;
-    __shared__ uint32_t pre[MAX_BATCH + 1];
-    __shared__ uint32_t chunk;
-    if (threadIdx.x == 0) {
-        uint32_t acc = 0;
-        for (int i = 0; i < n_items; ++i) {
-            pre[i] = acc;
-            acc += (items[i].counters->paths[bounce] + TRACE_BLOCK - 1u) / TRACE_BLOCK;
+// The photon gathers a bounce queued (shade_vertex): one per thread, or one
+// per eight lanes where they are few (at most SRT_GATHER_GROUP_WAVES for each
+// group of the grid's lanes).  Their own launch, so that the lanes of a warp
+// all walk a range: in the shading kernel, where one vertex in three lies in a
+// caustic and walks up to 64 photons, 11 of 32 lanes were active.  Shading with
+// the gathers, per frame: caustic slab at 1080p 2.35 -> 1.53 ms, Cornell 640x480
+// 0.72 -> 0.48, config 1 0.28 -> 0.16, config 2 1.72 -> 1.57; frames 5.19 -> 4.14,
+// 2.30 -> 1.98, 0.91 -> 0.73, 8.17 -> 8.01 ms.  Threshold 0 / 1 / 2 / 4 / 8 / 64:
+// slab 1.60 / 1.55 / 1.53 / 1.53 / 1.53 / 1.73, Cornell 0.59 / 0.53 / 0.50 / 0.48 /
+// 0.48 / 0.48, config 1 0.23 / 0.17 / 0.16 / 0.17 / 0.16 / 0.17, config 2 1.56 / 1.56
+// / 1.56 / 1.57 / 1.60 / 1.59.
+#ifndef SRT_GATHER_GROUP_WAVES
+#define SRT_GATHER_GROUP_WAVES 4
+#endif
+__global__ void __launch_bounds__(TRACE_BLOCK, SRT_SHADE_MIN_BLOCKS) k_gather(FrameArgs a, uint32_t bounce) {
+    const uint32_t n = a.counters->gathers[bounce];
+    const GatherConst& k = a.counters->gather;
+    if (n <= gridDim.x * (TRACE_BLOCK / GROUP) * SRT_GATHER_GROUP_WAVES) {
+        const uint32_t c = threadIdx.x & 7u, group = threadIdx.x / GROUP;
+        for (uint32_t base = blockIdx.x * (TRACE_BLOCK / GROUP); base < n; base += gridDim.x * (TRACE_BLOCK / GROUP)) {
+            const uint32_t q = base + group;
+            const bool have = q < n;
+            const float4 p = have ? a.pb.ga_p[q] : splat4(0.f), nn = have ? a.pb.ga_n[q] : splat4(0.f);
+            const uint2 range = make_uint2(have ? a.pb.ga_start[q] : 0u, __float_as_uint(nn.w));
+            const uint32_t id = __float_as_uint(p.w);
+            const float4 gl = gather_group(a.gather, k, have, range, xyz(p), xyz(nn), have ? a.pb.wl[id] : splat4(0.f));
+            if (have && c == 0u) a.pb.rad[id] = a.pb.rad[id] + a.pb.ga_f[q] * gl;
         }
-        pre[n_items] = acc;
+        return;
     }
-    int cur = -1;
-    constexpr int kWords = (int)(sizeof(FrameArgs) / sizeof(uint32_t));
-    static_assert(sizeof(FrameArgs) % sizeof(uint32_t) == 0, "FrameArgs is copied as words");
-    while (true) {
-        __syncthreads();  // the previous chunk is done with `chunk` and `sa`
-        if (threadIdx.x == 0) chunk = atomicAdd(fetch, 1u);
-        __syncthreads();
-        const uint32_t c = chunk;
-        if (c >= pre[n_items]) break;
-        int sc = 0;
-        while (sc + 1 < n_items && pre[sc + 1] <= c) ++sc;
-        if (sc != cur) {  // block-uniform
-            const uint32_t* src = reinterpret_cast<const uint32_t*>(items + sc);
-            uint32_t* dst = reinterpret_cast<uint32_t*>(&sa);
-            for (int k = (int)threadIdx.x; k < kWords; k += TRACE_BLOCK) dst[k] = src[k];
-            cur = sc;
-            __syncthreads();
-        }
-        const uint32_t n = sa.counters->paths[bounce];
-        const uint32_t q = (c - pre[sc]) * TRACE_BLOCK + threadIdx.x;
-        if (sa.guiding) shade_slot<true>(sa, bounce, q, n);
-        else shade_slot<false>(sa, bounce, q, n);
+    for (uint32_t q = blockIdx.x * TRACE_BLOCK + threadIdx.x; q < n; q += gridDim.x * TRACE_BLOCK) {
+        const float4 p = a.pb.ga_p[q], nn = a.pb.ga_n[q];
+        const uint32_t id = __float_as_uint(p.w);
+        const float4 gl = gather(a.gather, k, make_uint2(a.pb.ga_start[q], __float_as_uint(nn.w)), xyz(p), xyz(nn),
+                                 a.pb.wl[id]);
+        a.pb.rad[id] = a.pb.rad[id] + a.pb.ga_f[q] * gl;
     }
 }
 
@@ -659,9 +779,21 @@ __global__ void __launch_bounds__(TRACE_BLOCK, SRT_TAIL_MIN_BLOCKS) k_tail(Frame
         if (live && c == 0u) {
             a.pb.hit[id] = prim != MISS ? make_float4(t, __uint_as_float(prim), u, v)
                                         : make_float4(0.f, __uint_as_float(MISS), 0.f, 0.f);
-            vo = shade_vertex<GUIDE>(a, id, b);
+            vo = shade_vertex<GUIDE, true>(a, id, b);
         }
         __syncwarp();  // the path's next ray, written by the group's first lane, is read by all
+        if (__any_sync(FULL, vo.gather)) {
+            const bool ga = __shfl_sync(FULL, (int)vo.gather, (int)shift) != 0;
+            const uint2 range = make_uint2(__shfl_sync(FULL, vo.ga_range.x, (int)shift),
+                                           __shfl_sync(FULL, vo.ga_range.y, (int)shift));
+            const float3 p = f3(__shfl_sync(FULL, vo.ga_p.x, (int)shift), __shfl_sync(FULL, vo.ga_p.y, (int)shift),
+                                __shfl_sync(FULL, vo.ga_p.z, (int)shift));
+            const float3 nn = f3(__shfl_sync(FULL, vo.ga_n.x, (int)shift), __shfl_sync(FULL, vo.ga_n.y, (int)shift),
+                                 __shfl_sync(FULL, vo.ga_n.z, (int)shift));
+            const float4 gl = gather_group(a.gather, a.counters->gather, ga, range, p, nn,
+                                           ga ? a.pb.wl[id] : splat4(0.f));
+            if (ga && c == 0u) a.pb.rad[id] = a.pb.rad[id] + vo.ga_f * gl;
+        }
         const uint32_t alive = __ballot_sync(FULL, vo.alive), shadow = __ballot_sync(FULL, vo.shadow);
         if (shadow) {
             const float3 so = f3(__shfl_sync(FULL, vo.sh_o.x, (int)shift), __shfl_sync(FULL, vo.sh_o.y, (int)shift),
@@ -780,7 +912,9 @@ __global__ void k_gather_queries(GatherArgs g, uint32_t frame, const float* __re
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float* a = q + 10 * i;
-    out[i] = gather(g, frame, f3(a[0], a[1], a[2]), f3(a[3], a[4], a[5]), f4(a[6], a[7], a[8], a[9]));
+    const GatherConst k = gather_const(g, frame);
+    const float3 p = f3(a[0], a[1], a[2]);
+    out[i] = gather(g, k, gather_range(g, k, p), p, f3(a[3], a[4], a[5]), f4(a[6], a[7], a[8], a[9]));
 }
 
 __global__ void k_test_math(int op, uint32_t n, const void* __restrict__ in, void* __restrict__ out,
@@ -898,9 +1032,9 @@ int launch_photon_pass(FrameArgs& a, cudaStream_t st) {
     ++launches;
     launches += sort_pairs(a.ph.keys, a.ph.vals, a.ph.keys2, a.ph.vals2, a.ph.capacity, &a.counters->photons_stored, 0,
                            (int)a.gather.hash_bits + 1, a.ph.sort_scratch, st, &a.ph.sorted_keys, &a.ph.sorted_vals);
-    cudaMemsetAsync(a.ph.ranges, 0, sizeof(uint2) << a.gather.hash_bits, st);
+    cudaMemsetAsync(a.ph.ranges, 0, sizeof(uint2) * range_entries(a.gather.hash_bits), st);
     k_grid_ranges<<<grid, 256, 0, st>>>(a.ph.sorted_keys, a.ph.sorted_vals, &a.counters->photons_stored, 0,
-                                        a.gather.hash_bits, a.ph.photons, a.ph.sorted, a.ph.ranges);
+                                        a.gather.hash_bits, a.ph.photons, a.ph.sorted, a.ph.capacity, a.ph.ranges);
     ++launches;
     return launches;
 }
@@ -913,8 +1047,8 @@ int launch_grid_build(const float4* photons, uint32_t n, uint32_t frame, float c
     ++launches;
     launches += sort_pairs(ph.keys, ph.vals, ph.keys2, ph.vals2, n, nullptr, 0, (int)hash_bits + 1, ph.sort_scratch, st,
                            &ph.sorted_keys, &ph.sorted_vals);
-    cudaMemsetAsync(ph.ranges, 0, sizeof(uint2) << hash_bits, st);
-    k_grid_ranges<<<grid, 256, 0, st>>>(ph.sorted_keys, ph.sorted_vals, nullptr, n, hash_bits, photons, ph.sorted,
+    cudaMemsetAsync(ph.ranges, 0, sizeof(uint2) * range_entries(hash_bits), st);
+    k_grid_ranges<<<grid, 256, 0, st>>>(ph.sorted_keys, ph.sorted_vals, nullptr, n, hash_bits, photons, ph.sorted, n,
                                         ph.ranges);
     ++launches;
     return launches;
@@ -928,8 +1062,8 @@ int launch_raygen(const FrameArgs& a, cudaStream_t st) {
 int launch_bounce(const FrameArgs& a, uint32_t bounce, cudaStream_t st, int stage) {
     int launches = 0;
     uint32_t grid = blocks_for((uint64_t)a.width * a.height, TRACE_BLOCK);
-    if (stage == 0 || stage == 1) launches += launch_trace_closest(a, bounce, st);
-    if (stage == 0 || stage == 2 || stage == 4) {
+    if (stage == 1) launches += launch_trace_closest(a, bounce, st);
+    if (stage == 2 || stage == 4) {
         if (a.guiding) k_shade<true><<<grid, TRACE_BLOCK, 0, st>>>(a, bounce);
         else k_shade<false><<<grid, TRACE_BLOCK, 0, st>>>(a, bounce);
         ++launches;
@@ -943,15 +1077,15 @@ int launch_bounce(const FrameArgs& a, uint32_t bounce, cudaStream_t st, int stag
                                    a.pb.sort_scratch, st, &sk, &sv);
         }
     }
-    if (stage == 0 || stage == 3) launches += launch_trace_shadow(a, bounce, st);
+    if (stage == 3) launches += launch_trace_shadow(a, bounce, st);
     return launches;
 }
 
-int launch_shade_multi(const FrameArgs* items, int n_items, uint32_t bounce, uint32_t* fetch, int sm_count,
-                       cudaStream_t st) {
-    if (n_items <= 0) return 0;
-    const uint32_t grid = (uint32_t)(sm_count > 0 ? sm_count : 148) * SRT_SHADE_MIN_BLOCKS;
-    k_shade_multi<<<grid, TRACE_BLOCK, 0, st>>>(items, n_items, bounce, fetch);
+int launch_gather(const FrameArgs& a, uint32_t bounce, cudaStream_t st) {
+    if (!a.gather.enabled) return 0;
+    const uint32_t grid = std::min(blocks_for((uint64_t)a.width * a.height, TRACE_BLOCK / GROUP),
+                                   (uint32_t)(a.sm_count > 0 ? a.sm_count : 148) * SRT_SHADE_MIN_BLOCKS);
+    k_gather<<<grid, TRACE_BLOCK, 0, st>>>(a, bounce);
     return 1;
 }
 

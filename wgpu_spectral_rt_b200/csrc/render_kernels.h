@@ -13,14 +13,23 @@ constexpr int MAX_PHOTON_BOUNCES = 16;  // photon_max_bounces limit (the referen
 constexpr int PHOTON_BLOCK = 128;   // emitter ids per photon-trace block
 constexpr int TRACE_BLOCK = 128;
 
+// What the photon gather needs besides its query, the same for a whole frame.
+struct GatherConst {
+    float3 j;           // grid jitter
+    float r, r2;        // gather radius and its square
+    float density;      // scale of the weighted sum
+};
+
 // Device counters of one frame (zeroed at frame start).
 struct FrameCounters {
     uint32_t paths[MAX_BOUNCES + 1];    // active paths entering bounce i
     uint32_t shadow[MAX_BOUNCES + 1];   // shadow rays emitted at bounce i
+    uint32_t gathers[MAX_BOUNCES + 1];  // photon gathers queued at bounce i
     uint32_t photon_paths[MAX_PHOTON_BOUNCES + 1];  // live photon paths entering bounce i
     uint32_t fetch[3][MAX_BOUNCES + 1];  // persistent traversal: next queue position, by TRAV_* kind and bounce
     uint32_t photons_stored;
     uint32_t photons_emitted;  // emitted by this photon pass (photon_paths[0] holds those that may scatter)
+    GatherConst gather;        // written by the frame's ray generation
     uint32_t pad;
 };
 
@@ -46,6 +55,10 @@ struct PathBuffers {
     uint32_t* queue[2];
     float4 *sh_o, *sh_d, *sh_c;
     uint32_t* sh_id;
+    // photon gathers of one bounce: point + path id, normal + end of the photon
+    // range, throughput x reflectance / pi, start of the range
+    float4 *ga_p, *ga_n, *ga_f;
+    uint32_t* ga_start;
     // ray reordering of the live queue between bounces
     uint32_t *sort_keys, *sort_keys_alt, *sort_vals_alt, *sort_scratch;
 };
@@ -59,19 +72,23 @@ struct PhotonBuffers {
     float4* staging;        // per emitter: the stored photon, 2 float4
     uint32_t* block_counts; // per block of PHOTON_BLOCK emitters; scanned in place into offsets
     float4* photons;        // emission order, 2 per photon
-    float4* sorted;         // (hash, index) order, 2 per photon
+    float4* sorted;         // (hash, index) order: position + wavelength of every photon,
+                            // then (from entry `capacity`) direction + energy
     uint32_t *keys, *vals, *keys2, *vals2;
     uint32_t* sort_scratch;
-    uint2* ranges;          // 2^hash_bits (start, end)
+    uint2* ranges;          // 2^hash_bits (start, end), then one entry: .x = a photon's energy is not finite
     uint32_t capacity;      // = photons per frame
     uint32_t n_blocks;
     // after a sort: which buffers hold the sorted keys / values
     uint32_t *sorted_keys, *sorted_vals;
 };
 
+constexpr size_t range_entries(uint32_t hash_bits) { return ((size_t)1 << hash_bits) + 1; }
+
 struct GatherArgs {
-    const float4* photons;  // sorted
-    const uint2* ranges;
+    const float4* pos;      // sorted: position + wavelength
+    const float4* dir;      // sorted: direction + energy
+    const uint2* ranges;    // 2^hash_bits + 1 entries
     uint32_t hash_bits;
     uint32_t cap;
     float cell, r0, rexp, spectral_radius, inv_norm_count;
@@ -113,7 +130,9 @@ int launch_photon_pass(FrameArgs& a, cudaStream_t st);
 // Camera paths: raygen, then per bounce trace / shade / shadow; finalize.
 int launch_raygen(const FrameArgs& a, cudaStream_t st);
 int launch_bounce(const FrameArgs& a, uint32_t bounce, cudaStream_t st,
-                  int stage /* 0 all, 1 trace, 2 shade, 3 shadow, 4 shade without the guided continuation */);
+                  int stage /* 1 trace, 2 shade, 3 shadow, 4 shade without the guided continuation */);
+// The photon gathers the shading of `bounce` queued: after it, and before its shadow rays (both add to the radiance).
+int launch_gather(const FrameArgs& a, uint32_t bounce, cudaStream_t st);
 int launch_trace_closest(const FrameArgs& a, uint32_t bounce, cudaStream_t st);  // trace_kernels.cu
 int launch_trace_shadow(const FrameArgs& a, uint32_t bounce, cudaStream_t st);   // trace_kernels.cu
 // Closest hit for the rays named by queue[0 .. *count) (queue NULL: 0 .. *count),
@@ -127,10 +146,6 @@ int launch_trace_queue(const DevScene& s, uint32_t bounce, const uint32_t* queue
 int launch_tail(const FrameArgs& a, uint32_t first, cudaStream_t st);
 // Paths that one wave of launch_tail holds at once for these frame arguments (8 lanes each).
 uint32_t tail_paths(const FrameArgs& a);
-// The shading of bounce `bounce` of n_items scenes (device table of their
-// frame arguments) in one persistent launch; *fetch starts at 0.
-int launch_shade_multi(const FrameArgs* items, int n_items, uint32_t bounce, uint32_t* fetch, int sm_count,
-                       cudaStream_t st);
 int launch_finalize(const FrameArgs& a, cudaStream_t st);
 int launch_frame_stats(const FrameArgs& a, cudaStream_t st);
 
