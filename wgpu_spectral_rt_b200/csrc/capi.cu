@@ -310,6 +310,7 @@ struct srt_scene {
     uint4* mesh_infos = nullptr;
     float4* materials = nullptr;
     float4* lights = nullptr;
+    float4* light_frames = nullptr;
     InstDev* inst = nullptr;
     InstFwd* fwd = nullptr;
     BvhOutputs bvh{};
@@ -346,6 +347,7 @@ struct srt_scene {
         cudaFree(mesh_infos);
         cudaFree(materials);
         cudaFree(lights);
+        cudaFree(light_frames);
         cudaFree(inst);
         cudaFree(fwd);
         cudaFree(bvh.nodes);
@@ -447,6 +449,7 @@ srt_status scene_build_impl(srt_ctx* c, const srt_scene_arrays* a,
     CUDA_TRY(c, upload(&s->mesh_infos, a->mesh_infos, 16ull * a->n_meshes, 16ull * a->n_meshes, st));
     CUDA_TRY(c, upload(&s->materials, a->materials, 32ull * a->n_materials, 32ull * a->n_materials, st));
     CUDA_TRY(c, upload(&s->lights, a->lights, 64ull * a->n_lights, 64ull * a->n_lights, st));
+    CUDA_TRY(c, dev_alloc(&s->light_frames, a->n_lights));
     CUDA_TRY(c, upload(&s->inst, inst.data(), sizeof(InstDev) * inst.size(), sizeof(InstDev) * inst.size(), st));
     CUDA_TRY(c, upload(&s->fwd, fwd.data(), sizeof(InstFwd) * fwd.size(), sizeof(InstFwd) * fwd.size(), st));
     BvhInputs bi{s->vtx, s->idx, s->mesh_infos, s->inst, s->fwd, a->n_instances, (uint32_t)total,
@@ -472,6 +475,7 @@ srt_status scene_build_impl(srt_ctx* c, const srt_scene_arrays* a,
     d.mesh_infos = s->mesh_infos;
     d.materials = s->materials;
     d.lights = s->lights;
+    d.light_frames = s->light_frames;
     d.n_lights = a->n_lights;
     d.inst = s->inst;
     d.tri_inst = s->bvh.tri_inst;
@@ -531,9 +535,10 @@ srt_status scene_build_impl(srt_ctx* c, const srt_scene_arrays* a,
         s->n_light_insts = (uint32_t)li.size();
         launch_expand_lights(s->light_insts, s->n_light_insts, nullptr, s->vtx, s->idx, s->mesh_infos, s->inst, s->fwd,
                              s->lights, st);
-        CUDA_TRY(c, cudaGetLastError());
-        CUDA_TRY(c, cudaStreamSynchronize(st));
     }
+    launch_light_frames(s->lights, s->n_lights, s->light_frames, st);
+    CUDA_TRY(c, cudaGetLastError());
+    CUDA_TRY(c, cudaStreamSynchronize(st));
     ctx_retain(c);
     *out = s.release();
     return SRT_OK;
@@ -586,6 +591,7 @@ extern "C" srt_status srt_scene_update_instances(srt_scene* s, const uint32_t* i
                         s->inst, s->fwd, st);
     launch_expand_lights(s->light_insts, s->n_light_insts, s->moved, s->vtx, s->idx, s->mesh_infos, s->inst, s->fwd,
                          s->lights, st);
+    launch_light_frames(s->lights, s->n_lights, s->light_frames, st);
     refit_bvh8(s->bvh.nodes, s->bvh.tris, s->bvh, s->refit_aux, s->refit_err, st);
     CUDA_TRY(c, cudaGetLastError());
     uint32_t herr = 0;
@@ -918,7 +924,7 @@ struct srt_renderer {
         cudaFree(counters);
         cudaFree(stats);
         cudaFree(err);
-        void* bufs[] = {pb.ga_p, pb.ga_n, pb.ga_f, pb.ga_start, pb.ray_o, pb.ray_d, pb.hit, pb.thr, pb.wl, pb.rad, pb.misc, pb.queue[0], pb.queue[1],
+        void* bufs[] = {pb.ga_p, pb.ga_n, pb.ga_f, pb.ga_start, pb.ray_o, pb.ray_d, pb.hit, pb.thr, pb.wl, pb.rad, pb.light, pb.misc, pb.queue[0], pb.queue[1],
                         pb.sh_o, pb.sh_d, pb.sh_c, pb.sh_id, pb.sort_keys, pb.sort_keys_alt, pb.sort_vals_alt,
                         pb.sort_scratch, ph.ray_o, ph.ray_d, ph.state, ph.hit, ph.flags,
                         ph.queue[0], ph.queue[1], ph.staging, ph.block_counts, ph.photons, ph.sorted,
@@ -1226,6 +1232,7 @@ extern "C" srt_status srt_renderer_create(srt_ctx* c, srt_scene* s, uint32_t w, 
     CUDA_TRY(c, dev_alloc(&pb.thr, np));
     CUDA_TRY(c, dev_alloc(&pb.wl, np));
     CUDA_TRY(c, dev_alloc(&pb.rad, np));
+    CUDA_TRY(c, dev_alloc(&pb.light, np));
     CUDA_TRY(c, dev_alloc(&pb.misc, np));
     CUDA_TRY(c, dev_alloc(&pb.queue[0], np));
     CUDA_TRY(c, dev_alloc(&pb.queue[1], np));

@@ -51,6 +51,7 @@ constexpr int TRAV_CLOSEST = 0, TRAV_SHADOW = 1, TRAV_PHOTON = 2;
 
 struct PathBuffers {
     float4 *ray_o, *ray_d, *hit, *thr, *wl, *rad;
+    float4* light;  // blackbody radiance at the first light's temperature, once a vertex has needed it
     uint4* misc;  // rng, flags, pixel, pad
     uint32_t* queue[2];
     float4 *sh_o, *sh_d, *sh_c;
@@ -127,6 +128,8 @@ struct FrameArgs {
 
 // Photon pass: trace, compaction, grid keys, radix sort, ranges.
 int launch_photon_pass(FrameArgs& a, cudaStream_t st);
+// Unit normal and area of every light (DevScene.light_frames), after any change of the lights.
+int launch_light_frames(const float4* lights, uint32_t n, float4* frames, cudaStream_t st);
 // Camera paths: raygen, then per bounce trace / shade / shadow; finalize.
 int launch_raygen(const FrameArgs& a, cudaStream_t st);
 int launch_bounce(const FrameArgs& a, uint32_t bounce, cudaStream_t st,
