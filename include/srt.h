@@ -167,8 +167,8 @@ typedef struct srt_stats {
     uint64_t frames;
     uint64_t paths;             /* camera paths started */
     uint64_t rays_closest;      /* camera-path closest-hit rays */
-    uint64_t rays_shadow;       /* any-hit (shadow) rays */
-    uint64_t rays_photon;       /* photon-pass closest-hit rays */
+    uint64_t rays_shadow;       /* any-hit (shadow) rays, those that could add nothing (not traced) included */
+    uint64_t rays_photon;       /* photon-pass closest-hit rays, the emitted ones that cannot scatter (not traced) included */
     uint64_t photons_emitted;
     uint64_t photons_stored;
     uint64_t nodes_visited[3];  /* SRT_FLAG_COUNT_VISITS only: camera closest, shadow, photon */

@@ -54,7 +54,10 @@ def test_lights_of_several_temperatures_match_the_oracle(srt, orc, ctx, temps, t
     u = srt.camera_uniform([0.0, 0.0, 3.0], -np.pi / 2, 0.0, W / H, 0)
     r.render(u)
     g = r.read_accum()[..., :3]
-    ref = o.render_frame(u, W, H, p)[0][..., :3]
+    ref, _, _, counts = o.render_frame(u, W, H, p)
+    ref = ref[..., :3]
+    # light samples behind the surface are not traced, but counted: the oracle traces them
+    assert abs(r.stats()["rays_shadow"] - int(counts[2])) <= 0.01 * int(counts[2])
     ok = (np.abs(g - ref) <= 1e-3 * np.maximum(np.abs(ref), 1e-3)).all(-1)
     assert ref.mean() > 0 and ok.mean() >= 0.97, ok.mean()
     r.close()

@@ -23,7 +23,8 @@ struct GatherConst {
 // Device counters of one frame (zeroed at frame start).
 struct FrameCounters {
     uint32_t paths[MAX_BOUNCES + 1];    // active paths entering bounce i
-    uint32_t shadow[MAX_BOUNCES + 1];   // shadow rays emitted at bounce i
+    uint32_t shadow[MAX_BOUNCES + 1];   // shadow rays queued at bounce i
+    uint32_t dark[MAX_BOUNCES + 1];     // light samples whose shadow ray could add zeros only: not queued
     uint32_t gathers[MAX_BOUNCES + 1];  // photon gathers queued at bounce i
     uint32_t photon_paths[MAX_PHOTON_BOUNCES + 1];  // live photon paths entering bounce i
     uint32_t fetch[3][MAX_BOUNCES + 1];  // persistent traversal: next queue position, by TRAV_* kind and bounce
