@@ -609,52 +609,63 @@ SRT_DEV bool scatters_photons(float4 extra) {
     return type == 1u || type == 2u || type == 4u || type == 5u;
 }
 
-// Whether the ray meets the box of a leaf that holds a scattering triangle
-// (S.scatter), on a walk of such subtrees only.  Conservative: the closest-hit
-// traversal reaches a triangle through boxes that pass the same slab test with
-// a t_max no larger than `tmax`, so a ray refused here has no scattering
-// triangle as its closest hit.  `stack`: STACK entries of this thread, stride
-// `stride` (one entry per level at most).
-template <int STACK>
-SRT_DEV bool may_scatter(const DevScene& S, float3 o, float3 d, float tmin, float tmax, uint2* stack, int stride,
-                         uint32_t* err) {
-    if (S.n_nodes == 0u || !(d.x != 0.0f || d.y != 0.0f || d.z != 0.0f)) return false;
+// Walk of a ray over the subtrees that hold scattering triangles (S.scatter),
+// one node per step, to the first leaf box of theirs that it meets.
+// Conservative: the closest-hit traversal reaches a triangle through boxes that
+// pass the same slab test with a t_max no larger than `tmax`, so a ray that
+// meets no such leaf has no scattering triangle as its closest hit.
+struct ScatterWalk {
+    float3 o, idir;
+    uint32_t oct;
+    uint2 g;  // child base; child slots left (bits 8..15) | imask
+    int sp;
+};
+constexpr int WALK_ON = 0, WALK_MAY_SCATTER = 1, WALK_DONE = 2;
+
+// False: the ray cannot hit anything.
+SRT_DEV bool scatter_init(ScatterWalk& W, const DevScene& S, float3 o, float3 d) {
+    W.o = o;
     const float eps = 1e-12f;
-    const float3 idir = f3(1.0f / (fabsf(d.x) > eps ? d.x : copysignf(eps, d.x)),
-                           1.0f / (fabsf(d.y) > eps ? d.y : copysignf(eps, d.y)),
-                           1.0f / (fabsf(d.z) > eps ? d.z : copysignf(eps, d.z)));
-    const uint32_t oct = (d.x < 0.f ? 1u : 0u) | (d.y < 0.f ? 2u : 0u) | (d.z < 0.f ? 4u : 0u);
-    uint2 g = make_uint2(0u, 0x101u);  // child base; child slots left (bits 8..15) | imask; the root as slot 0
-    int sp = 0;
-    while (true) {
-        if ((g.y & 0xFF00u) == 0u) {
-            if (sp == 0) return false;
-            --sp;
-            g = stack[sp * stride];
-        }
-        const uint32_t slot = (uint32_t)__ffs(g.y >> 8) - 1u;
-        g.y &= ~(0x100u << slot);
-        const uint32_t idx = g.x + __popc(g.y & ((1u << slot) - 1u) & 0xFFu);
-        if (g.y & 0xFF00u) {
-            if (sp >= STACK) {
-                atomicOr(err, ERR_STACK_OVERFLOW);
-                return false;
-            }
-            stack[sp * stride] = g;
-            ++sp;
-        }
-        if (idx >= S.n_nodes) {
-            atomicOr(err, ERR_BAD_INDEX);
-            return false;
-        }
-        const uint32_t scatter = __ldg(S.scatter + idx);
-        const uint4* np = reinterpret_cast<const uint4*>(S.nodes + idx);
-        const uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
-        const uint32_t hits = node_hits(w0, w1, w2, w3, w4, o, idir, oct, tmin, tmax) & scatter;
-        const uint32_t imask = w0.w >> 24;
-        if (hits & ~imask) return true;
-        g = make_uint2(w1.x, (hits << 8) | imask);
+    W.idir = f3(1.0f / (fabsf(d.x) > eps ? d.x : copysignf(eps, d.x)),
+                1.0f / (fabsf(d.y) > eps ? d.y : copysignf(eps, d.y)),
+                1.0f / (fabsf(d.z) > eps ? d.z : copysignf(eps, d.z)));
+    W.oct = (d.x < 0.f ? 1u : 0u) | (d.y < 0.f ? 2u : 0u) | (d.z < 0.f ? 4u : 0u);
+    W.g = make_uint2(0u, 0x101u);  // the root as child slot 0
+    W.sp = 0;
+    return S.n_nodes != 0u && (d.x != 0.0f || d.y != 0.0f || d.z != 0.0f);
+}
+// `stack`: STACK entries of this thread, stride `stride` (one entry per level at most).
+template <int STACK>
+SRT_DEV int scatter_step(const DevScene& S, ScatterWalk& W, float tmin, float tmax, uint2* stack, int stride,
+                         uint32_t* err) {
+    if ((W.g.y & 0xFF00u) == 0u) {
+        if (W.sp == 0) return WALK_DONE;
+        --W.sp;
+        W.g = stack[W.sp * stride];
     }
+    const uint32_t slot = (uint32_t)__ffs(W.g.y >> 8) - 1u;
+    W.g.y &= ~(0x100u << slot);
+    const uint32_t idx = W.g.x + __popc(W.g.y & ((1u << slot) - 1u) & 0xFFu);
+    if (W.g.y & 0xFF00u) {
+        if (W.sp >= STACK) {
+            atomicOr(err, ERR_STACK_OVERFLOW);
+            return WALK_DONE;
+        }
+        stack[W.sp * stride] = W.g;
+        ++W.sp;
+    }
+    if (idx >= S.n_nodes) {
+        atomicOr(err, ERR_BAD_INDEX);
+        return WALK_DONE;
+    }
+    const uint32_t scatter = __ldg(S.scatter + idx);
+    const uint4* np = reinterpret_cast<const uint4*>(S.nodes + idx);
+    const uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
+    const uint32_t hits = node_hits(w0, w1, w2, w3, w4, W.o, W.idir, W.oct, tmin, tmax) & scatter;
+    const uint32_t imask = w0.w >> 24;
+    if (hits & ~imask) return WALK_MAY_SCATTER;
+    W.g = make_uint2(w1.x, (hits << 8) | imask);
+    return WALK_ON;
 }
 
 // Stack-based traversal of the compressed BVH8.  A node group holds the

@@ -184,7 +184,7 @@ SRT_DEV float4 gather_group(const GatherArgs& g, const GatherConst& k, bool acti
 //
 // Emission culls first: a photon path whose first surface does not scatter
 // (diffuse, emitter) ends there without storing anything, so an emitted ray
-// that meets no leaf box with a scattering triangle (may_scatter: a walk of
+// that meets no leaf box with a scattering triangle (scatter_step: a walk of
 // the scene's tree restricted to those subtrees) needs no closest hit, and
 // none of its state is written.  Config 2 (4.2M emitted, 31k scatter): photon pass 2.12 -> 1.59 ms alone (closest hits of bounce 0
 // 1.42 -> 0.50 ms, emission 0.09 -> 0.66 ms), frame 8.87 -> 8.35 ms; eight
@@ -225,50 +225,80 @@ SRT_DEV uint32_t ray_sort_key(float3 o, float3 d, float4 bmin, float4 binv) {
 
 constexpr uint32_t PH_CAUSTIC = 0x1u;
 
-// Emission (photon_emit.wgsl:159-214), one thread per emitter id: the light
-// point and direction, the cull, and for the rays that may scatter the
-// wavelength, energy and state; they are queued for bounce 0 (any order: a
-// path's results go to its emitter's slot).
+// Emission (photon_emit.wgsl:159-214) in persistent warps: a lane takes an
+// emitter id, draws its light point and direction and walks (scatter_step);
+// once SRT_EMIT_REFILL lanes are done, the rays that may scatter get their
+// wavelength, energy and state and are queued for bounce 0 (any order: a
+// path's results go to its emitter's slot), and the lanes take new ids.  The
+// walks end after 1 to ~10 nodes; one ray per thread, a warp waited for its
+// longest.  Config-2 photon pass alone 1.46 -> 1.25 ms (refill at 4 / 8 / 12 / 16 /
+// 24 idle lanes: 1.36 / 1.27 / 1.25 / 1.25 / 1.30).
+#ifndef SRT_EMIT_REFILL
+#define SRT_EMIT_REFILL 16
+#endif
+constexpr int EMIT_FETCH = MAX_BOUNCES;  // the emission's id counter: fetch[TRAV_PHOTON][EMIT_FETCH]
+static_assert(MAX_PHOTON_BOUNCES < EMIT_FETCH, "photon bounces use the counters below");
+
 template <int STACK>
 __global__ void __launch_bounds__(TRACE_BLOCK, SRT_SHADE_MIN_BLOCKS) k_photon_emit(FrameArgs a) {
     extern __shared__ uint2 stack_smem[];
-    const uint32_t e = blockIdx.x * TRACE_BLOCK + threadIdx.x;
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
     const DevScene& S = a.scene;
-    bool live = e < a.photons_per_frame;
-    if (live) {
-        uint32_t frame = a.cam->frame_count;
-        uint32_t s = pcg_hash(e + frame * 927163u + a.seed);
-        uint32_t nl = S.n_lights;  // > 0: the pass is skipped without lights
-        uint32_t li = min(__float2uint_rz(rng_next(s) * (float)nl), nl - 1u);
-        float4 L0 = S.lights[4 * li], L1 = S.lights[4 * li + 1], L2 = S.lights[4 * li + 2];
-        float3 v0 = xyz(L0), v1 = xyz(L1), v2 = xyz(L2);
-        const float4 lf = S.light_frames[li];
-        float3 normal = xyz(lf);
-        float r1 = rng_next(s);
-        float r2 = rng_next(s);
-        float sr1 = sqrtf(r1);
-        float u = 1.0f - sr1, v = r2 * sr1, w = 1.0f - u - v;
-        float3 emit_pos = v0 * u + v1 * v + v2 * w;
-        float3 emit_dir = normalize(normal + random_unit_vector(s));
-        float3 pos = emit_pos + emit_dir * 0.001f;
-        live = may_scatter<STACK>(S, pos, emit_dir, 0.0001f, 100.0f, stack_smem + threadIdx.x, TRACE_BLOCK, a.err);
-        if (live) {
-            float4 LP = S.lights[4 * li + 3];
-            float area = lf.w;
-            float cmin = cauchy_cdf(LAMBDA_MIN), cmax = cauchy_cdf(LAMBDA_MAX), crange = cmax - cmin;
-            float lambda =
-                clampf(555.0f + 40.0f * tanf(PI * ((cmin + rng_next(s) * crange) - 0.5f)), LAMBDA_MIN, LAMBDA_MAX);
-            float dw = (lambda - 555.0f) / 40.0f;
-            float pdf = (1.0f / (crange * PI * 40.0f)) / (1.0f + dw * dw);
-            float energy = (blackbody(lambda, LP.y) / pdf) * area * PI * LP.z;
-            a.ph.ray_o[e] = f4(pos.x, pos.y, pos.z, 0.0001f);
-            a.ph.ray_d[e] = f4(emit_dir.x, emit_dir.y, emit_dir.z, 100.0f);
-            a.ph.state[e] = f4(lambda, energy, __uint_as_float(s), __uint_as_float(0u));
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    const uint32_t n = a.photons_per_frame, nl = S.n_lights;  // nl > 0: the pass is skipped without lights
+    const uint32_t seed = a.cam->frame_count * 927163u + a.seed;
+    uint32_t* fetch = &a.counters->fetch[TRAV_PHOTON][EMIT_FETCH];
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.counters->photons_emitted = n;
+    ScatterWalk W;
+    float3 dir = f3(0.f, 0.f, 0.f);
+    uint32_t e = 0u, s = 0u, li = 0u;
+    int state = WALK_DONE;
+    bool exhausted = false;
+    while (true) {
+        const uint32_t idle = __ballot_sync(FULL, state != WALK_ON);
+        if (idle == FULL || (!exhausted && __popc(idle) >= SRT_EMIT_REFILL)) {
+            const bool live = state == WALK_MAY_SCATTER;
+            if (live) {
+                const float4 LP = S.lights[4 * li + 3], lf = S.light_frames[li];
+                float cmin = cauchy_cdf(LAMBDA_MIN), cmax = cauchy_cdf(LAMBDA_MAX), crange = cmax - cmin;
+                float lambda =
+                    clampf(555.0f + 40.0f * tanf(PI * ((cmin + rng_next(s) * crange) - 0.5f)), LAMBDA_MIN, LAMBDA_MAX);
+                float dw = (lambda - 555.0f) / 40.0f;
+                float pdf = (1.0f / (crange * PI * 40.0f)) / (1.0f + dw * dw);
+                float energy = (blackbody(lambda, LP.y) / pdf) * lf.w * PI * LP.z;
+                a.ph.ray_o[e] = f4(W.o.x, W.o.y, W.o.z, 0.0001f);
+                a.ph.ray_d[e] = f4(dir.x, dir.y, dir.z, 100.0f);
+                a.ph.state[e] = f4(lambda, energy, __uint_as_float(s), __uint_as_float(0u));
+            }
+            const uint32_t slot = warp_push(live, &a.counters->photon_paths[0]);
+            if (live) a.ph.queue[0][slot] = e;
+            if (state != WALK_ON) state = WALK_DONE;
+            if (exhausted) break;  // every lane is done
+            uint32_t base = 0u;
+            if (lane == 0u) base = atomicAdd(fetch, (uint32_t)__popc(idle));
+            base = __shfl_sync(FULL, base, 0);
+            exhausted = base + (uint32_t)__popc(idle) >= n;
+            if (state != WALK_ON) {
+                e = base + __popc(idle & lt);
+                if (e < n) {
+                    s = pcg_hash(e + seed);
+                    li = min(__float2uint_rz(rng_next(s) * (float)nl), nl - 1u);
+                    const float4 L0 = S.lights[4 * li], L1 = S.lights[4 * li + 1], L2 = S.lights[4 * li + 2],
+                                 lf = S.light_frames[li];
+                    float r1 = rng_next(s);
+                    float r2 = rng_next(s);
+                    float sr1 = sqrtf(r1);
+                    float u = 1.0f - sr1, v = r2 * sr1, w = 1.0f - u - v;
+                    float3 emit_pos = xyz(L0) * u + xyz(L1) * v + xyz(L2) * w;
+                    dir = normalize(xyz(lf) + random_unit_vector(s));
+                    if (scatter_init(W, S, emit_pos + dir * 0.001f, dir)) state = WALK_ON;
+                }
+            }
+            continue;
         }
+        if (state == WALK_ON)
+            state = scatter_step<STACK>(S, W, 0.0001f, 100.0f, stack_smem + threadIdx.x, TRACE_BLOCK, a.err);
     }
-    const uint32_t slot = warp_push(live, &a.counters->photon_paths[0]);
-    if (live) a.ph.queue[0][slot] = e;
-    if (e == 0) a.counters->photons_emitted = a.photons_per_frame;
 }
 
 // One bounce of the photon loop after its closest-hit query
@@ -1046,16 +1076,17 @@ int launch_photon_pass(FrameArgs& a, cudaStream_t st) {
     const uint32_t n = a.photons_per_frame;
     cudaMemsetAsync(a.ph.flags, 0, n, st);
     const uint32_t blocks = blocks_for(n, TRACE_BLOCK);
+    const uint32_t grid_max = (uint32_t)(a.sm_count > 0 ? a.sm_count : 148) * SRT_SHADE_MIN_BLOCKS;
+    const uint32_t pass_grid = std::min(blocks, grid_max);
     if (a.scene.depth <= (uint32_t)TRAV_STACK_SMALL)
-        k_photon_emit<TRAV_STACK_SMALL><<<blocks, TRACE_BLOCK, sizeof(uint2) * TRAV_STACK_SMALL * TRACE_BLOCK, st>>>(a);
-    else k_photon_emit<TRAV_STACK><<<blocks, TRACE_BLOCK, sizeof(uint2) * TRAV_STACK * TRACE_BLOCK, st>>>(a);
+        k_photon_emit<TRAV_STACK_SMALL><<<pass_grid, TRACE_BLOCK, sizeof(uint2) * TRAV_STACK_SMALL * TRACE_BLOCK, st>>>(a);
+    else k_photon_emit<TRAV_STACK><<<pass_grid, TRACE_BLOCK, sizeof(uint2) * TRAV_STACK * TRACE_BLOCK, st>>>(a);
     ++launches;
-    const uint32_t shade_grid = std::min(blocks, (uint32_t)(a.sm_count > 0 ? a.sm_count : 148) * SRT_SHADE_MIN_BLOCKS);
     for (uint32_t b = 0; b < a.photon_max_bounces; ++b) {
         launches += launch_trace_queue(a.scene, b, a.ph.queue[b & 1], &a.counters->photon_paths[b],
                                        &a.counters->fetch[TRAV_PHOTON][b], n, a.ph.ray_o, a.ph.ray_d, a.ph.hit,
                                        TRAV_PHOTON, a.count_visits, a.err, a.stats, a.sm_count, st);
-        k_photon_shade<<<shade_grid, TRACE_BLOCK, 0, st>>>(a, b);
+        k_photon_shade<<<pass_grid, TRACE_BLOCK, 0, st>>>(a, b);
         ++launches;
     }
     // stored photons in emitter order
