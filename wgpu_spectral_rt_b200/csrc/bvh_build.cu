@@ -138,10 +138,10 @@ struct Bvh2 {
 // COLLAPSE_TRI) or a wide node (area x COLLAPSE_NODE + its children's forest of
 // `width` roots).  choice byte i (i = 2 .. width): roots given to the left
 // child, 0: the same forest as i - 1; byte 0: 1 if the node alone is a leaf.
-// Against opening the child of largest area until a node is full: config 2
-// 186k instead of 267k nodes, 6.75 instead of 7.20 visits and 4.84 instead of
-// 4.56 triangle tests per camera ray, the frame unchanged (7.30 ms); Cornell
-// 640x480 1.86 -> 1.77 ms, animated 512x384 3.76 -> 3.69, caustic slab 4.04 -> 4.00.
+// Against opening the child of largest area until a node is full, everywhere
+// (k_collapse still does at the top): config 2 186k instead of 267k nodes, closest
+// hits 3.26 -> 3.22 ms, shadow rays 1.95 -> 1.87; Cornell 640x480 0.73 -> 0.70 and
+// 0.47 -> 0.42, photon pass of the animated scene 0.94 -> 0.89.
 // Weight of a triangle 0.15 / 0.3 / 0.5 / 0.8 of a node: config 2 closest hits
 // 3.29 / 3.26 / 3.26 / 3.24 ms, shadow rays 1.93 / 1.95 / 1.96 / 1.99; animated
 // 1.01 / 1.00 / 1.00 / 1.00 and 0.54 / 0.54 / 0.57 / 0.57.
@@ -859,13 +859,45 @@ __global__ void k_collapse(Bvh2 b, const uint2* __restrict__ qin, uint32_t n_in,
     uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n_in) return;
     uint2 q = qin[e];
-    // the children: the forest of `width` roots that collapse_costs chose
     uint32_t refs[8];
     int roots[8];  // how many roots refs[c] may become
     int nc = 1;
     refs[0] = q.x;
     roots[0] = 1;
-    if (!(q.x & LEAF)) {
+    const uint32_t below = (q.x & LEAF) ? 1u : b.inode[q.x].w - b.inode[q.x].z + 1u;
+    if (!(q.x & LEAF) && below > tri_cap / 2u) {
+        // a node over more than half of the triangles: the child of largest
+        // area opened until it is full.  The recurrence would make the big flat
+        // leaves (walls) its children, where the quanta are coarsest and every
+        // ray that starts on a wall meets its box: with it at the root too,
+        // bounce 0 of config 2 0.342 vs 0.325 ms, its shadow rays 1.94 vs 1.87 ms
+        // per frame, prism 96x64 camera rays 38 vs 33 us and shadow rays 20 vs
+        // 12 us (opened down to n / 8 or n / 64 triangles: config 2 shadow rays
+        // 1.88, 1.89 ms, closest hits 3.26, 3.27 vs 3.22).
+        uint4 nd = b.inode[q.x];
+        refs[0] = nd.x;
+        refs[1] = nd.y;
+        nc = 2;
+        while (nc < width) {
+            int best = -1;
+            float best_area = -1.0f;
+            for (int c = 0; c < nc; ++c) {
+                if (refs[c] & LEAF) continue;
+                float3 lo, hi;
+                ref_box(b, refs[c], lo, hi);
+                const float area = half_area(lo, hi);
+                if (area > best_area) {
+                    best_area = area;
+                    best = c;
+                }
+            }
+            if (best < 0) break;
+            nd = b.inode[refs[best]];
+            refs[best] = nd.x;
+            refs[nc++] = nd.y;
+        }
+    } else if (!(q.x & LEAF)) {
+        // the forest of `width` roots that collapse_costs chose
         const uint4 nd = b.inode[q.x];
         const int k = (int)choice_of(b, q.x, width);
         refs[0] = nd.x;
