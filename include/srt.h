@@ -458,7 +458,7 @@ srt_status srt_photon_grid_build(srt_ctx* ctx, const srt_photon* photons, uint32
  * may be NULL) and the work is enqueued on `stream` (a cudaStream_t, NULL =
  * legacy default stream) of the current device.  No context is needed.
  * Temporary storage comes from one fixed __device__ array in the library
- * (16.5 MiB, held by every GPU that loads the library until exit); n above
+ * (17 MiB, held by every GPU that loads the library until exit); n above
  * SRT_GRID_NOALLOC_MAX_PHOTONS returns SRT_ERR_CAPACITY.  Alignment:
  * photons 16 bytes, keys_out and ranges_out 8 bytes; a misaligned pointer
  * returns SRT_ERR_INVALID_ARG before any device work.  n = 0 only clears

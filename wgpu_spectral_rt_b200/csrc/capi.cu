@@ -94,7 +94,7 @@ srt_status check_device_error(srt_ctx* c, uint32_t* d_err) {
     if (h != 0u) {
         CUDA_TRY(c, cudaMemsetAsync(d_err, 0, 4, c->stream));
         char buf[96];
-        if (h & ERR_MMA_TIMEOUT) {  // a bounded wait gave up; the context stays usable
+        if (h & (ERR_MMA_TIMEOUT | ERR_WAIT_TIMEOUT)) {  // a bounded wait gave up; the context stays usable
             std::snprintf(buf, sizeof buf, "a bounded device wait gave up (error word 0x%x)", h);
             return fail(c, SRT_ERR_TIMEOUT, buf);
         }
@@ -927,7 +927,7 @@ struct srt_renderer {
         void* bufs[] = {pb.ga_p, pb.ga_n, pb.ga_f, pb.ga_start, pb.ray_o, pb.ray_d, pb.hit, pb.thr, pb.wl, pb.rad, pb.light, pb.misc, pb.queue[0], pb.queue[1],
                         pb.sh_o, pb.sh_d, pb.sh_c, pb.sh_id, pb.sort_keys, pb.sort_keys_alt, pb.sort_vals_alt,
                         pb.sort_scratch, ph.ray_o, ph.ray_d, ph.state, ph.hit, ph.flags,
-                        ph.queue[0], ph.queue[1], ph.staging, ph.block_counts, ph.photons, ph.sorted,
+                        ph.queue[0], ph.queue[1], ph.staging, ph.deposit, ph.photons, ph.sorted,
                         ph.keys, ph.vals, ph.keys2, ph.vals2, ph.sort_scratch, ph.ranges, accum, accum64, ldr};
         for (void* b : bufs) cudaFree(b);
         guide_free(guide);
@@ -1263,19 +1263,18 @@ extern "C" srt_status srt_renderer_create(srt_ctx* c, srt_scene* s, uint32_t w, 
     PhotonBuffers& ph = r->ph;
     uint32_t cap = p.photons_per_frame;
     ph.capacity = cap;
-    ph.n_blocks = (cap + PHOTON_BLOCK - 1) / PHOTON_BLOCK;
     if (cap > 0) {
-        size_t slots = (size_t)ph.n_blocks * PHOTON_BLOCK;
-        CUDA_TRY(c, dev_alloc(&ph.ray_o, slots));
-        CUDA_TRY(c, dev_alloc(&ph.ray_d, slots));
-        CUDA_TRY(c, dev_alloc(&ph.state, slots));
-        CUDA_TRY(c, dev_alloc(&ph.hit, slots));
+        const size_t slots = (size_t)deposit_tiles(cap) * DEPOSIT_TILE;
+        CUDA_TRY(c, dev_alloc(&ph.ray_o, cap));
+        CUDA_TRY(c, dev_alloc(&ph.ray_d, cap));
+        CUDA_TRY(c, dev_alloc(&ph.state, cap));
+        CUDA_TRY(c, dev_alloc(&ph.hit, cap));
         CUDA_TRY(c, dev_alloc(&ph.flags, slots));
         CUDA_TRY(c, cudaMemset(ph.flags, 0, slots));
-        CUDA_TRY(c, dev_alloc(&ph.queue[0], slots));
-        CUDA_TRY(c, dev_alloc(&ph.queue[1], slots));
-        CUDA_TRY(c, dev_alloc(&ph.staging, 2ull * slots));
-        CUDA_TRY(c, dev_alloc(&ph.block_counts, ph.n_blocks));
+        CUDA_TRY(c, dev_alloc(&ph.queue[0], cap));
+        CUDA_TRY(c, dev_alloc(&ph.queue[1], cap));
+        CUDA_TRY(c, dev_alloc(&ph.staging, 2ull * cap));
+        CUDA_TRY(c, dev_alloc(&ph.deposit, deposit_words(cap)));
         CUDA_TRY(c, dev_alloc(&ph.photons, 2ull * cap));
         CUDA_TRY(c, dev_alloc(&ph.sorted, 2ull * cap));
         CUDA_TRY(c, dev_alloc(&ph.keys, cap));
@@ -1695,7 +1694,7 @@ srt_status temp_grid(srt_ctx* c, const srt_photon* photons, uint32_t n, uint32_t
     CUDA_TRY(c, dev_alloc(&t.ph.ranges, range_entries(bits)));
     if (n) CUDA_TRY(c, cudaMemcpyAsync(t.src, photons, (size_t)n * 32, cudaMemcpyHostToDevice, c->stream));
     t.ph.capacity = n;
-    launch_grid_build(t.src, n, frame, cell, bits, t.ph, c->stream);
+    launch_grid_build(t.src, n, frame, cell, bits, t.ph, c->d_err, c->stream);
     CUDA_TRY(c, cudaGetLastError());
     return SRT_OK;
 }

@@ -27,6 +27,7 @@ constexpr int TRAV_STACK_SMALL = 16;  // stack for trees of at most 16 levels (l
 constexpr uint32_t ERR_STACK_OVERFLOW = 0x1u;
 constexpr uint32_t ERR_QUEUE_OVERFLOW = 0x2u;
 constexpr uint32_t ERR_BAD_INDEX = 0x4u;
+constexpr uint32_t ERR_WAIT_TIMEOUT = 0x40u;  // a bounded look-back (deposit, sort) gave up
 
 // ------------------------------------------------------------------ layouts
 // Per instance (64 B): mesh/material ids, first flattened triangle and the

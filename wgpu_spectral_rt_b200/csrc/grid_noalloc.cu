@@ -8,7 +8,7 @@
 // temporary storage from one file-scope __device__ array of fixed size, and
 // works only on buffers the caller already owns.
 //
-// The array (GRID_NOALLOC_SCRATCH_WORDS 32-bit words, 16.5 MiB) lives in
+// The array (GRID_NOALLOC_SCRATCH_WORDS 32-bit words, 17 MiB) lives in
 // every GPU that loads this library until the process exits.  Every call
 // shares it, so calls that overlap on the GPU (concurrent streams, or several
 // host threads) race on it and must be serialised by the caller.  Each call
@@ -27,29 +27,20 @@ namespace srt {
 
 // Photon capacity of the scratch: the reference's MAX_PHOTONS (2^20).
 constexpr uint32_t GRID_NOALLOC_MAX_PHOTONS = 1u << 20;
-// keys, values and their ping-pong copies (4 words per photon) + sort histograms
+// keys, values and their ping-pong copies (4 words per photon) + the sort's scratch
 constexpr size_t GRID_NOALLOC_SCRATCH_WORDS =
-    4ull * GRID_NOALLOC_MAX_PHOTONS + 256ull * (GRID_NOALLOC_MAX_PHOTONS / RS_TILE) + 256ull;
+    4ull * GRID_NOALLOC_MAX_PHOTONS + radix_scratch_words(GRID_NOALLOC_MAX_PHOTONS);
 
 static __device__ __align__(256) uint32_t g_grid_noalloc_scratch[GRID_NOALLOC_SCRATCH_WORDS];
 
 namespace {
 
-__global__ void k_noalloc_keys(const float4* __restrict__ photons, uint32_t n, uint32_t frame, float cell,
-                               uint32_t hash_bits, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-    float3 j = grid_jitter(frame, cell);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float4 p0 = photons[2 * i], p1 = photons[2 * i + 1];
-        keys[i] = p1.w == 0.0f ? (1u << hash_bits) : grid_hash(xyz(p0), j, cell, hash_bits);
-        vals[i] = i;
-    }
-}
-
 // Sorted (hash, index) pairs -> 64-bit keys and the [start, end) range of
 // every non-empty bucket (ranges were cleared before).
 __global__ void k_noalloc_ranges(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals, uint32_t n,
                                  uint32_t hash_bits, unsigned long long* __restrict__ keys_out,
-                                 uint2* __restrict__ ranges) {
+                                 uint2* __restrict__ ranges, const uint32_t* __restrict__ sort_scratch) {
+    if (sort_scratch[RS_GAVE_UP] != 0u) return;  // the sort's bounded wait gave up (calls overlapped): empty ranges
     uint32_t sentinel = 1u << hash_bits;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t h = keys[i];
@@ -118,29 +109,22 @@ cudaError_t launch(void (*k)(P...), uint32_t grid, uint32_t block, cudaStream_t 
     return e;
 }
 
-// sort_pairs (radix_sort.cuh) with every launch checked as above.
-cudaError_t sort_pairs_checked(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint32_t n,
-                               int end_bit, uint32_t* scratch, cudaStream_t st, uint32_t** out_keys,
-                               uint32_t** out_vals) {
-    const uint32_t tiles = (n + RS_TILE - 1) / RS_TILE;
-    uint32_t* hist = scratch;
-    uint32_t* row_total = scratch + (size_t)256 * tiles;
+// Clears the sort scratch's head (a launch, so that its own status comes back).
+__global__ void k_noalloc_clear(uint32_t* __restrict__ scratch) { rs_clear(scratch, RS_HEAD); }
+
+// sort_passes (radix_sort.cuh) with every launch checked as above.
+cudaError_t sort_passes_checked(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint32_t n,
+                                int end_bit, uint32_t* scratch, cudaStream_t st, uint32_t** out_keys,
+                                uint32_t** out_vals) {
+    const uint32_t tiles = rs_tiles(n);
     const uint32_t* no_dev_count = nullptr;
     uint32_t *ki = keys, *vi = vals, *ko = keys_alt, *vo = vals_alt;
-    for (int shift = 0; shift < end_bit; shift += 8) {
-        cudaError_t e = launch(k_rs_upsweep, tiles, RS_THREADS, st, (const uint32_t*)ki, no_dev_count, n, shift,
-                               tiles, hist);
-        if (e == cudaSuccess) e = launch(k_rs_rowscan, 256u, 1024u, st, hist, tiles, row_total);
-        if (e == cudaSuccess)
-            e = launch(k_rs_scatter, tiles, RS_THREADS, st, (const uint32_t*)ki, (const uint32_t*)vi, ko, vo,
-                       no_dev_count, n, shift, tiles, (const uint32_t*)hist, (const uint32_t*)row_total);
+    for (int p = 0; p < rs_passes(0, end_bit); ++p) {
+        const cudaError_t e = launch(k_rs_pass, tiles, RS_THREADS, st, (const uint32_t*)ki, (const uint32_t*)vi, ko, vo,
+                                     no_dev_count, n, 8 * p, p, tiles, scratch);
         if (e != cudaSuccess) return e;
-        uint32_t* t = ki;
-        ki = ko;
-        ko = t;
-        t = vi;
-        vi = vo;
-        vo = t;
+        std::swap(ki, ko);
+        std::swap(vi, vo);
     }
     *out_keys = ki;
     *out_vals = vi;
@@ -192,22 +176,23 @@ extern "C" srt_status srt_photon_grid_build_noalloc(void* stream, const srt_phot
     uint32_t* vals = s + GRID_NOALLOC_MAX_PHOTONS;
     uint32_t* keys2 = s + 2ull * GRID_NOALLOC_MAX_PHOTONS;
     uint32_t* vals2 = s + 3ull * GRID_NOALLOC_MAX_PHOTONS;
-    uint32_t* hist = s + 4ull * GRID_NOALLOC_MAX_PHOTONS;
-    if (ranges_out) {
+    uint32_t* scratch = s + 4ull * GRID_NOALLOC_MAX_PHOTONS;
+    if (n == 0) {
+        if (!ranges_out) return SRT_OK;
         e = cudaMemsetAsync(ranges_out, 0, sizeof(uint2) << hash_bits, st);
-        if (e != cudaSuccess) {
-            (void)cudaGetLastError();
-            return SRT_ERR_CUDA;
-        }
+        if (e != cudaSuccess) (void)cudaGetLastError();
+        return e == cudaSuccess ? SRT_OK : SRT_ERR_CUDA;
     }
-    if (n == 0) return SRT_OK;
-    const uint32_t grid = 148 * 8;
-    e = launch(k_noalloc_keys, grid, 256u, st, reinterpret_cast<const float4*>(photons), n, frame_count, cell_size,
-               hash_bits, keys, vals);
-    uint32_t *sk = nullptr, *sv = nullptr;
-    if (e == cudaSuccess) e = sort_pairs_checked(keys, vals, keys2, vals2, n, (int)hash_bits + 1, hist, st, &sk, &sv);
+    e = launch(k_noalloc_clear, 1u, 1024u, st, scratch);
     if (e == cudaSuccess)
-        e = launch(k_noalloc_ranges, grid, 256u, st, (const uint32_t*)sk, (const uint32_t*)sv, n, hash_bits,
-                   reinterpret_cast<unsigned long long*>(keys_out), reinterpret_cast<uint2*>(ranges_out));
+        e = launch(grid_keys_kernel(), grid_keys_blocks(n), GRID_KEYS_THREADS, st,
+                   reinterpret_cast<const float4*>(photons), n, frame_count, cell_size, hash_bits, keys, vals, scratch,
+                   reinterpret_cast<uint2*>(ranges_out), 1u << hash_bits);
+    uint32_t *sk = nullptr, *sv = nullptr;
+    if (e == cudaSuccess) e = sort_passes_checked(keys, vals, keys2, vals2, n, (int)hash_bits + 1, scratch, st, &sk, &sv);
+    if (e == cudaSuccess)
+        e = launch(k_noalloc_ranges, 148u * 8u, 256u, st, (const uint32_t*)sk, (const uint32_t*)sv, n, hash_bits,
+                   reinterpret_cast<unsigned long long*>(keys_out), reinterpret_cast<uint2*>(ranges_out),
+                   (const uint32_t*)scratch);
     return e == cudaSuccess ? SRT_OK : SRT_ERR_CUDA;
 }

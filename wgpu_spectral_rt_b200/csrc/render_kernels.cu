@@ -249,6 +249,12 @@ __global__ void __launch_bounds__(TRACE_BLOCK, SRT_SHADE_MIN_BLOCKS) k_photon_em
     const uint32_t seed = a.cam->frame_count * 927163u + a.seed;
     uint32_t* fetch = &a.counters->fetch[TRAV_PHOTON][EMIT_FETCH];
     if (blockIdx.x == 0 && threadIdx.x == 0) a.counters->photons_emitted = n;
+    // what the rest of the pass starts from: no photon stored, no deposit tile
+    // done, no digit counted
+    rs_clear(reinterpret_cast<uint32_t*>(a.ph.flags), deposit_tiles(n) * (DEPOSIT_TILE / 4u));
+    rs_clear(a.ph.deposit, deposit_words(n));
+    rs_clear(a.ph.sort_scratch, RS_HEAD);
+    rs_clear_status(a.ph.sort_scratch, n);
     ScatterWalk W;
     float3 dir = f3(0.f, 0.f, 0.f);
     uint32_t e = 0u, s = 0u, li = 0u;
@@ -391,60 +397,131 @@ __global__ void __launch_bounds__(TRACE_BLOCK, SRT_SHADE_MIN_BLOCKS) k_photon_sh
     }
 }
 
-// Emitter-ordered compaction of the stored photons: per-block counts, an
-// exclusive scan of the counts (k_rs_rowscan), then the scatter.
-__global__ void __launch_bounds__(PHOTON_BLOCK) k_deposit_count(FrameArgs a) {
-    __shared__ uint32_t warp_cnt[PHOTON_BLOCK / 32];
-    uint32_t e = blockIdx.x * PHOTON_BLOCK + threadIdx.x;
-    bool stored = e < a.photons_per_frame && a.ph.flags[e] != 0u;
-    uint32_t m = __ballot_sync(0xFFFFFFFFu, stored);
-    if ((threadIdx.x & 31) == 0) warp_cnt[threadIdx.x >> 5] = __popc(m);
+// The grid key of a photon (build_grid.wgsl:54-73): its cell's hash, or the
+// sentinel bucket for a photon without energy.
+SRT_DEV uint32_t photon_key(float4 p0, float4 p1, float3 jitter, float cell, uint32_t hash_bits) {
+    return p1.w == 0.0f ? (1u << hash_bits) : grid_hash(xyz(p0), jitter, cell, hash_bits);
+}
+constexpr int GRID_PASSES = RS_PASSES;  // digit counts kept by the key kernels: hash_bits <= 26, at most 4 passes
+SRT_DEV void clear_counts(uint32_t* h) {
+    for (uint32_t i = threadIdx.x; i < GRID_PASSES * 256u; i += blockDim.x) h[i] = 0u;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t t = 0;
-        for (int w = 0; w < PHOTON_BLOCK / 32; ++w) t += warp_cnt[w];
-        a.ph.block_counts[blockIdx.x] = t;
-    }
 }
 
-__global__ void __launch_bounds__(PHOTON_BLOCK) k_deposit_scatter(FrameArgs a) {
-    __shared__ uint32_t warp_cnt[PHOTON_BLOCK / 32];
-    uint32_t e = blockIdx.x * PHOTON_BLOCK + threadIdx.x;
-    bool stored = e < a.photons_per_frame && a.ph.flags[e] != 0u;
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t m = __ballot_sync(0xFFFFFFFFu, stored);
-    if (lane == 0) warp_cnt[warp] = __popc(m);
+// Emitter-ordered compaction of the stored photons and their grid keys, in one
+// launch: a tile of emitter flags per block, the photons before it by
+// look-back over the tiles (a warp reads 32 of them at once), each stored photon
+// copied to its place with its key, the keys' digits counted for the sort.
+// Against a count, a scan by one block (32 us for 4M emitters), the copy and the
+// keys, 76 us in four launches, and three memsets: with the sort's passes the
+// photon pass of config 2 1.25 -> 1.14 ms, Cornell 0.82 -> 0.77 ms.
+static_assert(DEPOSIT_TILE == RS_THREADS * 16, "16 flags per thread");
+__global__ void __launch_bounds__(RS_THREADS) k_deposit(FrameArgs a) {
+    __shared__ uint32_t counts[GRID_PASSES * 256];
+    __shared__ uint32_t warp_sums[RS_WARPS], ticket, before;
+    clear_counts(counts);
+    uint32_t* status = a.ph.deposit + 2;
+    if (threadIdx.x == 0) ticket = atomicAdd(&a.ph.deposit[0], 1u);
     __syncthreads();
-    uint32_t before = a.ph.block_counts[blockIdx.x];
-    for (int w = 0; w < warp; ++w) before += warp_cnt[w];
-    if (stored) {
-        uint32_t dst = before + __popc(m & ((1u << lane) - 1u));
-        a.ph.photons[2 * dst] = a.ph.staging[2 * e];
-        a.ph.photons[2 * dst + 1] = a.ph.staging[2 * e + 1];
+    const uint32_t tile = ticket, tiles = deposit_tiles(a.photons_per_frame);
+    const uint32_t first = tile * DEPOSIT_TILE + threadIdx.x * 16u;
+    const uint4 f = *reinterpret_cast<const uint4*>(a.ph.flags + first);  // (flags past the last emitter are clear)
+    uint32_t stored = 0u;
+    const uint32_t w[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)  // bytes of 0 or 1 to bits
+        stored |= ((w[i] & 1u) | ((w[i] >> 7) & 2u) | ((w[i] >> 14) & 4u) | ((w[i] >> 21) & 8u)) << (4 * i);
+    const uint32_t mine = __popc(stored);
+    uint32_t dst = rs_block_exclusive(mine, warp_sums);
+    if (threadIdx.x == RS_THREADS - 1) {
+        const uint32_t total = dst + mine;
+        atomicExch(&status[tile], (tile == 0u ? RS_PREFIX : RS_SUM) | total);
+        warp_sums[0] = total;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-        atomicAdd(&a.stats->photons_stored, (unsigned long long)a.counters->photons_stored);
+    __syncthreads();
+    if (threadIdx.x < 32u) {
+        // 32 tiles before this one at a time, up to the nearest that knows its prefix
+        uint32_t sum = 0u;
+        for (uint32_t t = tile; t > 0u;) {
+            const bool in = threadIdx.x < t;
+            const volatile uint32_t* p = status + (in ? t - 1u - threadIdx.x : 0u);
+            uint32_t s = in ? *p : RS_PREFIX;
+            for (uint32_t polls = 0; __any_sync(0xFFFFFFFFu, s == 0u) && polls < RS_POLLS; ++polls)
+                if (s == 0u) s = *p;
+            if (s == 0u) {
+                atomicOr(a.err, ERR_WAIT_TIMEOUT);
+                s = RS_PREFIX;
+            }
+            const uint32_t done = __ballot_sync(0xFFFFFFFFu, (s & RS_PREFIX) != 0u);
+            const uint32_t last = done != 0u ? (uint32_t)__ffs(done) - 1u : 31u;
+            sum += __reduce_add_sync(0xFFFFFFFFu, threadIdx.x <= last ? (s & RS_COUNT) : 0u);
+            if (done != 0u) break;
+            t -= 32u;
+        }
+        if (threadIdx.x == 0u) {
+            before = sum;
+            const uint32_t all = sum + warp_sums[0];
+            if (tile > 0u) atomicExch(&status[tile], RS_PREFIX | all);
+            if (tile + 1u == tiles) {
+                a.counters->photons_stored = all;
+                atomicAdd(&a.stats->photons_stored, (unsigned long long)all);
+            }
+        }
+    }
+    __syncthreads();
+    dst += before;
+    const float3 j = grid_jitter(a.cam->frame_count, a.gather.cell);
+    const int passes = rs_passes(0, (int)a.gather.hash_bits + 1);
+    while (stored != 0u) {
+        const uint32_t e = first + (uint32_t)__ffs(stored) - 1u;
+        stored &= stored - 1u;
+        const float4 p0 = a.ph.staging[2ull * e], p1 = a.ph.staging[2ull * e + 1];
+        const uint32_t key = photon_key(p0, p1, j, a.gather.cell, a.gather.hash_bits);
+        a.ph.photons[2ull * dst] = p0;
+        a.ph.photons[2ull * dst + 1] = p1;
+        a.ph.keys[dst] = key;
+        a.ph.vals[dst] = dst;
+        rs_count_key(counts, key, 0, passes);
+        ++dst;
+    }
+    __syncthreads();
+    rs_flush_counts(counts, a.ph.sort_scratch, passes);
 }
 
-__global__ void k_grid_keys(const float4* __restrict__ photons, const uint32_t* n_dev, uint32_t n_host,
-                            const uint32_t* frame_dev, uint32_t frame_host, float cell, uint32_t hash_bits,
-                            uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-    uint32_t n = n_dev ? *n_dev : n_host;
-    uint32_t frame = frame_dev ? *frame_dev : frame_host;
-    float3 j = grid_jitter(frame, cell);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float4 p0 = photons[2 * i], p1 = photons[2 * i + 1];
-        keys[i] = p1.w == 0.0f ? (1u << hash_bits) : grid_hash(xyz(p0), j, cell, hash_bits);
+// Keys of a photon array, their digits counted for the sort (its scratch's
+// head cleared before), and every bucket emptied.
+__global__ void __launch_bounds__(GRID_KEYS_THREADS) k_grid_keys(const float4* __restrict__ photons, uint32_t n, uint32_t frame,
+                                                          float cell, uint32_t hash_bits, uint32_t* __restrict__ keys,
+                                                          uint32_t* __restrict__ vals, uint32_t* __restrict__ scratch,
+                                                          uint2* __restrict__ ranges, uint32_t entries) {
+    __shared__ uint32_t counts[GRID_PASSES * 256];
+    clear_counts(counts);
+    const float3 j = grid_jitter(frame, cell);
+    const int passes = rs_passes(0, (int)hash_bits + 1);
+    for (uint32_t i = blockIdx.x * GRID_KEYS_THREADS + threadIdx.x; i < n; i += gridDim.x * GRID_KEYS_THREADS) {
+        const uint32_t key = photon_key(photons[2ull * i], photons[2ull * i + 1], j, cell, hash_bits);
+        keys[i] = key;
         vals[i] = i;
+        rs_count_key(counts, key, 0, passes);
     }
+    rs_clear_status(scratch, n);
+    if (ranges != nullptr)
+        for (uint32_t i = blockIdx.x * GRID_KEYS_THREADS + threadIdx.x; i < entries; i += gridDim.x * GRID_KEYS_THREADS)
+            ranges[i] = make_uint2(0u, 0u);
+    __syncthreads();
+    rs_flush_counts(counts, scratch, passes);
 }
 
 __global__ void k_grid_ranges(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
                               const uint32_t* n_dev, uint32_t n_host, uint32_t hash_bits,
                               const float4* __restrict__ photons, float4* __restrict__ sorted, uint32_t capacity,
-                              uint2* __restrict__ ranges) {
+                              uint2* __restrict__ ranges, const uint32_t* __restrict__ scratch, uint32_t* err) {
     uint32_t n = n_dev ? *n_dev : n_host;
     uint32_t sentinel = 1u << hash_bits;
+    if (n != 0u && scratch[RS_GAVE_UP] != 0u) {  // the sort's wait gave up: no grid
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, ERR_WAIT_TIMEOUT);
+        return;
+    }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t h = keys[i];
         uint32_t v = vals[i];
@@ -950,27 +1027,31 @@ __global__ void k_finalize(FrameArgs a) {
                            (unsigned char)__float2uint_rn(clampf(fc.z, 0.f, 1.f) * 255.0f), 255);
 }
 
+// One lane per bounce (a chain of loads per bounce on one thread took 6 us at
+// the end of every frame).
 __global__ void k_frame_stats(FrameArgs a) {
-    if (threadIdx.x != 0) return;
-    unsigned long long c = 0, s = 0;
-    for (uint32_t i = 0; i < a.max_depth; ++i) {
-        c += a.counters->paths[i];
-        s += a.counters->shadow[i] + a.counters->dark[i];
-        a.stats->rays_bounce[TRAV_CLOSEST][i] += a.counters->paths[i];
-        a.stats->rays_bounce[TRAV_SHADOW][i] += a.counters->shadow[i] + a.counters->dark[i];
+    static_assert(MAX_BOUNCES + 1 == 32 && MAX_PHOTON_BOUNCES < 32, "one warp");
+    const uint32_t i = threadIdx.x;
+    const bool camera = i < a.max_depth, photon = a.photons_per_frame > 0u && i < a.photon_max_bounces;
+    const uint32_t c = camera ? a.counters->paths[i] : 0u;
+    const uint32_t s = camera ? a.counters->shadow[i] + a.counters->dark[i] : 0u;
+    // bounce 0: every emitted ray, also those the cull answered
+    const uint32_t p = !photon ? 0u : i == 0u ? a.ph_counters->photons_emitted : a.ph_counters->photon_paths[i];
+    unsigned long long all[3] = {c, s, p};
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        for (int k = 0; k < 3; ++k) all[k] += __shfl_down_sync(0xFFFFFFFFu, all[k], o);
+    if (camera) {
+        a.stats->rays_bounce[TRAV_CLOSEST][i] += c;
+        a.stats->rays_bounce[TRAV_SHADOW][i] += s;
     }
-    a.stats->closest_rays += c;
-    a.stats->shadow_rays += s;
-    a.stats->paths += a.counters->paths[0];
-    unsigned long long pr = 0;
-    if (a.photons_per_frame > 0u)
-        for (uint32_t i = 0; i < a.photon_max_bounces; ++i) {
-            // bounce 0: every emitted ray, also those the cull answered
-            const uint32_t k = i == 0u ? a.ph_counters->photons_emitted : a.ph_counters->photon_paths[i];
-            pr += k;
-            a.stats->rays_bounce[TRAV_PHOTON][i] += k;
-        }
-    a.stats->photon_rays += pr;
+    if (photon) a.stats->rays_bounce[TRAV_PHOTON][i] += p;
+    if (i == 0u) {
+        a.stats->closest_rays += all[0];
+        a.stats->shadow_rays += all[1];
+        a.stats->photon_rays += all[2];
+        a.stats->paths += c;
+    }
 }
 
 // ------------------------------------------------------------------ batch / test kernels
@@ -1074,7 +1155,7 @@ inline uint32_t blocks_for(uint64_t n, uint32_t b) { return (uint32_t)((n + b - 
 int launch_photon_pass(FrameArgs& a, cudaStream_t st) {
     int launches = 0;
     const uint32_t n = a.photons_per_frame;
-    cudaMemsetAsync(a.ph.flags, 0, n, st);
+    cudaMemsetAsync(a.ph.ranges, 0, sizeof(uint2) * range_entries(a.gather.hash_bits), st);
     const uint32_t blocks = blocks_for(n, TRACE_BLOCK);
     const uint32_t grid_max = (uint32_t)(a.sm_count > 0 ? a.sm_count : 148) * SRT_SHADE_MIN_BLOCKS;
     const uint32_t pass_grid = std::min(blocks, grid_max);
@@ -1089,35 +1170,32 @@ int launch_photon_pass(FrameArgs& a, cudaStream_t st) {
         k_photon_shade<<<pass_grid, TRACE_BLOCK, 0, st>>>(a, b);
         ++launches;
     }
-    // stored photons in emitter order
-    k_deposit_count<<<a.ph.n_blocks, PHOTON_BLOCK, 0, st>>>(a);
-    k_rs_rowscan<<<1, 1024, 0, st>>>(a.ph.block_counts, a.ph.n_blocks, &a.counters->photons_stored);
-    k_deposit_scatter<<<a.ph.n_blocks, PHOTON_BLOCK, 0, st>>>(a);
-    launches += 3;
-    uint32_t grid = 148 * 8;
-    k_grid_keys<<<grid, 256, 0, st>>>(a.ph.photons, &a.counters->photons_stored, 0,
-                                      &a.cam->frame_count, 0, a.gather.cell, a.gather.hash_bits, a.ph.keys, a.ph.vals);
+    // stored photons in emitter order with their keys, then the grid
+    k_deposit<<<deposit_tiles(n), RS_THREADS, 0, st>>>(a);
     ++launches;
-    launches += sort_pairs(a.ph.keys, a.ph.vals, a.ph.keys2, a.ph.vals2, a.ph.capacity, &a.counters->photons_stored, 0,
-                           (int)a.gather.hash_bits + 1, a.ph.sort_scratch, st, &a.ph.sorted_keys, &a.ph.sorted_vals);
-    cudaMemsetAsync(a.ph.ranges, 0, sizeof(uint2) * range_entries(a.gather.hash_bits), st);
-    k_grid_ranges<<<grid, 256, 0, st>>>(a.ph.sorted_keys, a.ph.sorted_vals, &a.counters->photons_stored, 0,
-                                        a.gather.hash_bits, a.ph.photons, a.ph.sorted, a.ph.capacity, a.ph.ranges);
+    launches += sort_passes(a.ph.keys, a.ph.vals, a.ph.keys2, a.ph.vals2, a.ph.capacity, &a.counters->photons_stored, 0,
+                            (int)a.gather.hash_bits + 1, a.ph.sort_scratch, st, &a.ph.sorted_keys, &a.ph.sorted_vals);
+    k_grid_ranges<<<148 * 8, 256, 0, st>>>(a.ph.sorted_keys, a.ph.sorted_vals, &a.counters->photons_stored, 0,
+                                           a.gather.hash_bits, a.ph.photons, a.ph.sorted, a.ph.capacity, a.ph.ranges,
+                                           a.ph.sort_scratch, a.err);
     ++launches;
     return launches;
 }
 
+GridKeysKernel grid_keys_kernel() { return k_grid_keys; }
+
 int launch_grid_build(const float4* photons, uint32_t n, uint32_t frame, float cell, uint32_t hash_bits,
-                      PhotonBuffers& ph, cudaStream_t st) {
+                      PhotonBuffers& ph, uint32_t* err, cudaStream_t st) {
     int launches = 0;
-    uint32_t grid = 148 * 8;
-    k_grid_keys<<<grid, 256, 0, st>>>(photons, nullptr, n, nullptr, frame, cell, hash_bits, ph.keys, ph.vals);
+    cudaMemsetAsync(ph.sort_scratch, 0, RS_HEAD * sizeof(uint32_t), st);
+    k_grid_keys<<<grid_keys_blocks(n), GRID_KEYS_THREADS, 0, st>>>(photons, n, frame, cell, hash_bits, ph.keys, ph.vals,
+                                                           ph.sort_scratch, ph.ranges,
+                                                           (uint32_t)range_entries(hash_bits));
     ++launches;
-    launches += sort_pairs(ph.keys, ph.vals, ph.keys2, ph.vals2, n, nullptr, 0, (int)hash_bits + 1, ph.sort_scratch, st,
-                           &ph.sorted_keys, &ph.sorted_vals);
-    cudaMemsetAsync(ph.ranges, 0, sizeof(uint2) * range_entries(hash_bits), st);
-    k_grid_ranges<<<grid, 256, 0, st>>>(ph.sorted_keys, ph.sorted_vals, nullptr, n, hash_bits, photons, ph.sorted, n,
-                                        ph.ranges);
+    launches += sort_passes(ph.keys, ph.vals, ph.keys2, ph.vals2, n, nullptr, 0, (int)hash_bits + 1, ph.sort_scratch, st,
+                            &ph.sorted_keys, &ph.sorted_vals);
+    k_grid_ranges<<<148 * 8, 256, 0, st>>>(ph.sorted_keys, ph.sorted_vals, nullptr, n, hash_bits, photons, ph.sorted, n,
+                                           ph.ranges, ph.sort_scratch, err);
     ++launches;
     return launches;
 }

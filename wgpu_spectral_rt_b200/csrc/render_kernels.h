@@ -10,7 +10,9 @@ namespace srt {
 
 constexpr int MAX_BOUNCES = 31;     // max_depth limit (queue counters per bounce)
 constexpr int MAX_PHOTON_BOUNCES = 16;  // photon_max_bounces limit (the reference uses 5)
-constexpr int PHOTON_BLOCK = 128;   // emitter ids per photon-trace block
+constexpr uint32_t DEPOSIT_TILE = 8192;  // emitter flags per block of the deposit
+constexpr uint32_t deposit_tiles(uint32_t photons) { return (photons + DEPOSIT_TILE - 1u) / DEPOSIT_TILE; }
+constexpr uint32_t deposit_words(uint32_t photons) { return deposit_tiles(photons) + 2u; }
 constexpr int TRACE_BLOCK = 128;
 
 // What the photon gather needs besides its query, the same for a whole frame.
@@ -69,10 +71,10 @@ struct PhotonBuffers {
     float4 *ray_o, *ray_d;  // per emitter: ray origin + tmin, direction + tmax
     float4* state;          // per emitter: wavelength, energy, rng (bits), flags (bits)
     float4* hit;            // per emitter: closest hit (t, triangle, u, v)
-    uint8_t* flags;         // per emitter: 1 if a photon was stored
+    uint8_t* flags;         // per emitter (whole deposit tiles): 1 if a photon was stored
     uint32_t* queue[2];     // live emitter ids, by bounce parity
     float4* staging;        // per emitter: the stored photon, 2 float4
-    uint32_t* block_counts; // per block of PHOTON_BLOCK emitters; scanned in place into offsets
+    uint32_t* deposit;      // deposit tile counter, -, then a look-back word per tile
     float4* photons;        // emission order, 2 per photon
     float4* sorted;         // (hash, index) order: position + wavelength of every photon,
                             // then (from entry `capacity`) direction + energy
@@ -80,7 +82,6 @@ struct PhotonBuffers {
     uint32_t* sort_scratch;
     uint2* ranges;          // 2^hash_bits (start, end), then one entry: .x = a photon's energy is not finite
     uint32_t capacity;      // = photons per frame
-    uint32_t n_blocks;
     // after a sort: which buffers hold the sorted keys / values
     uint32_t *sorted_keys, *sorted_vals;
 };
@@ -188,7 +189,15 @@ int launch_trace_multi(const MultiTraceItem* items, int n_items, int any_hit, bo
 
 // Grid over a photon array already on the device (n on host).
 int launch_grid_build(const float4* photons, uint32_t n, uint32_t frame, float cell, uint32_t hash_bits,
-                      PhotonBuffers& ph, cudaStream_t st);
+                      PhotonBuffers& ph, uint32_t* err, cudaStream_t st);
+// Its first step: keys and identity values of n photons, the keys' digits
+// counted into the sort scratch (head cleared before), ranges[0 .. entries)
+// cleared (ranges may be NULL).
+typedef void (*GridKeysKernel)(const float4* photons, uint32_t n, uint32_t frame, float cell, uint32_t hash_bits,
+                               uint32_t* keys, uint32_t* vals, uint32_t* scratch, uint2* ranges, uint32_t entries);
+GridKeysKernel grid_keys_kernel();
+constexpr uint32_t GRID_KEYS_THREADS = 512;
+constexpr uint32_t grid_keys_blocks(uint32_t) { return 148u * 4u; }
 int launch_gather_queries(const GatherArgs& g, uint32_t frame, const float* queries, uint32_t n_q, float4* out,
                           cudaStream_t st);
 int launch_trace_batch(const DevScene& s, const float4* rays, uint32_t n, float4* hits, int any_hit, uint32_t* err,
