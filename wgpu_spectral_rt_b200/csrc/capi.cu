@@ -383,13 +383,23 @@ bool instance_rows(const srt_instance& in, InstDev* d, InstFwd* f) {
                     (r[0] * r[8] - r[2] * r[6]) / det, (r[2] * r[3] - r[0] * r[5]) / det,
                     (r[3] * r[7] - r[4] * r[6]) / det, (r[1] * r[6] - r[0] * r[7]) / det,
                     (r[0] * r[4] - r[1] * r[3]) / det};
-    d->w2o0 = make_float4((float)iv[0], (float)iv[1], (float)iv[2], 0.f);
-    d->w2o1 = make_float4((float)iv[3], (float)iv[4], (float)iv[5], 0.f);
-    d->w2o2 = make_float4((float)iv[6], (float)iv[7], (float)iv[8], 0.f);
+    d->w2o0 = make_float4((float)iv[0], (float)iv[1], (float)iv[2], d->w2o0.w);
+    d->w2o1 = make_float4((float)iv[3], (float)iv[4], (float)iv[5], d->w2o1.w);
+    d->w2o2 = make_float4((float)iv[6], (float)iv[7], (float)iv[8], d->w2o2.w);
     f->r0 = make_float4(M[0], M[4], M[8], M[12]);
     f->r1 = make_float4(M[1], M[5], M[9], M[13]);
     f->r2 = make_float4(M[2], M[6], M[10], M[14]);
     return true;
+}
+
+// The words of an instance's hits kept in the .w lanes of its rows (InstDev).
+void instance_words(InstDev* d, const srt_mesh_info& mesh, const srt_material& mat) {
+    const float t = mat.extra[0];  // the device's conversion: truncated, saturated, NaN -> 0
+    const uint32_t words[3] = {mesh.vertex_offset, mesh.index_offset - 3u * d->tri_offset,
+                               t >= 4294967296.0f ? 0xFFFFFFFFu : (t > 0.0f ? (uint32_t)t : 0u)};
+    std::memcpy(&d->w2o0.w, &words[0], 4);
+    std::memcpy(&d->w2o1.w, &words[1], 4);
+    std::memcpy(&d->w2o2.w, &words[2], 4);
 }
 
 srt_status scene_build_impl(srt_ctx* c, const srt_scene_arrays* a,
@@ -436,6 +446,7 @@ srt_status scene_build_impl(srt_ctx* c, const srt_scene_arrays* a,
         d.mat_id = in.mat_id;
         d.tri_offset = (uint32_t)total;
         d.tri_count = mesh_tris[in.mesh_id];
+        instance_words(&d, a->mesh_infos[in.mesh_id], a->materials[in.mat_id]);
         inst[i] = d;
         total += mesh_tris[in.mesh_id];
     }

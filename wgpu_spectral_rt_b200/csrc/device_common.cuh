@@ -34,7 +34,10 @@ constexpr uint32_t ERR_WAIT_TIMEOUT = 0x40u;  // a bounded look-back (deposit, s
 // rows of world_to_object (inverse of the instance's linear part).
 struct InstDev {
     uint32_t mesh_id, mat_id, tri_offset, tri_count;
-    float4 w2o0, w2o1, w2o2;  // rows; .w unused
+    // rows; the .w lanes hold words a hit needs next, a load earlier than from
+    // the mesh and material tables: the mesh's first vertex, its first index - 3
+    // tri_offset (mod 2^32), the material type
+    float4 w2o0, w2o1, w2o2;
 };
 
 // Compressed 8-wide BVH node, 80 B = 5 x uint4 (layout of Ylitie, Karras and
@@ -1381,10 +1384,8 @@ SRT_DEV Surface surface_at(const DevScene& S, uint32_t prim, float u, float v, f
     Surface sf;
     uint32_t ii = __ldg(&S.tri_inst[prim]);
     const InstDev& in = S.inst[ii];
-    uint4 mi = __ldg(&S.mesh_infos[in.mesh_id]);
-    uint32_t io = mi.y + (prim - in.tri_offset) * 3u;
-    uint32_t i0 = __ldg(&S.indices[io]) + mi.x, i1 = __ldg(&S.indices[io + 1]) + mi.x,
-             i2 = __ldg(&S.indices[io + 2]) + mi.x;
+    const uint32_t vo = __float_as_uint(in.w2o0.w), io = __float_as_uint(in.w2o1.w) + prim * 3u;
+    uint32_t i0 = __ldg(&S.indices[io]) + vo, i1 = __ldg(&S.indices[io + 1]) + vo, i2 = __ldg(&S.indices[io + 2]) + vo;
     float4 p0 = __ldg(&S.vtx[2 * i0]), n0 = __ldg(&S.vtx[2 * i0 + 1]);
     float4 p1 = __ldg(&S.vtx[2 * i1]), n1 = __ldg(&S.vtx[2 * i1 + 1]);
     float4 p2 = __ldg(&S.vtx[2 * i2]), n2 = __ldg(&S.vtx[2 * i2 + 1]);

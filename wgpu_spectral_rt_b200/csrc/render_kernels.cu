@@ -770,12 +770,10 @@ SRT_DEV VertexOut shade_vertex(const FrameArgs& a, uint32_t id, uint32_t bounce)
 
 // One bounce of every live path: shade_vertex, then the live paths, shadow
 // rays and guided vertices go to their queues (warp-aggregated slots).
-// shade_slot is one thread's vertex: queue position q of `bounce` (q >= n:
-// no vertex; the thread still takes part in the warp's queue pushes).
+// shade_slot is one thread's vertex, of path `id` (not valid: no vertex; the
+// thread still takes part in the warp's queue pushes).
 template <bool GUIDE>
-SRT_DEV void shade_slot(const FrameArgs& a, uint32_t bounce, uint32_t q, uint32_t n) {
-    bool valid = q < n;
-    uint32_t id = valid ? a.pb.queue[bounce & 1][q] : 0u;
+SRT_DEV void shade_slot(const FrameArgs& a, uint32_t bounce, uint32_t id, bool valid) {
     VertexOut v;
     if (valid) v = shade_vertex<GUIDE, false>(a, id, bounce);
     uint32_t slot = warp_push(v.alive, &a.counters->paths[bounce + 1]);
@@ -803,11 +801,51 @@ SRT_DEV void shade_slot(const FrameArgs& a, uint32_t bounce, uint32_t q, uint32_
     }
 }
 
+#ifndef SRT_SHADE_BLOCK
+#define SRT_SHADE_BLOCK 256
+#endif
+constexpr uint32_t SHADE_BLOCK = SRT_SHADE_BLOCK, SHADE_WARPS = SHADE_BLOCK / 32;
+// A block's vertices are dealt to its threads by kind of material, so that most
+// warps run one branch of shade_vertex (on config 2 from bounce 1 on, 15 of 32
+// lanes were active).  With the words a hit needs next in the instance record,
+// shading per frame: config 2 1.53 -> 1.41 ms, caustic slab 1.52 -> 1.47, others
+// within 2 %; blocks of 128 / 512: config 2 1.44, 1.46, slab 1.49, 1.53.
+constexpr uint32_t SHADE_KINDS = 4;  // ends here (no hit, emitter); diffuse; glossy; dielectric or film
+
 template <bool GUIDE>
-__global__ void __launch_bounds__(TRACE_BLOCK, SRT_SHADE_MIN_BLOCKS) k_shade(FrameArgs a, uint32_t bounce) {
-    uint32_t n = a.counters->paths[bounce];
-    if (blockIdx.x * blockDim.x >= n) return;
-    shade_slot<GUIDE>(a, bounce, blockIdx.x * blockDim.x + threadIdx.x, n);
+__global__ void __launch_bounds__(SHADE_BLOCK, SRT_SHADE_MIN_BLOCKS * TRACE_BLOCK / SHADE_BLOCK)
+    k_shade(FrameArgs a, uint32_t bounce) {
+    __shared__ uint32_t ids[SHADE_BLOCK], counts[SHADE_KINDS][SHADE_WARPS];
+    const uint32_t n = a.counters->paths[bounce];
+    const uint32_t first = blockIdx.x * SHADE_BLOCK, q = first + threadIdx.x;
+    if (first >= n) return;
+    const bool valid = q < n;
+    uint32_t id = valid ? a.pb.queue[bounce & 1][q] : 0u;
+    uint32_t kind = 0u;
+    if (valid) {
+        const uint32_t prim = __float_as_uint(a.pb.hit[id].y);
+        if (prim != MISS) {
+            const uint32_t type = __float_as_uint(a.scene.inst[__ldg(&a.scene.tri_inst[prim])].w2o2.w);
+            kind = type == 3u ? 0u : (type == 1u || type == 5u) ? 2u : (type == 2u || type == 4u) ? 3u : 1u;
+        }
+    }
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+    uint32_t mine = 0u;
+#pragma unroll
+    for (uint32_t k = 0; k < SHADE_KINDS; ++k) {
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, valid && kind == k);
+        if (lane == 0u) counts[k][warp] = (uint32_t)__popc(m);
+        if (kind == k) mine = m;
+    }
+    __syncthreads();
+    uint32_t at = __popc(mine & lt);
+    for (uint32_t k = 0; k < SHADE_KINDS; ++k)
+        for (uint32_t w = 0; w < SHADE_WARPS; ++w)
+            if (k < kind || (k == kind && w < warp)) at += counts[k][w];
+    if (valid) ids[at] = id;
+    __syncthreads();
+    if (valid) id = ids[threadIdx.x];
+    shade_slot<GUIDE>(a, bounce, id, valid);
 }
 
 // The photon gathers a bounce queued (shade_vertex): one per thread, or one
@@ -1213,11 +1251,11 @@ int launch_raygen(const FrameArgs& a, cudaStream_t st) {
 
 int launch_bounce(const FrameArgs& a, uint32_t bounce, cudaStream_t st, int stage) {
     int launches = 0;
-    uint32_t grid = blocks_for((uint64_t)a.width * a.height, TRACE_BLOCK);
+    const uint32_t grid = blocks_for((uint64_t)a.width * a.height, SHADE_BLOCK);
     if (stage == 1) launches += launch_trace_closest(a, bounce, st);
     if (stage == 2 || stage == 4) {
-        if (a.guiding) k_shade<true><<<grid, TRACE_BLOCK, 0, st>>>(a, bounce);
-        else k_shade<false><<<grid, TRACE_BLOCK, 0, st>>>(a, bounce);
+        if (a.guiding) k_shade<true><<<grid, SHADE_BLOCK, 0, st>>>(a, bounce);
+        else k_shade<false><<<grid, SHADE_BLOCK, 0, st>>>(a, bounce);
         ++launches;
         if (a.guiding && stage != 4 && bounce + 1 < a.max_depth && bounce < a.guide_bounces)
             launches += launch_guide_infer(a, bounce, st);
