@@ -121,11 +121,25 @@ SRT_DEV uint32_t pcg_hash(uint32_t input) {
     return (word >> 22u) ^ word;
 }
 // rand(): f32(u32) / 4294967295.0 — the f32 constant is 2^32, so the
-// quotient is an exact scaling of the rounded u32.
+// quotient is an exact scaling of the rounded u32, and so is the product with
+// 2^-32: the same bits without a division (config-2 frame 7.00 -> 6.90 ms,
+// caustic slab 3.88 -> 3.84).  The guide's kernels keep the division
+// (SRT_RNG_DIVIDE): they are compiled with contraction, and there the product
+// moves which multiplies the compiler fuses, so a frozen guide's image changes
+// in its last bits, and at a few pixels in its decisions.
 SRT_DEV float rng_next(uint32_t& s) {
     s = pcg_hash(s);
+#ifdef SRT_RNG_DIVIDE
     return __fdiv_rn(__uint2float_rn(s), 4294967296.0f);
+#else
+    return __fmul_rn(__uint2float_rn(s), 2.3283064365386963e-10f);
+#endif
 }
+// powf out of line: the shading kernels call it at several places, and its
+// inlined copies were a large part of the code their warps wait for (config-2
+// shading 1.40 -> 1.33 ms per frame, caustic slab 1.47 -> 1.43; blackbody4 or
+// sincosf out of line too: 1.35, 1.37).
+static __device__ __noinline__ float powf_call(float a, float b) { return powf(a, b); }
 SRT_DEV float3 random_unit_vector(uint32_t& s) {
     float u1 = rng_next(s);
     float u2 = rng_next(s);
@@ -183,7 +197,7 @@ SRT_DEV float blackbody(float lambda_nm, float temp_k) {
     const float h = 6.62607015e-34f, c = 299792458.0f, k = 1.380649e-23f;
     float c1 = 2.0f * h * c * c;
     float c2 = (h * c) / (k * temp_k);
-    return c1 / (powf(lm, 5.0f) * (expf(c2 / lm) - 1.0f)) * 1e-13f;
+    return c1 / (powf_call(lm, 5.0f) * (expf(c2 / lm) - 1.0f)) * 1e-13f;
 }
 SRT_DEV float4 blackbody4(float4 wl, float t) {
     float4 o = splat4(0.f);
@@ -233,7 +247,7 @@ SRT_DEV float4 thin_film4(float cos1, float n1, float n2, float n3, float d, flo
 SRT_DEV float schlick(float cosine, float ri) {
     float r0 = (1.0f - ri) / (1.0f + ri);
     r0 = r0 * r0;
-    return r0 + (1.0f - r0) * powf(1.0f - cosine, 5.0f);
+    return r0 + (1.0f - r0) * powf_call(1.0f - cosine, 5.0f);
 }
 SRT_DEV float g1_schlick_ggx(float nv, float r) {  // shader.wgsl:207-213
     float k = (r * r) / 2.0f;
@@ -287,7 +301,7 @@ SRT_DEV Scatter sample_bsdf(float3 r_dir, float3 ffn, float4 color, float4 extra
             float vh = fmaxf(dot(v, h), 0.0f);
             float4 F;
             if (type == 1u) {
-                float p = powf(clampf(1.0f - vh, 0.0f, 1.0f), 5.0f);
+                float p = powf_call(clampf(1.0f - vh, 0.0f, 1.0f), 5.0f);
                 F = spec + (splat4(1.0f) - spec) * p;
             } else {
                 F = thin_film4(vh, 1.0f, extra.z, extra.w, fmaxf(extra.y, 50.0f), wl);
@@ -1219,9 +1233,9 @@ SRT_DEV bool group_init(GroupTrav<STACK>& T, const DevScene& S, float3 o, float3
 }
 
 // One node visit and its triangles for the groups with `active` set; true
-// when the group's ray is finished (ANY: at its first hit).
-template <bool ANY, int STACK>
-SRT_DEV bool group_step(const DevScene& S, GroupTrav<STACK>& T, bool active, uint32_t* err, uint32_t& n_nodes,
+// when the group's ray is finished (`any`, the same in the warp: at its first hit).
+template <int STACK>
+SRT_DEV bool group_step(const DevScene& S, GroupTrav<STACK>& T, bool active, bool any, uint32_t* err, uint32_t& n_nodes,
                         uint32_t& n_tris) {
     constexpr uint32_t FULL = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31u, c = lane & 7u, shift = lane & 24u;
@@ -1331,7 +1345,7 @@ SRT_DEV bool group_step(const DevScene& S, GroupTrav<STACK>& T, bool active, uin
             }
         }
     }
-    if (ANY) {
+    if (any) {
         if ((__ballot_sync(FULL, active && T.id != MISS) >> shift) & 0xFFu) fin = true;
     } else {
         float t = fminf(T.t, T.tbest);

@@ -19,6 +19,7 @@
 #include <cmath>
 #include <vector>
 
+#define SRT_RNG_DIVIDE
 #include "guide.cuh"
 #include "render_kernels.h"
 #include "umma.cuh"

@@ -937,69 +937,83 @@ __global__ void __launch_bounds__(TRACE_BLOCK, SRT_TAIL_MIN_BLOCKS) k_tail(Frame
             }
         }
         if (__ballot_sync(FULL, live) == 0u) break;  // exhausted: a fetch that gave no path was past the end
-        // closest hits
-        uint32_t nodes = 0u, tris = 0u;
-        T.id = MISS;
-        bool act = false;
-        if (live) {
-            if (b > first && c == 0u) atomicAdd(&n_closest[b], 1u);  // paths[first] was counted by the last shading step
-            const float4 o = a.pb.ray_o[id], d = a.pb.ray_d[id];
-            act = group_init(T, a.scene, xyz(o), xyz(d), o.w, d.w);
-        }
-        while (__any_sync(FULL, act))
-            if (group_step<false>(a.scene, T, act, a.err, nodes, tris)) act = false;
-        float t, u, v;
-        uint32_t prim;
-        group_closest(T, t, prim, u, v);
-        if (COUNT && live) {
-            atomicAdd(&a.stats->nodes_bounce[TRAV_CLOSEST][b], (unsigned long long)nodes);
-            atomicAdd(&a.stats->tris_bounce[TRAV_CLOSEST][b], (unsigned long long)tris);
-        }
-        // shading
+        // two rays per bounce through one copy of the traversal: the closest
+        // hit, then (after shading) the shadow ray.  A warp runs this loop's
+        // code once per bounce and waits for it: with a copy for each ray the
+        // kernel took 0.201 vs 0.174 ms on config 2, 0.176 vs 0.146 on the caustic
+        // slab, 0.117 vs 0.100 on config 1.
         VertexOut vo;
-        if (live && c == 0u) {
-            a.pb.hit[id] = prim != MISS ? make_float4(t, __uint_as_float(prim), u, v)
-                                        : make_float4(0.f, __uint_as_float(MISS), 0.f, 0.f);
-            vo = shade_vertex<GUIDE, true>(a, id, b);
-        }
-        __syncwarp();  // the path's next ray, written by the group's first lane, is read by all
-        if (__any_sync(FULL, vo.gather)) {
-            const bool ga = __shfl_sync(FULL, (int)vo.gather, (int)shift) != 0;
-            const uint2 range = make_uint2(__shfl_sync(FULL, vo.ga_range.x, (int)shift),
-                                           __shfl_sync(FULL, vo.ga_range.y, (int)shift));
-            const float3 p = f3(__shfl_sync(FULL, vo.ga_p.x, (int)shift), __shfl_sync(FULL, vo.ga_p.y, (int)shift),
-                                __shfl_sync(FULL, vo.ga_p.z, (int)shift));
-            const float3 nn = f3(__shfl_sync(FULL, vo.ga_n.x, (int)shift), __shfl_sync(FULL, vo.ga_n.y, (int)shift),
-                                 __shfl_sync(FULL, vo.ga_n.z, (int)shift));
-            const float4 gl = gather_group(a.gather, a.counters->gather, ga, range, p, nn,
-                                           ga ? a.pb.wl[id] : splat4(0.f));
-            if (ga && c == 0u) a.pb.rad[id] = a.pb.rad[id] + vo.ga_f * gl;
-        }
-        const uint32_t alive = __ballot_sync(FULL, vo.alive), shadow = __ballot_sync(FULL, vo.shadow);
-        if (shadow) {
-            const float3 so = f3(__shfl_sync(FULL, vo.sh_o.x, (int)shift), __shfl_sync(FULL, vo.sh_o.y, (int)shift),
-                                 __shfl_sync(FULL, vo.sh_o.z, (int)shift));
-            const float3 sd = f3(__shfl_sync(FULL, vo.sh_d.x, (int)shift), __shfl_sync(FULL, vo.sh_d.y, (int)shift),
-                                 __shfl_sync(FULL, vo.sh_d.z, (int)shift));
-            const float smax = __shfl_sync(FULL, vo.sh_tmax, (int)shift);
-            const bool has = ((shadow >> shift) & 1u) != 0u;
-            nodes = tris = 0u;
-            T.id = MISS;
-            act = has && group_init(T, a.scene, so, sd, 0.001f, smax);
-            while (__any_sync(FULL, act))
-                if (group_step<true>(a.scene, T, act, a.err, nodes, tris)) act = false;
-            const bool occluded = group_occluded(T);
-            if (has && c == 0u) {
-                atomicAdd(&n_shadow[b], 1u);
-                if (!occluded) {  // as the shadow-ray kernel adds it (shader.wgsl:659-669)
-                    const float4 r = a.pb.rad[id], k = vo.sh_c;
-                    a.pb.rad[id] = make_float4(__fadd_rn(r.x, k.x), __fadd_rn(r.y, k.y), __fadd_rn(r.z, k.z),
-                                               __fadd_rn(r.w, k.w));
+        uint32_t alive = 0u;
+#pragma unroll 1
+        for (int ray = 0; ray < 2; ++ray) {
+            uint32_t nodes = 0u, tris = 0u;
+            float3 ro = f3(0.f, 0.f, 0.f), rd = ro;
+            float rmin = 0.001f, rmax = 0.f;
+            bool has = live;
+            if (ray == 0) {
+                if (live) {
+                    // paths[first] was counted by the last shading step
+                    if (b > first && c == 0u) atomicAdd(&n_closest[b], 1u);
+                    const float4 o = a.pb.ray_o[id], d = a.pb.ray_d[id];
+                    ro = xyz(o);
+                    rd = xyz(d);
+                    rmin = o.w;
+                    rmax = d.w;
                 }
+            } else {
+                const uint32_t shadow = __ballot_sync(FULL, vo.shadow);
+                if (shadow == 0u) break;
+                ro = f3(__shfl_sync(FULL, vo.sh_o.x, (int)shift), __shfl_sync(FULL, vo.sh_o.y, (int)shift),
+                        __shfl_sync(FULL, vo.sh_o.z, (int)shift));
+                rd = f3(__shfl_sync(FULL, vo.sh_d.x, (int)shift), __shfl_sync(FULL, vo.sh_d.y, (int)shift),
+                        __shfl_sync(FULL, vo.sh_d.z, (int)shift));
+                rmax = __shfl_sync(FULL, vo.sh_tmax, (int)shift);
+                has = ((shadow >> shift) & 1u) != 0u;
             }
+            T.id = MISS;
+            bool act = has && group_init(T, a.scene, ro, rd, rmin, rmax);
+            while (__any_sync(FULL, act))
+                if (group_step(a.scene, T, act, ray == 1, a.err, nodes, tris)) act = false;
             if (COUNT && has) {
-                atomicAdd(&a.stats->nodes_bounce[TRAV_SHADOW][b], (unsigned long long)nodes);
-                atomicAdd(&a.stats->tris_bounce[TRAV_SHADOW][b], (unsigned long long)tris);
+                const int kind = ray == 0 ? TRAV_CLOSEST : TRAV_SHADOW;
+                atomicAdd(&a.stats->nodes_bounce[kind][b], (unsigned long long)nodes);
+                atomicAdd(&a.stats->tris_bounce[kind][b], (unsigned long long)tris);
+            }
+            if (ray == 0) {
+                float t, u, v;
+                uint32_t prim;
+                group_closest(T, t, prim, u, v);
+                if (live && c == 0u) {
+                    a.pb.hit[id] = prim != MISS ? make_float4(t, __uint_as_float(prim), u, v)
+                                                : make_float4(0.f, __uint_as_float(MISS), 0.f, 0.f);
+                    vo = shade_vertex<GUIDE, true>(a, id, b);
+                }
+                __syncwarp();  // the path's next ray, written by the group's first lane, is read by all
+                alive = __ballot_sync(FULL, vo.alive);
+                if (__any_sync(FULL, vo.gather)) {
+                    const bool ga = __shfl_sync(FULL, (int)vo.gather, (int)shift) != 0;
+                    const uint2 range = make_uint2(__shfl_sync(FULL, vo.ga_range.x, (int)shift),
+                                                   __shfl_sync(FULL, vo.ga_range.y, (int)shift));
+                    const float3 p =
+                        f3(__shfl_sync(FULL, vo.ga_p.x, (int)shift), __shfl_sync(FULL, vo.ga_p.y, (int)shift),
+                           __shfl_sync(FULL, vo.ga_p.z, (int)shift));
+                    const float3 nn =
+                        f3(__shfl_sync(FULL, vo.ga_n.x, (int)shift), __shfl_sync(FULL, vo.ga_n.y, (int)shift),
+                           __shfl_sync(FULL, vo.ga_n.z, (int)shift));
+                    const float4 gl = gather_group(a.gather, a.counters->gather, ga, range, p, nn,
+                                                   ga ? a.pb.wl[id] : splat4(0.f));
+                    if (ga && c == 0u) a.pb.rad[id] = a.pb.rad[id] + vo.ga_f * gl;
+                }
+            } else {
+                const bool occluded = group_occluded(T);
+                if (has && c == 0u) {
+                    atomicAdd(&n_shadow[b], 1u);
+                    if (!occluded) {  // as the shadow-ray kernel adds it (shader.wgsl:659-669)
+                        const float4 r = a.pb.rad[id], k = vo.sh_c;
+                        a.pb.rad[id] = make_float4(__fadd_rn(r.x, k.x), __fadd_rn(r.y, k.y), __fadd_rn(r.z, k.z),
+                                                   __fadd_rn(r.w, k.w));
+                    }
+                }
             }
         }
         if (vo.dark) atomicAdd(&n_shadow[b], 1u);

@@ -171,7 +171,7 @@ SRT_DEV void trace_groups(const DevScene& S, const uint32_t* queue, uint32_t n, 
             if (exhausted) break;
             continue;
         }
-        fin = group_step<ANY>(S, T, active && !fin, err, n_nodes, n_tris) || fin;
+        fin = group_step(S, T, active && !fin, ANY, err, n_nodes, n_tris) || fin;
         if (__any_sync(FULL, fin)) {
             if (ANY) {
                 const bool occluded = group_occluded(T);
