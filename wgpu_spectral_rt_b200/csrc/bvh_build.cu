@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "bvh_build.h"
+#include "dev_arena.h"
 #include "radix_sort.cuh"
 
 namespace srt {
@@ -999,11 +1000,6 @@ __global__ void k_collapse(Bvh2 b, const uint2* __restrict__ qin, uint32_t n_in,
     nodes[q.y] = nd;
 }
 
-template <typename T>
-cudaError_t dalloc(T** p, size_t count) {
-    return cudaMalloc((void**)p, sizeof(T) * (count ? count : 1));
-}
-
 }  // namespace
 
 cudaError_t build_bvh8(const BvhInputs& in, cudaStream_t st, BvhOutputs* out, std::string* msg) {
@@ -1011,6 +1007,8 @@ cudaError_t build_bvh8(const BvhInputs& in, cudaStream_t st, BvhOutputs* out, st
     out->nodes = nullptr;
     out->tris = nullptr;
     out->tri_inst = nullptr;
+    out->scatter = nullptr;
+    out->mem = nullptr;
     out->n_nodes = 0;
     out->depth = 0;
     out->kernel_launches = 0;
@@ -1031,32 +1029,48 @@ cudaError_t build_bvh8(const BvhInputs& in, cudaStream_t st, BvhOutputs* out, st
     SahTask* sah_tasks[2] = {nullptr, nullptr};
     uint32_t* sah_bins = nullptr;
     Bvh2 b{};
+    // two allocations instead of 30: opening a scene of 331k triangles spent
+    // most of its 32 ms in cudaMalloc and cudaFree
+    DevArena kept, tmp;
     if (n == 0) return cudaSuccess;
     {
-        CK(dalloc(&out->tri_inst, n));
-        CK(dalloc(&out->tris, n));
-        uint32_t node_cap = n > 1 ? n - 1 : 1;
-        CK(dalloc(&out->nodes, node_cap));
-        CK(dalloc(&flat, n));
-        CK(dalloc(&cen, n));
-        CK(dalloc(&bounds, 6));
-        CK(dalloc(&keys, n));
-        CK(dalloc(&vals, n));
-        CK(dalloc(&keys2, n));
-        CK(dalloc(&vals2, n));
-        CK(dalloc(&scratch, radix_scratch_words(n)));
-        CK(dalloc(&counters, 4));
-        CK(dalloc(&err, 1));
-        CK(dalloc(&qa, node_cap));
-        CK(dalloc(&qb, node_cap));
-        CK(dalloc(&b.inode, node_cap));
-        CK(dalloc(&b.ibox, 2 * (size_t)node_cap));
-        CK(dalloc(&b.lbox, 2 * (size_t)n));
-        CK(dalloc(&b.iparent, node_cap));
-        CK(dalloc(&b.lparent, n));
-        CK(dalloc(&b.flags, node_cap));
-        CK(dalloc(&b.cost, 2 * (size_t)node_cap));
-        CK(dalloc(&b.choice, node_cap));
+        const uint32_t node_cap = n > 1 ? n - 1 : 1;
+        kept.add(&out->tri_inst, n);
+        kept.add(&out->tris, n);
+        kept.add(&out->nodes, node_cap);
+        kept.add(&out->scatter, node_cap);
+        CK(kept.commit());
+        tmp.add(&flat, n);
+        tmp.add(&cen, n);
+        tmp.add(&bounds, 6);
+        tmp.add(&keys, n);
+        tmp.add(&vals, n);
+        tmp.add(&keys2, n);
+        tmp.add(&vals2, n);
+        tmp.add(&scratch, radix_scratch_words(n));
+        tmp.add(&counters, 4);
+        tmp.add(&err, 1);
+        tmp.add(&qa, node_cap);
+        tmp.add(&qb, node_cap);
+        tmp.add(&b.inode, node_cap);
+        tmp.add(&b.ibox, 2 * (size_t)node_cap);
+        tmp.add(&b.lbox, 2 * (size_t)n);
+        tmp.add(&b.iparent, node_cap);
+        tmp.add(&b.lparent, n);
+        tmp.add(&b.flags, node_cap);
+        tmp.add(&b.cost, 2 * (size_t)node_cap);
+        tmp.add(&b.choice, node_cap);
+        const bool sah = in.builder != BVH_BUILDER_LBVH && n >= 2;
+        const uint32_t task_cap = n / 2 + 1;
+        // tasks that bin in global memory hold more than SAH_SMALL primitives
+        // of disjoint ranges: at most n / (SAH_SMALL + 1) per level
+        const uint32_t bin_cap = n / (SAH_SMALL + 1) + 1;
+        if (sah) {
+            tmp.add(&sah_tasks[0], task_cap);
+            tmp.add(&sah_tasks[1], task_cap);
+            tmp.add(&sah_bins, (size_t)bin_cap * SAH_TASK_WORDS);
+        }
+        CK(tmp.commit());
         uint32_t init_bounds[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
         CK(cudaMemcpyAsync(bounds, init_bounds, sizeof(init_bounds), cudaMemcpyHostToDevice, st));
         CK(cudaMemsetAsync(b.flags, 0, sizeof(uint32_t) * node_cap, st));
@@ -1067,7 +1081,7 @@ cudaError_t build_bvh8(const BvhInputs& in, cudaStream_t st, BvhOutputs* out, st
                                       out->tri_inst, cen, bounds);
         ++out->kernel_launches;
         uint32_t* sv = nullptr;
-        if (in.builder == BVH_BUILDER_LBVH || n < 2) {
+        if (!sah) {
             k_morton<<<grid, B, 0, st>>>(cen, bounds, n, keys, vals);
             ++out->kernel_launches;
             uint32_t* sk;
@@ -1081,13 +1095,6 @@ cudaError_t build_bvh8(const BvhInputs& in, cudaStream_t st, BvhOutputs* out, st
             // permutation and position -> task ping-pong buffers)
             uint32_t *perm = keys, *perm2 = keys2;
             int *pt = (int*)vals, *pt2 = (int*)vals2;
-            const uint32_t task_cap = n / 2 + 1;
-            // tasks that bin in global memory hold more than SAH_SMALL primitives
-            // of disjoint ranges: at most n / (SAH_SMALL + 1) per level
-            const uint32_t bin_cap = n / (SAH_SMALL + 1) + 1;
-            CK(dalloc(&sah_tasks[0], task_cap));
-            CK(dalloc(&sah_tasks[1], task_cap));
-            CK(dalloc(&sah_bins, (size_t)bin_cap * SAH_TASK_WORDS));
             // counters: node alloc, -, next tasks, bin slots of the next level
             CK(cudaMemcpyAsync(counters, std::array<uint32_t, 4>{1u, 0u, 0u, 0u}.data(), 16, cudaMemcpyHostToDevice, st));
             k_sah_root<<<grid, B, 0, st>>>(bounds, n, sah_tasks[0], pt, perm, counters + 3, bin_cap);
@@ -1170,36 +1177,14 @@ cudaError_t build_bvh8(const BvhInputs& in, cudaStream_t st, BvhOutputs* out, st
         out->depth = depth;
     }
 done:
-    cudaFree(sah_tasks[0]);
-    cudaFree(sah_tasks[1]);
-    cudaFree(sah_bins);
-    cudaFree(flat);
-    cudaFree(cen);
-    cudaFree(bounds);
-    cudaFree(keys);
-    cudaFree(vals);
-    cudaFree(keys2);
-    cudaFree(vals2);
-    cudaFree(scratch);
-    cudaFree(counters);
-    cudaFree(err);
-    cudaFree(qa);
-    cudaFree(qb);
-    cudaFree(b.inode);
-    cudaFree(b.ibox);
-    cudaFree(b.lbox);
-    cudaFree(b.iparent);
-    cudaFree(b.lparent);
-    cudaFree(b.flags);
-    cudaFree(b.cost);
-    cudaFree(b.choice);
+    out->mem = kept.detach();
     if (e != cudaSuccess) {
-        cudaFree(out->nodes);
-        cudaFree(out->tris);
-        cudaFree(out->tri_inst);
+        cudaFree(out->mem);
+        out->mem = nullptr;
         out->nodes = nullptr;
         out->tris = nullptr;
         out->tri_inst = nullptr;
+        out->scatter = nullptr;
     }
 #undef CK
     return e;

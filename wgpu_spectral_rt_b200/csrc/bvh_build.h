@@ -49,14 +49,16 @@ struct BvhOutputs {
     Node8* nodes;        // device, n_nodes entries (node 0 = root)
     TriSlot* tris;       // device, n_tris leaf slots
     uint32_t* tri_inst;  // device, flattened triangle -> instance
+    uint8_t* scatter;    // device, room for one byte per node (launch_scatter_masks)
+    void* mem;           // the allocation that holds the four arrays
     uint32_t n_nodes;
     uint32_t depth;      // number of 8-wide levels
     int kernel_launches;
     uint32_t level_start[66];  // nodes of level L: [level_start[L], level_start[L + 1]), L < depth
 };
 
-// Builds the tree on `st` (synchronising it); device memory in `out` is
-// owned by the caller afterwards (cudaFree).
+// Builds the tree on `st` (synchronising it); the arrays in
+// `out` are owned by the caller afterwards (cudaFree of out->mem).
 cudaError_t build_bvh8(const BvhInputs& in, cudaStream_t st, BvhOutputs* out, std::string* msg);
 
 // Per node, the child slots whose subtree holds a triangle of a material that

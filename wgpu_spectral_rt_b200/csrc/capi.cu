@@ -10,11 +10,13 @@
 #include <algorithm>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
 
 #include "bvh_build.h"
+#include "dev_arena.h"
 #include "host_scene.h"
 #include "radix_sort.cuh"
 #include "render_kernels.h"
@@ -33,6 +35,17 @@ bool env_fault(const char* what) {
 }  // namespace
 
 struct srt_ctx {
+    // One workspace kept between calls that bring their own data
+    // (srt_trace_rays), up to WORK_KEEP bytes; a call takes it out while it runs,
+    // so that a second thread's call finds none and allocates its own (250k ray
+    // queries from host arrays 2.55 -> 1.2 ms).
+    static constexpr size_t WORK_KEEP = 64ull << 20;
+    struct Work {
+        void* p = nullptr;
+        size_t bytes = 0;
+    };
+    std::mutex work_mutex;
+    Work work;
     int device = 0;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
@@ -54,6 +67,7 @@ void ctx_free(srt_ctx* c) {
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     cudaFree(c->d_err);
+    cudaFree(c->work.p);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
 }
@@ -80,11 +94,46 @@ srt_status cuda_fail(srt_ctx* c, cudaError_t e, const char* where) {
         if (_e != cudaSuccess) return cuda_fail(ctx, _e, #expr); \
     } while (0)
 
+cudaError_t dev_commit(DevArena& a) {
+    if (env_fault("alloc")) return cudaErrorMemoryAllocation;
+    return a.commit();
+}
 template <typename T>
 cudaError_t dev_alloc(T** p, size_t count) {
     if (env_fault("alloc")) return cudaErrorMemoryAllocation;
     return cudaMalloc((void**)p, sizeof(T) * (count ? count : 1));
 }
+
+// The context's workspace, or an allocation of this call: `bytes` at get().
+// The call synchronises the stream before the workspace goes back.
+struct CallWork {
+    srt_ctx* c;
+    srt_ctx::Work w;
+    explicit CallWork(srt_ctx* ctx) : c(ctx) {
+        std::lock_guard<std::mutex> lock(c->work_mutex);
+        std::swap(w, c->work);
+    }
+    CallWork(const CallWork&) = delete;
+    ~CallWork() {
+        if (w.bytes <= srt_ctx::WORK_KEEP) {
+            std::lock_guard<std::mutex> lock(c->work_mutex);
+            if (c->work.bytes < w.bytes) std::swap(w, c->work);
+        }
+        cudaFree(w.p);
+    }
+    cudaError_t get(void** p, size_t bytes) {
+        if (env_fault("alloc")) return cudaErrorMemoryAllocation;
+        if (w.bytes < bytes) {
+            cudaFree(w.p);
+            w = srt_ctx::Work{};
+            const cudaError_t e = cudaMalloc(&w.p, bytes);
+            if (e != cudaSuccess) return e;
+            w.bytes = bytes;
+        }
+        *p = w.p;
+        return cudaSuccess;
+    }
+};
 
 // Reads and clears a device error word.
 srt_status check_device_error(srt_ctx* c, uint32_t* d_err) {
@@ -314,7 +363,7 @@ struct srt_scene {
     InstDev* inst = nullptr;
     InstFwd* fwd = nullptr;
     BvhOutputs bvh{};
-    uint8_t* scatter = nullptr;  // scatter masks of bvh's nodes (launch_scatter_masks)
+    DevArena mem, refit_mem;  // the arrays above; those of an instance update
     DevScene dev{};
     uint64_t n_tris = 0;
     uint32_t n_lights = 0;
@@ -337,35 +386,8 @@ struct srt_scene {
     int width = 8;
     uint32_t leaf = 2;  // triangles of the largest leaf (rebuilds keep it)
     uint32_t n_inst = 0;
-    ~srt_scene() {
-        cudaFree(light_insts);
-        cudaFree(moved);
-        cudaFree(refit_aux);
-        cudaFree(refit_err);
-        cudaFree(vtx);
-        cudaFree(idx);
-        cudaFree(mesh_infos);
-        cudaFree(materials);
-        cudaFree(lights);
-        cudaFree(light_frames);
-        cudaFree(inst);
-        cudaFree(fwd);
-        cudaFree(bvh.nodes);
-        cudaFree(bvh.tris);
-        cudaFree(bvh.tri_inst);
-        cudaFree(scatter);
-    }
+    ~srt_scene() { cudaFree(bvh.mem); }
 };
-
-namespace {
-template <typename T>
-cudaError_t upload(T** dst, const void* src, size_t bytes, size_t alloc_bytes, cudaStream_t st) {
-    cudaError_t e = dev_alloc((char**)dst, alloc_bytes ? alloc_bytes : 16);
-    if (e != cudaSuccess) return e;
-    if (bytes) e = cudaMemcpyAsync(*dst, src, bytes, cudaMemcpyHostToDevice, st);
-    return e;
-}
-}  // namespace
 
 namespace {
 // World-to-object rows (FP64 inverse of the 3x3 part) and object-to-world
@@ -455,14 +477,36 @@ srt_status scene_build_impl(srt_ctx* c, const srt_scene_arrays* a,
     if (!s) return SRT_ERR_OOM;
     s->ctx = c;
     cudaStream_t st = c->stream;
-    CUDA_TRY(c, upload(&s->vtx, a->vertices, sizeof(srt_vertex) * a->n_vertices, sizeof(srt_vertex) * a->n_vertices, st));
-    CUDA_TRY(c, upload(&s->idx, a->indices, 4ull * a->n_indices, 4ull * a->n_indices, st));
-    CUDA_TRY(c, upload(&s->mesh_infos, a->mesh_infos, 16ull * a->n_meshes, 16ull * a->n_meshes, st));
-    CUDA_TRY(c, upload(&s->materials, a->materials, 32ull * a->n_materials, 32ull * a->n_materials, st));
-    CUDA_TRY(c, upload(&s->lights, a->lights, 64ull * a->n_lights, 64ull * a->n_lights, st));
-    CUDA_TRY(c, dev_alloc(&s->light_frames, a->n_lights));
-    CUDA_TRY(c, upload(&s->inst, inst.data(), sizeof(InstDev) * inst.size(), sizeof(InstDev) * inst.size(), st));
-    CUDA_TRY(c, upload(&s->fwd, fwd.data(), sizeof(InstFwd) * fwd.size(), sizeof(InstFwd) * fwd.size(), st));
+    std::vector<LightInst> li;
+    if (light_instances)
+        for (const srt_light_instance_rec& r : *light_instances) {
+            if (r.instance >= a->n_instances || (uint64_t)r.first_light + r.count > a->n_lights ||
+                r.count != mesh_tris[a->instances[r.instance].mesh_id])
+                return fail(c, SRT_ERR_INVALID_ARG, "light instance record out of range");
+            li.push_back(LightInst{r.instance, r.first_light, r.count, 0u,
+                                   make_float4(r.params[0], r.params[1], r.params[2], r.params[3])});
+        }
+    s->mem.add(&s->vtx, sizeof(srt_vertex) / sizeof(float4) * a->n_vertices);
+    s->mem.add(&s->idx, a->n_indices);
+    s->mem.add(&s->mesh_infos, a->n_meshes);
+    s->mem.add(&s->materials, 2ull * a->n_materials);
+    s->mem.add(&s->lights, 4ull * a->n_lights);
+    s->mem.add(&s->light_frames, a->n_lights);
+    s->mem.add(&s->inst, inst.size());
+    s->mem.add(&s->fwd, fwd.size());
+    if (!li.empty()) s->mem.add(&s->light_insts, li.size());
+    CUDA_TRY(c, dev_commit(s->mem));
+    auto upload = [st](void* dst, const void* src, size_t bytes) {
+        return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st) : cudaSuccess;
+    };
+    CUDA_TRY(c, upload(s->vtx, a->vertices, sizeof(srt_vertex) * a->n_vertices));
+    CUDA_TRY(c, upload(s->idx, a->indices, 4ull * a->n_indices));
+    CUDA_TRY(c, upload(s->mesh_infos, a->mesh_infos, 16ull * a->n_meshes));
+    CUDA_TRY(c, upload(s->materials, a->materials, 32ull * a->n_materials));
+    CUDA_TRY(c, upload(s->lights, a->lights, 64ull * a->n_lights));
+    CUDA_TRY(c, upload(s->inst, inst.data(), sizeof(InstDev) * inst.size()));
+    CUDA_TRY(c, upload(s->fwd, fwd.data(), sizeof(InstFwd) * fwd.size()));
+    if (!li.empty()) CUDA_TRY(c, upload(s->light_insts, li.data(), sizeof(LightInst) * li.size()));
     BvhInputs bi{s->vtx, s->idx, s->mesh_infos, s->inst, s->fwd, a->n_instances, (uint32_t)total,
                  c->bvh_builder == SRT_BVH_LBVH ? BVH_BUILDER_LBVH : BVH_BUILDER_SAH, c->bvh_width, c->bvh_leaf};
     s->builder = bi.builder;
@@ -474,8 +518,7 @@ srt_status scene_build_impl(srt_ctx* c, const srt_scene_arrays* a,
     if (e != cudaSuccess) return fail(c, e == cudaErrorMemoryAllocation ? SRT_ERR_OOM : SRT_ERR_CUDA, "BVH build: " + msg);
     if (s->bvh.depth > (uint32_t)TRAV_STACK)
         return fail(c, SRT_ERR_UNSUPPORTED, "BVH deeper than the traversal stack");
-    CUDA_TRY(c, dev_alloc(&s->scatter, s->bvh.n_nodes));
-    launch_scatter_masks(s->bvh, s->inst, s->materials, s->scatter, st);
+    launch_scatter_masks(s->bvh, s->inst, s->materials, s->bvh.scatter, st);
     CUDA_TRY(c, cudaGetLastError());
     CUDA_TRY(c, cudaStreamSynchronize(st));
     s->n_tris = total;
@@ -492,7 +535,7 @@ srt_status scene_build_impl(srt_ctx* c, const srt_scene_arrays* a,
     d.tri_inst = s->bvh.tri_inst;
     d.nodes = s->bvh.nodes;
     d.tris = s->bvh.tris;
-    d.scatter = s->scatter;
+    d.scatter = s->bvh.scatter;
     d.n_nodes = s->bvh.n_nodes;
     d.n_tris = (uint32_t)total;
     d.depth = s->bvh.depth;
@@ -530,19 +573,9 @@ srt_status scene_build_impl(srt_ctx* c, const srt_scene_arrays* a,
     s->h_inst.assign(a->instances, a->instances + a->n_instances);
     s->h_mesh_tris = mesh_tris;
     s->h_instdev = inst;
-    if (light_instances && !light_instances->empty()) {
+    if (!li.empty()) {
         // scene-side GPU ingestion: the light instances' triangles are
         // expanded to world space on the device (builder.rs:101-129)
-        std::vector<LightInst> li;
-        for (const srt_light_instance_rec& r : *light_instances) {
-            if (r.instance >= a->n_instances || (uint64_t)r.first_light + r.count > a->n_lights ||
-                r.count != mesh_tris[a->instances[r.instance].mesh_id])
-                return fail(c, SRT_ERR_INVALID_ARG, "light instance record out of range");
-            LightInst L{r.instance, r.first_light, r.count, 0u,
-                        make_float4(r.params[0], r.params[1], r.params[2], r.params[3])};
-            li.push_back(L);
-        }
-        CUDA_TRY(c, upload(&s->light_insts, li.data(), sizeof(LightInst) * li.size(), sizeof(LightInst) * li.size(), st));
         s->n_light_insts = (uint32_t)li.size();
         launch_expand_lights(s->light_insts, s->n_light_insts, nullptr, s->vtx, s->idx, s->mesh_infos, s->inst, s->fwd,
                              s->lights, st);
@@ -582,9 +615,11 @@ extern "C" srt_status srt_scene_update_instances(srt_scene* s, const uint32_t* i
         if (!instance_rows(in, &nd[k], &nf[k])) return fail(c, SRT_ERR_INVALID_ARG, "instance transform is singular");
     }
     if (!s->moved) {
-        CUDA_TRY(c, dev_alloc(&s->moved, ni));
-        CUDA_TRY(c, dev_alloc(&s->refit_aux, 2ull * std::max(1u, s->bvh.n_nodes)));
-        CUDA_TRY(c, dev_alloc(&s->refit_err, 1));
+        s->refit_mem.release();
+        s->refit_mem.add(&s->moved, ni);
+        s->refit_mem.add(&s->refit_aux, 2ull * std::max(1u, s->bvh.n_nodes));
+        s->refit_mem.add(&s->refit_err, 1);
+        CUDA_TRY(c, dev_commit(s->refit_mem));
     }
     std::vector<uint8_t> moved(ni, 0);
     CUDA_TRY(c, cudaStreamSynchronize(st));  // frames in flight read the instances
@@ -675,30 +710,19 @@ extern "C" srt_status srt_scene_rebuild_bvh(srt_scene* s, uint32_t width) {
         e = cudaErrorInvalidValue;
         msg = "BVH deeper than the traversal stack";
     }
-    uint8_t* scatter = nullptr;
-    if (e == cudaSuccess) e = dev_alloc(&scatter, nb.n_nodes);
     if (e == cudaSuccess) {
-        launch_scatter_masks(nb, s->inst, s->materials, scatter, st);
+        launch_scatter_masks(nb, s->inst, s->materials, nb.scatter, st);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
-        cudaFree(nb.nodes);
-        cudaFree(nb.tris);
-        cudaFree(nb.tri_inst);
-        cudaFree(scatter);
+        cudaFree(nb.mem);
         return fail(c, e == cudaErrorMemoryAllocation ? SRT_ERR_OOM : SRT_ERR_CUDA, "BVH rebuild: " + msg);
     }
-    cudaFree(s->bvh.nodes);
-    cudaFree(s->bvh.tris);
-    cudaFree(s->bvh.tri_inst);
-    cudaFree(s->scatter);
+    cudaFree(s->bvh.mem);
     s->bvh = nb;
-    s->scatter = scatter;
     // refit scratch is sized by the node count: allocated again on the next update
-    cudaFree(s->moved);
-    cudaFree(s->refit_aux);
-    cudaFree(s->refit_err);
+    s->refit_mem.release();
     s->moved = nullptr;
     s->refit_aux = nullptr;
     s->refit_err = nullptr;
@@ -707,7 +731,7 @@ extern "C" srt_status srt_scene_rebuild_bvh(srt_scene* s, uint32_t width) {
     d.tri_inst = s->bvh.tri_inst;
     d.nodes = s->bvh.nodes;
     d.tris = s->bvh.tris;
-    d.scatter = s->scatter;
+    d.scatter = s->bvh.scatter;
     d.n_nodes = s->bvh.n_nodes;
     d.depth = s->bvh.depth;
     s->gen += 1;
@@ -772,6 +796,8 @@ struct srt_renderer {
     srt_params p{};
     FrameArgs args{};
     srt_camera_uniform* cam_dev = nullptr;
+    DevArena mem, pipe_mem;  // all device arrays; the pipelined photon pass's (ensure_pipe)
+    void* pinned = nullptr;  // the allocation of cam_ring, ph_ring and counts_host
     srt_camera_uniform* cam_ring = nullptr;  // pinned staging
     cudaEvent_t ring_ev[4] = {};
     int ring_i = 0;
@@ -864,7 +890,7 @@ struct srt_renderer {
     const FrameCounters* last_photon_counters() const { return last_set >= 0 ? pipe[last_set].counters : counters; }
     const float4* last_photons() const { return last_set >= 0 ? pipe[last_set].photons : ph.photons; }
     // The second photon set, both sets' counters and uniforms, the photon
-    // branch's stream and events, the pinned staging (once).
+    // branch's stream and events (once).
     cudaError_t ensure_pipe() {
         if (pipe_alloc) return cudaSuccess;
         cudaError_t e;
@@ -872,16 +898,21 @@ struct srt_renderer {
         pipe[0].photons = ph.photons;
         pipe[0].sorted = ph.sorted;
         pipe[0].ranges = ph.ranges;
-        if ((e = dev_alloc(&pipe[1].photons, 2ull * cap)) != cudaSuccess) return e;
-        if ((e = dev_alloc(&pipe[1].sorted, 2ull * cap)) != cudaSuccess) return e;
-        if ((e = dev_alloc(&pipe[1].ranges, range_entries(p.hash_bits))) != cudaSuccess) return e;
-        if ((e = cudaMemset(pipe[1].ranges, 0, sizeof(uint2) * range_entries(p.hash_bits))) != cudaSuccess) return e;
+        pipe_mem.release();  // an earlier call may have failed half way
+        pipe_mem.add(&pipe[1].photons, 2ull * cap);
+        pipe_mem.add(&pipe[1].sorted, 2ull * cap);
+        pipe_mem.add(&pipe[1].ranges, range_entries(p.hash_bits));
         for (auto& ps : pipe) {
-            if ((e = dev_alloc(&ps.counters, 1)) != cudaSuccess) return e;
-            if ((e = cudaMemset(ps.counters, 0, sizeof(FrameCounters))) != cudaSuccess) return e;
-            if ((e = dev_alloc(&ps.cam, 1)) != cudaSuccess) return e;
+            pipe_mem.add(&ps.counters, 1);
+            pipe_mem.add(&ps.cam, 1);
         }
-        if ((e = cudaMallocHost((void**)&ph_ring, 8 * sizeof(srt_camera_uniform))) != cudaSuccess) return e;
+        if ((e = dev_commit(pipe_mem)) != cudaSuccess) return e;
+        cudaStream_t st = ctx->stream;
+        const size_t range_bytes = sizeof(uint2) * range_entries(p.hash_bits);
+        if ((e = cudaMemsetAsync(pipe[1].ranges, 0, range_bytes, st)) != cudaSuccess) return e;
+        for (auto& ps : pipe)
+            if ((e = cudaMemsetAsync(ps.counters, 0, sizeof(FrameCounters), st)) != cudaSuccess) return e;
+        if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
         if ((e = cudaStreamCreateWithFlags(&ph_stream, cudaStreamNonBlocking)) != cudaSuccess) return e;
         if ((e = cudaEventCreateWithFlags(&pfork_ev, cudaEventDisableTiming)) != cudaSuccess) return e;
         if ((e = cudaEventCreateWithFlags(&pjoin_ev, cudaEventDisableTiming)) != cudaSuccess) return e;
@@ -904,18 +935,7 @@ struct srt_renderer {
         if (ph_stream) cudaStreamDestroy(ph_stream);
         if (pfork_ev) cudaEventDestroy(pfork_ev);
         if (pjoin_ev) cudaEventDestroy(pjoin_ev);
-        cudaFreeHost(ph_ring);
-        for (int k = 0; k < 2; ++k) {
-            if (k == 1) {  // set 0's arrays are `ph`'s, freed below
-                cudaFree(pipe[k].photons);
-                cudaFree(pipe[k].sorted);
-                cudaFree(pipe[k].ranges);
-            }
-            cudaFree(pipe[k].counters);
-            cudaFree(pipe[k].cam);
-        }
         if (counts_ev) cudaEventDestroy(counts_ev);
-        if (counts_host) cudaFreeHost(counts_host);
         if (cap_stream) cudaStreamDestroy(cap_stream);
         if (side_stream) cudaStreamDestroy(side_stream);
         if (fork_ev) cudaEventDestroy(fork_ev);
@@ -926,21 +946,11 @@ struct srt_renderer {
         for (auto& e : ring_ev)
             if (e) cudaEventDestroy(e);
         for (auto& e : ev) cudaEventDestroy(e);
-        cudaFree(cam_dev);
-        cudaFreeHost(cam_ring);
+        cudaFreeHost(pinned);
         for (int k = 0; k < 2; ++k) {
             cudaFreeHost(ldr_pinned[k]);
             if (ldr_ev[k]) cudaEventDestroy(ldr_ev[k]);
         }
-        cudaFree(counters);
-        cudaFree(stats);
-        cudaFree(err);
-        void* bufs[] = {pb.ga_p, pb.ga_n, pb.ga_f, pb.ga_start, pb.ray_o, pb.ray_d, pb.hit, pb.thr, pb.wl, pb.rad, pb.light, pb.misc, pb.queue[0], pb.queue[1],
-                        pb.sh_o, pb.sh_d, pb.sh_c, pb.sh_id, pb.sort_keys, pb.sort_keys_alt, pb.sort_vals_alt,
-                        pb.sort_scratch, ph.ray_o, ph.ray_d, ph.state, ph.hit, ph.flags,
-                        ph.queue[0], ph.queue[1], ph.staging, ph.deposit, ph.photons, ph.sorted,
-                        ph.keys, ph.vals, ph.keys2, ph.vals2, ph.sort_scratch, ph.ranges, accum, accum64, ldr};
-        for (void* b : bufs) cudaFree(b);
         guide_free(guide);
     }
 
@@ -1228,74 +1238,80 @@ extern "C" srt_status srt_renderer_create(srt_ctx* c, srt_scene* s, uint32_t w, 
     r->h = h;
     r->p = p;
     size_t np = (size_t)w * h;
-    CUDA_TRY(c, dev_alloc(&r->cam_dev, 1));
-    CUDA_TRY(c, cudaMallocHost((void**)&r->cam_ring, 4 * sizeof(srt_camera_uniform)));
-    for (auto& e : r->ring_ev) CUDA_TRY(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    CUDA_TRY(c, dev_alloc(&r->counters, 1));
-    CUDA_TRY(c, dev_alloc(&r->stats, 1));
-    CUDA_TRY(c, dev_alloc(&r->err, 1));
-    CUDA_TRY(c, cudaMemset(r->stats, 0, sizeof(DevStats)));
-    CUDA_TRY(c, cudaMemset(r->err, 0, 4));
+    DevArena& mem = r->mem;
+    mem.add(&r->cam_dev, 1);
+    mem.add(&r->counters, 1);
+    mem.add(&r->stats, 1);
+    mem.add(&r->err, 1);
     PathBuffers& pb = r->pb;
-    CUDA_TRY(c, dev_alloc(&pb.ray_o, np));
-    CUDA_TRY(c, dev_alloc(&pb.ray_d, np));
-    CUDA_TRY(c, dev_alloc(&pb.hit, np));
-    CUDA_TRY(c, dev_alloc(&pb.thr, np));
-    CUDA_TRY(c, dev_alloc(&pb.wl, np));
-    CUDA_TRY(c, dev_alloc(&pb.rad, np));
-    CUDA_TRY(c, dev_alloc(&pb.light, np));
-    CUDA_TRY(c, dev_alloc(&pb.misc, np));
-    CUDA_TRY(c, dev_alloc(&pb.queue[0], np));
-    CUDA_TRY(c, dev_alloc(&pb.queue[1], np));
-    CUDA_TRY(c, dev_alloc(&pb.sh_o, np));
-    CUDA_TRY(c, dev_alloc(&pb.sh_d, np));
-    CUDA_TRY(c, dev_alloc(&pb.sh_c, np));
-    CUDA_TRY(c, dev_alloc(&pb.sh_id, np));
+    mem.add(&pb.ray_o, np);
+    mem.add(&pb.ray_d, np);
+    mem.add(&pb.hit, np);
+    mem.add(&pb.thr, np);
+    mem.add(&pb.wl, np);
+    mem.add(&pb.rad, np);
+    mem.add(&pb.light, np);
+    mem.add(&pb.misc, np);
+    mem.add(&pb.queue[0], np);
+    mem.add(&pb.queue[1], np);
+    mem.add(&pb.sh_o, np);
+    mem.add(&pb.sh_d, np);
+    mem.add(&pb.sh_c, np);
+    mem.add(&pb.sh_id, np);
     if (p.photons_per_frame > 0) {
-        CUDA_TRY(c, dev_alloc(&pb.ga_p, np));
-        CUDA_TRY(c, dev_alloc(&pb.ga_n, np));
-        CUDA_TRY(c, dev_alloc(&pb.ga_f, np));
-        CUDA_TRY(c, dev_alloc(&pb.ga_start, np));
+        mem.add(&pb.ga_p, np);
+        mem.add(&pb.ga_n, np);
+        mem.add(&pb.ga_f, np);
+        mem.add(&pb.ga_start, np);
     }
     if (p.flags & SRT_FLAG_RAY_SORT) {
-        CUDA_TRY(c, dev_alloc(&pb.sort_keys, np));
-        CUDA_TRY(c, dev_alloc(&pb.sort_keys_alt, np));
-        CUDA_TRY(c, dev_alloc(&pb.sort_vals_alt, np));
-        CUDA_TRY(c, dev_alloc(&pb.sort_scratch, radix_scratch_words((uint32_t)np)));
+        mem.add(&pb.sort_keys, np);
+        mem.add(&pb.sort_keys_alt, np);
+        mem.add(&pb.sort_vals_alt, np);
+        mem.add(&pb.sort_scratch, radix_scratch_words((uint32_t)np));
     }
-    CUDA_TRY(c, dev_alloc(&r->accum, np));
-    CUDA_TRY(c, cudaMemset(r->accum, 0, np * sizeof(float4)));
-    if (p.flags & SRT_FLAG_FP64_ACCUM) {
-        CUDA_TRY(c, dev_alloc(&r->accum64, np));
-        CUDA_TRY(c, cudaMemset(r->accum64, 0, np * sizeof(double4)));
-    }
-    CUDA_TRY(c, dev_alloc(&r->ldr, np));
-    CUDA_TRY(c, cudaMemset(r->ldr, 0, np * 4));
+    mem.add(&r->accum, np);
+    if (p.flags & SRT_FLAG_FP64_ACCUM) mem.add(&r->accum64, np);
+    mem.add(&r->ldr, np);
     PhotonBuffers& ph = r->ph;
     uint32_t cap = p.photons_per_frame;
     ph.capacity = cap;
+    const size_t slots = (size_t)deposit_tiles(cap) * DEPOSIT_TILE;
     if (cap > 0) {
-        const size_t slots = (size_t)deposit_tiles(cap) * DEPOSIT_TILE;
-        CUDA_TRY(c, dev_alloc(&ph.ray_o, cap));
-        CUDA_TRY(c, dev_alloc(&ph.ray_d, cap));
-        CUDA_TRY(c, dev_alloc(&ph.state, cap));
-        CUDA_TRY(c, dev_alloc(&ph.hit, cap));
-        CUDA_TRY(c, dev_alloc(&ph.flags, slots));
-        CUDA_TRY(c, cudaMemset(ph.flags, 0, slots));
-        CUDA_TRY(c, dev_alloc(&ph.queue[0], cap));
-        CUDA_TRY(c, dev_alloc(&ph.queue[1], cap));
-        CUDA_TRY(c, dev_alloc(&ph.staging, 2ull * cap));
-        CUDA_TRY(c, dev_alloc(&ph.deposit, deposit_words(cap)));
-        CUDA_TRY(c, dev_alloc(&ph.photons, 2ull * cap));
-        CUDA_TRY(c, dev_alloc(&ph.sorted, 2ull * cap));
-        CUDA_TRY(c, dev_alloc(&ph.keys, cap));
-        CUDA_TRY(c, dev_alloc(&ph.vals, cap));
-        CUDA_TRY(c, dev_alloc(&ph.keys2, cap));
-        CUDA_TRY(c, dev_alloc(&ph.vals2, cap));
-        CUDA_TRY(c, dev_alloc(&ph.sort_scratch, radix_scratch_words(cap)));
-        CUDA_TRY(c, dev_alloc(&ph.ranges, range_entries(p.hash_bits)));
-        CUDA_TRY(c, cudaMemset(ph.ranges, 0, sizeof(uint2) * range_entries(p.hash_bits)));
+        mem.add(&ph.ray_o, cap);
+        mem.add(&ph.ray_d, cap);
+        mem.add(&ph.state, cap);
+        mem.add(&ph.hit, cap);
+        mem.add(&ph.flags, slots);
+        mem.add(&ph.queue[0], cap);
+        mem.add(&ph.queue[1], cap);
+        mem.add(&ph.staging, 2ull * cap);
+        mem.add(&ph.deposit, deposit_words(cap));
+        mem.add(&ph.photons, 2ull * cap);
+        mem.add(&ph.sorted, 2ull * cap);
+        mem.add(&ph.keys, cap);
+        mem.add(&ph.vals, cap);
+        mem.add(&ph.keys2, cap);
+        mem.add(&ph.vals2, cap);
+        mem.add(&ph.sort_scratch, radix_scratch_words(cap));
+        mem.add(&ph.ranges, range_entries(p.hash_bits));
     }
+    CUDA_TRY(c, dev_commit(mem));
+    CUDA_TRY(c, cudaMemsetAsync(r->stats, 0, sizeof(DevStats), c->stream));
+    CUDA_TRY(c, cudaMemsetAsync(r->err, 0, 4, c->stream));
+    CUDA_TRY(c, cudaMemsetAsync(r->accum, 0, np * sizeof(float4), c->stream));
+    if (r->accum64) CUDA_TRY(c, cudaMemsetAsync(r->accum64, 0, np * sizeof(double4), c->stream));
+    CUDA_TRY(c, cudaMemsetAsync(r->ldr, 0, np * 4, c->stream));
+    if (cap > 0) {
+        CUDA_TRY(c, cudaMemsetAsync(ph.flags, 0, slots, c->stream));
+        CUDA_TRY(c, cudaMemsetAsync(ph.ranges, 0, sizeof(uint2) * range_entries(p.hash_bits), c->stream));
+    }
+    // one pinned block: a pinned allocation costs 1.4 ms and more
+    CUDA_TRY(c, cudaMallocHost(&r->pinned, (4 + 8) * sizeof(srt_camera_uniform) + sizeof(uint32_t) * (MAX_BOUNCES + 1)));
+    r->cam_ring = (srt_camera_uniform*)r->pinned;
+    r->ph_ring = r->cam_ring + 4;
+    r->counts_host = (uint32_t*)(r->ph_ring + 8);
+    for (auto& e : r->ring_ev) CUDA_TRY(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     FrameArgs& a = r->args;
     a.scene = s->dev;
     r->scene_gen = s->gen;
@@ -1355,8 +1371,8 @@ extern "C" srt_status srt_renderer_create(srt_ctx* c, srt_scene* s, uint32_t w, 
     CUDA_TRY(c, cudaStreamCreateWithFlags(&r->train_stream, cudaStreamNonBlocking));
     CUDA_TRY(c, cudaEventCreateWithFlags(&r->tfork_ev, cudaEventDisableTiming));
     CUDA_TRY(c, cudaEventCreateWithFlags(&r->tjoin_ev, cudaEventDisableTiming));
-    CUDA_TRY(c, cudaMallocHost(&r->counts_host, sizeof(uint32_t) * (MAX_BOUNCES + 1)));
     CUDA_TRY(c, cudaEventCreateWithFlags(&r->counts_ev, cudaEventDisableTiming));
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     if (env_fault("launch")) return fail(c, SRT_ERR_CUDA, "injected launch failure");
     ctx_retain(c);
     *out = r.release();
@@ -1687,22 +1703,20 @@ namespace {
 struct TempPhotons {
     PhotonBuffers ph{};
     float4* src = nullptr;
-    ~TempPhotons() {
-        void* bufs[] = {ph.sorted, ph.keys, ph.vals, ph.keys2, ph.vals2, ph.sort_scratch, ph.ranges, src};
-        for (void* b : bufs) cudaFree(b);
-    }
+    DevArena mem;
 };
 
 srt_status temp_grid(srt_ctx* c, const srt_photon* photons, uint32_t n, uint32_t frame, float cell, uint32_t bits,
                      TempPhotons& t) {
-    CUDA_TRY(c, dev_alloc(&t.src, 2ull * n));
-    CUDA_TRY(c, dev_alloc(&t.ph.sorted, 2ull * n));
-    CUDA_TRY(c, dev_alloc(&t.ph.keys, n));
-    CUDA_TRY(c, dev_alloc(&t.ph.vals, n));
-    CUDA_TRY(c, dev_alloc(&t.ph.keys2, n));
-    CUDA_TRY(c, dev_alloc(&t.ph.vals2, n));
-    CUDA_TRY(c, dev_alloc(&t.ph.sort_scratch, radix_scratch_words(n)));
-    CUDA_TRY(c, dev_alloc(&t.ph.ranges, range_entries(bits)));
+    t.mem.add(&t.src, 2ull * n);
+    t.mem.add(&t.ph.sorted, 2ull * n);
+    t.mem.add(&t.ph.keys, n);
+    t.mem.add(&t.ph.vals, n);
+    t.mem.add(&t.ph.keys2, n);
+    t.mem.add(&t.ph.vals2, n);
+    t.mem.add(&t.ph.sort_scratch, radix_scratch_words(n));
+    t.mem.add(&t.ph.ranges, range_entries(bits));
+    CUDA_TRY(c, dev_commit(t.mem));
     if (n) CUDA_TRY(c, cudaMemcpyAsync(t.src, photons, (size_t)n * 32, cudaMemcpyHostToDevice, c->stream));
     t.ph.capacity = n;
     launch_grid_build(t.src, n, frame, cell, bits, t.ph, c->d_err, c->stream);
@@ -1775,19 +1789,14 @@ extern "C" srt_status srt_trace_rays(srt_scene* s, const srt_ray* rays, uint32_t
     srt_ctx* c = s->ctx;
     cudaSetDevice(c->device);
     if (n == 0) return SRT_OK;
-    float4 *dr = nullptr, *dh = nullptr;
-    CUDA_TRY(c, dev_alloc(&dr, 2ull * n));
-    cudaError_t e = dev_alloc(&dh, n);
-    if (e != cudaSuccess) {
-        cudaFree(dr);
-        return cuda_fail(c, e, "alloc");
-    }
+    CallWork work(c);
+    void* p = nullptr;
+    CUDA_TRY(c, work.get(&p, 48ull * n));
+    float4 *dr = (float4*)p, *dh = dr + 2ull * n;
     cudaMemcpyAsync(dr, rays, 32ull * n, cudaMemcpyHostToDevice, c->stream);
     launch_trace_batch(s->dev, dr, n, dh, any_hit, c->d_err, c->stream);
     cudaMemcpyAsync(hits, dh, 16ull * n, cudaMemcpyDeviceToHost, c->stream);
-    e = cudaStreamSynchronize(c->stream);
-    cudaFree(dr);
-    cudaFree(dh);
+    const cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "trace");
     return check_device_error(c, c->d_err);
 }

@@ -1,0 +1,70 @@
+// One device allocation for all arrays of one owner.
+//
+// cudaMalloc and cudaFree cost 0.2-1.3 ms each on a B200 host whatever the
+// size (64 KB 0.19 / 0.20 ms, 4 MB 1.1 / 1.0, 256 MB 0.4 / 0.5; under 64 KB they
+// are cheap only while a 2 MB page has room), and a renderer has about fifty
+// arrays: objects register their arrays first and take them from a single
+// allocation, which lives exactly as long as the object.  Opening a scene of
+// 331k triangles (build, renderer, two frames, release): 58 -> 29 ms.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstddef>
+#include <vector>
+
+namespace srt {
+
+class DevArena {
+  public:
+    static constexpr size_t ALIGN = 256;  // what cudaMalloc guarantees
+
+    DevArena() = default;
+    DevArena(const DevArena&) = delete;
+    DevArena& operator=(const DevArena&) = delete;
+    ~DevArena() { release(); }
+
+    // *p is set by commit(); at least one element, so that it is never null.
+    template <class T>
+    void add(T** p, size_t count) {
+        *p = nullptr;
+        slots_.push_back(Slot{(void**)p, bytes_});
+        bytes_ += (sizeof(T) * std::max<size_t>(count, 1) + ALIGN - 1) / ALIGN * ALIGN;
+    }
+
+    cudaError_t commit() {
+        if (slots_.empty()) return cudaSuccess;
+        cudaError_t e = cudaMalloc((void**)&base_, bytes_);
+        if (e == cudaSuccess)
+            for (const Slot& s : slots_) *s.p = base_ + s.offset;
+        slots_.clear();
+        return e;
+    }
+
+    // Frees the arrays (cudaFree waits for the work that uses them).
+    void release() {
+        cudaFree(base_);
+        base_ = nullptr;
+        bytes_ = 0;
+        slots_.clear();
+    }
+
+    // Hands the allocation to the caller, who frees it (cudaFree).
+    void* detach() {
+        void* p = base_;
+        base_ = nullptr;
+        return p;
+    }
+
+  private:
+    struct Slot {
+        void** p;
+        size_t offset;
+    };
+    char* base_ = nullptr;
+    size_t bytes_ = 0;
+    std::vector<Slot> slots_;
+};
+
+}  // namespace srt

@@ -20,6 +20,7 @@
 #include <vector>
 
 #define SRT_RNG_DIVIDE
+#include "dev_arena.h"
 #include "guide.cuh"
 #include "render_kernels.h"
 #include "umma.cuh"
@@ -1760,10 +1761,6 @@ int launch_guide_test_train(const GuideArgs& g, int phase, cudaStream_t st) {
 
 // ---------------------------------------------------------------- host side
 namespace {
-template <class T>
-cudaError_t galloc(T** p, size_t n) {
-    return cudaMalloc((void**)p, n * sizeof(T));
-}
 // splitmix64: the deterministic stream of the default initialisation
 uint64_t splitmix(uint64_t& x) {
     uint64_t z = (x += 0x9E3779B97F4A7C15ull);
@@ -1792,34 +1789,33 @@ void guide_default_params(uint64_t seed, float* out) {
 cudaError_t guide_alloc(GuideArgs& g, size_t n_verts) {
     g = GuideArgs{};
     g.steps = 1;
-    cudaError_t e = cudaSuccess;
-    auto chk = [&](cudaError_t r) {
-        if (e == cudaSuccess) e = r;
-    };
-    chk(galloc(&g.net.master, G_NPARAMS));
-    chk(galloc(&g.net.wbf, G_NPARAMS));
-    chk(galloc(&g.net.adam_m, G_NPARAMS));
-    chk(galloc(&g.net.adam_v, G_NPARAMS));
-    chk(galloc(&g.net.grad, G_NPARAMS));
+    DevArena mem;
+    mem.add(&g.net.master, G_NPARAMS);
+    mem.add(&g.net.wbf, G_NPARAMS);
+    mem.add(&g.net.adam_m, G_NPARAMS);
+    mem.add(&g.net.adam_v, G_NPARAMS);
+    mem.add(&g.net.grad, G_NPARAMS);
     if (n_verts > 0) {
-        chk(galloc(&g.gv.p, n_verts));
-        chk(galloc(&g.gv.n, n_verts));
-        chk(galloc(&g.gv.wo, n_verts));
-        chk(galloc(&g.gv.spec, n_verts));
-        chk(galloc(&g.gv.id, n_verts));
+        mem.add(&g.gv.p, n_verts);
+        mem.add(&g.gv.n, n_verts);
+        mem.add(&g.gv.wo, n_verts);
+        mem.add(&g.gv.spec, n_verts);
+        mem.add(&g.gv.id, n_verts);
     }
-    chk(galloc(&g.rec.x0, G_REC_CAP));
-    chk(galloc(&g.rec.x1, G_REC_CAP));
-    chk(galloc(&g.rec.x2, G_REC_CAP));
-    chk(galloc(&g.rec.w, G_REC_CAP));
-    chk(galloc(&g.rec.b, G_REC_CAP));
-    chk(galloc(&g.rec.thr, G_REC_CAP));
-    chk(galloc(&g.rec.rad, G_REC_CAP));
-    chk(galloc(&g.rec.pid, G_REC_CAP));
-    chk(galloc(&g.rec.weight, G_REC_CAP));
-    chk(galloc(&g.rec.act, (size_t)G_REC_CAP * G_ACT_STRIDE));
-    chk(galloc(&g.rec.delta, (size_t)G_REC_CAP * G_DELTA_STRIDE));
-    chk(galloc(&g.gc, 1));
+    mem.add(&g.rec.x0, G_REC_CAP);
+    mem.add(&g.rec.x1, G_REC_CAP);
+    mem.add(&g.rec.x2, G_REC_CAP);
+    mem.add(&g.rec.w, G_REC_CAP);
+    mem.add(&g.rec.b, G_REC_CAP);
+    mem.add(&g.rec.thr, G_REC_CAP);
+    mem.add(&g.rec.rad, G_REC_CAP);
+    mem.add(&g.rec.pid, G_REC_CAP);
+    mem.add(&g.rec.weight, G_REC_CAP);
+    mem.add(&g.rec.act, (size_t)G_REC_CAP * G_ACT_STRIDE);
+    mem.add(&g.rec.delta, (size_t)G_REC_CAP * G_DELTA_STRIDE);
+    mem.add(&g.gc, 1);
+    cudaError_t e = mem.commit();
+    mem.detach();  // freed through its first array (guide_free)
     if (e == cudaSuccess) {
         GuideCounters gc{};
         gc.threshold = 65536u;
@@ -1833,10 +1829,7 @@ cudaError_t guide_alloc(GuideArgs& g, size_t n_verts) {
 }
 
 void guide_free(GuideArgs& g) {
-    void* bufs[] = {g.net.master, g.net.wbf, g.net.adam_m, g.net.adam_v, g.net.grad,
-                    g.gv.p, g.gv.n, g.gv.wo, g.gv.spec, g.gv.id, g.rec.x0, g.rec.x1, g.rec.x2, g.rec.w, g.rec.b,
-                    g.rec.thr, g.rec.rad, g.rec.pid, g.rec.weight, g.rec.act, g.rec.delta, g.gc};
-    for (void* b : bufs) cudaFree(b);
+    cudaFree(g.net.master);  // the first array of the one allocation
     g = GuideArgs{};
 }
 
