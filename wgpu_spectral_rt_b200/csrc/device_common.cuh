@@ -5,6 +5,7 @@
 // one) in FP32; they are written for the GPU (float4 SIMD-style helpers,
 // register-resident state) and checked against the CPU oracle.
 #pragma once
+#include <cuda_fp16.h>
 
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -505,12 +506,11 @@ SRT_DEV bool intersect_tri(const Ray& ray, const RayShear& sh, float3 v0, float3
 }
 
 SRT_DEV uint32_t byte_of(uint32_t w, int i) { return (w >> (8 * i)) & 0xFFu; }
-// Byte k of w plus 2^23 as a float, without the integer-to-float conversion
-// unit: one byte permute builds the bit pattern 0x4B0000bb (= 2^23 + b
-// exactly).  The slab test folds the 2^23 bias into its addend,
-// t = fma(2^23 + q, a, b - 2^23 a), whose rounding moves a plane by at most
-// half a quantum; the builder pads every child box by one quantum.
-SRT_DEV float qbyte(uint32_t w, uint32_t k) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u | k)); }
+// A byte b as a float without the integer-to-float conversion unit is the bit
+// pattern 0x4B0000bb (= 2^23 + b exactly).  The group's slab test (group_step)
+// folds the 2^23 bias into its addend, t = fma(2^23 + q, a, b - 2^23 a), whose
+// rounding moves a plane by at most half a quantum (node_hits' 1024: 2^-14 of
+// one); the builder pads every child box by one quantum.
 SRT_DEV float unbias(float a, float b) { return fmaf(-8388608.0f, a, b); }
 
 // Two fused multiply-adds: one packed fma.rn.f32x2 with SRT_TRAV_FMA2 (the
@@ -540,33 +540,28 @@ struct TravCounters {
     unsigned long long* tris;
 };
 
-// Asynchronous 16-byte copies global -> shared (cp.async, L1-cached): a
-// lane starts fetching the next node into its shared-memory slot, tests
-// the pending triangles meanwhile, then waits for its own copies.
-SRT_DEV void cp_async16(void* smem, const void* gmem) {
-    const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
-}
-SRT_DEV void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-SRT_DEV void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-// Node idx into this lane's slot: 5 chunks, chunk k at nbuf[k * stride].
-SRT_DEV void fetch_node_async(const DevScene& S, uint32_t idx, uint4* nbuf, int stride) {
-    const uint4* np = reinterpret_cast<const uint4*>(S.nodes + idx);
-#pragma unroll
-    for (int k = 0; k < 5; ++k) cp_async16(nbuf + k * stride, np + k);
-    cp_async_commit();
+// Bytes 2p and 2p + 1 of w, each plus 1024, as floats (exact): one byte permute
+// builds the half pair 0x64bb64bb, and its two conversions run beside the fused
+// multiply-adds; the permutes share a half-rate unit with the minima and maxima.
+SRT_DEV float2 qpair(uint32_t w, uint32_t p) {
+    const uint32_t h = __byte_perm(w, 0x64646464u, p ? 0x4342u : 0x4140u);
+    return __half22float2(*reinterpret_cast<const __half2*>(&h));
 }
 
 // Child slab tests of one node (words w0..w4) for a ray with inverse
 // direction idir and octant oct: the slots whose box the ray meets within
-// [tmin, tbest].
+// [tmin, tbest].  A slot without a child may be among them: it has no imask bit
+// and no triangles.  (With a test per slot for a child, a compare and a select
+// for the bit, and a byte permute per plane: closest hits 3.25 vs 3.17 ms per
+// config-2 frame, shadow rays 1.88 vs 1.82.)
 SRT_DEV uint32_t node_hits(uint4 w0, uint4 w1, uint4 w2, uint4 w3, uint4 w4, float3 o, float3 idir, uint32_t oct,
                            float tmin, float tbest) {
     float sx = __uint_as_float((w0.w & 0xFFu) << 23), sy = __uint_as_float(((w0.w >> 8) & 0xFFu) << 23),
           sz = __uint_as_float(((w0.w >> 16) & 0xFFu) << 23);
     float ax = sx * idir.x, ay = sy * idir.y, az = sz * idir.z;
-    float bx = unbias(ax, (__uint_as_float(w0.x) - o.x) * idir.x), by = unbias(ay, (__uint_as_float(w0.y) - o.y) * idir.y),
-          bz = unbias(az, (__uint_as_float(w0.z) - o.z) * idir.z);
+    float bx = fmaf(-1024.0f, ax, (__uint_as_float(w0.x) - o.x) * idir.x),
+          by = fmaf(-1024.0f, ay, (__uint_as_float(w0.y) - o.y) * idir.y),
+          bz = fmaf(-1024.0f, az, (__uint_as_float(w0.z) - o.z) * idir.z);
     uint32_t nx0 = (oct & 1u) ? w3.z : w2.x, nx1 = (oct & 1u) ? w3.w : w2.y;
     uint32_t fx0 = (oct & 1u) ? w2.x : w3.z, fx1 = (oct & 1u) ? w2.y : w3.w;
     uint32_t ny0 = (oct & 2u) ? w4.x : w2.z, ny1 = (oct & 2u) ? w4.y : w2.w;
@@ -574,22 +569,28 @@ SRT_DEV uint32_t node_hits(uint4 w0, uint4 w1, uint4 w2, uint4 w3, uint4 w4, flo
     uint32_t nz0 = (oct & 4u) ? w4.z : w3.x, nz1 = (oct & 4u) ? w4.w : w3.y;
     uint32_t fz0 = (oct & 4u) ? w3.x : w4.z, fz1 = (oct & 4u) ? w3.y : w4.w;
     const float robust = 1.0000004f;
-    uint32_t hitmask = 0u;
+    uint32_t miss = 0u;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const uint32_t k = (uint32_t)(i & 3);
-        const uint32_t m = byte_of(i < 4 ? w1.z : w1.w, k);
-        const float2 tx = fma2(make_float2(qbyte(i < 4 ? nx0 : nx1, k), qbyte(i < 4 ? fx0 : fx1, k)),
-                               make_float2(ax, ax), make_float2(bx, bx));
-        const float2 ty = fma2(make_float2(qbyte(i < 4 ? ny0 : ny1, k), qbyte(i < 4 ? fy0 : fy1, k)),
-                               make_float2(ay, ay), make_float2(by, by));
-        const float2 tz = fma2(make_float2(qbyte(i < 4 ? nz0 : nz1, k), qbyte(i < 4 ? fz0 : fz1, k)),
-                               make_float2(az, az), make_float2(bz, bz));
-        const float tn = fmaxf(fmaxf(tx.x, ty.x), fmaxf(tz.x, tmin));
-        const float tf = fminf(fminf(tx.y, ty.y), fminf(tz.y, tbest)) * robust;
-        hitmask |= (m != 0u && tn <= tf) ? (1u << i) : 0u;
+    for (int j = 3; j >= 0; --j) {  // children 2j and 2j + 1
+        const uint32_t p = (uint32_t)(j & 1);
+        const float2 qnx = qpair(j < 2 ? nx0 : nx1, p), qfx = qpair(j < 2 ? fx0 : fx1, p),
+                     qny = qpair(j < 2 ? ny0 : ny1, p), qfy = qpair(j < 2 ? fy0 : fy1, p),
+                     qnz = qpair(j < 2 ? nz0 : nz1, p), qfz = qpair(j < 2 ? fz0 : fz1, p);
+#pragma unroll
+        for (int e = 1; e >= 0; --e) {
+            const float2 tx = fma2(make_float2(e ? qnx.y : qnx.x, e ? qfx.y : qfx.x), make_float2(ax, ax),
+                                   make_float2(bx, bx));
+            const float2 ty = fma2(make_float2(e ? qny.y : qny.x, e ? qfy.y : qfy.x), make_float2(ay, ay),
+                                   make_float2(by, by));
+            const float2 tz = fma2(make_float2(e ? qnz.y : qnz.x, e ? qfz.y : qfz.x), make_float2(az, az),
+                                   make_float2(bz, bz));
+            const float tn = fmaxf(fmaxf(tx.x, ty.x), fmaxf(tz.x, tmin));
+            const float tf = fminf(fminf(tx.y, ty.y), fminf(tz.y, tbest));
+            // the sign of tf * robust - tn shifted in: missed where it is negative
+            miss = __funnelshift_l(__float_as_uint(fmaf(tf, robust, -tn)), miss, 1);
+        }
     }
-    return hitmask;
+    return ~miss & 0xFFu;
 }
 
 // One node visit: the node's hit internal children (bits 24..31, ordered by
@@ -694,9 +695,9 @@ SRT_DEV int scatter_step(const DevScene& S, ScatterWalk& W, float tmin, float tm
 // minimum of (t, flattened triangle id), independent of traversal order.
 // `stack` is this thread's slice of shared memory, stride `stride` entries,
 // STACK entries deep (at least the tree depth: one entry per level).
-template <bool ANY, bool COUNT, int STACK = TRAV_STACK, bool PF = false>
+template <bool ANY, bool COUNT, int STACK = TRAV_STACK>
 SRT_DEV bool traverse(const DevScene& S, Ray ray, uint2* stack, int stride, float& t_out, uint32_t& prim_out,
-                      float& u_out, float& v_out, uint32_t* err, TravCounters cnt, uint4* nbuf = nullptr) {
+                      float& u_out, float& v_out, uint32_t* err, TravCounters cnt) {
     prim_out = MISS;
     if (S.n_nodes == 0u) return false;
     if (!(ray.d.x != 0.0f || ray.d.y != 0.0f || ray.d.z != 0.0f)) return false;
@@ -716,37 +717,6 @@ SRT_DEV bool traverse(const DevScene& S, Ray ray, uint2* stack, int stride, floa
     uint2 g = make_uint2(0u, (1u << (24 + (0u ^ (oct ^ 7u)))) | 1u);
     uint2 tg = make_uint2(0u, 0u);
     while (true) {
-        // ---- with PF: pick the next node and start fetching it before the
-        // triangle tests of the last node (the same visiting order)
-        bool have = true;
-        if (PF) {
-            if ((g.y & 0xFF000000u) == 0u) {
-                if (sp == 0) have = false;
-                else {
-                    --sp;
-                    g = stack[sp * stride];
-                }
-            }
-            if (have) {
-                int bit = 31 - __clz(g.y & 0xFF000000u);
-                g.y &= ~(1u << bit);
-                uint32_t slot = (uint32_t)(bit - 24) ^ (oct ^ 7u);
-                uint32_t idx = g.x + __popc(g.y & ((1u << slot) - 1u) & 0xFFu);
-                if (g.y & 0xFF000000u) {
-                    if (sp >= STACK) {
-                        atomicOr(err, ERR_STACK_OVERFLOW);
-                        break;
-                    }
-                    stack[sp * stride] = g;
-                    ++sp;
-                }
-                if (idx >= S.n_nodes) {
-                    atomicOr(err, ERR_BAD_INDEX);
-                    break;
-                }
-                fetch_node_async(S, idx, nbuf, stride);
-            }
-        }
         // ---- triangles of the last node
         while (tg.y != 0u) {
             int b = __ffs(tg.y) - 1;
@@ -760,7 +730,6 @@ SRT_DEV bool traverse(const DevScene& S, Ray ray, uint2* stack, int stride, floa
             if (intersect_tri(r, sh, xyz(a0), xyz(a1), xyz(a2), t, u, v)) {
                 uint32_t id = __float_as_uint(a0.w);
                 if (ANY) {
-                    if (PF) cp_async_wait_all();  // no copy into the slot outlives the ray
                     t_out = t;
                     prim_out = id;
                     if (COUNT) {
@@ -778,14 +747,6 @@ SRT_DEV bool traverse(const DevScene& S, Ray ray, uint2* stack, int stride, floa
                     }
                 }
             }
-        }
-        if (PF) {
-            if (!have) break;
-            cp_async_wait_all();
-            if (COUNT) ++n_nodes;
-            node_children(nbuf[0], nbuf[stride], nbuf[2 * stride], nbuf[3 * stride], nbuf[4 * stride], ray.o, idir, oct,
-                          ray.tmin, tbest, g, tg);
-            continue;
         }
         // ---- next node
         if ((g.y & 0xFF000000u) == 0u) {
@@ -830,77 +791,18 @@ SRT_DEV bool traverse(const DevScene& S, Ray ray, uint2* stack, int stride, floa
 // ------------------------------------------------------------------ resumable traversal
 // The same traversal as traverse<>, split into an init and a step so that a
 // persistent warp can hand a finished lane a new ray between steps.  One
-// step = the pending triangle tests of the last node + one node visit.
-#ifndef SRT_TRAV_ONE_TRI_PER_STEP
-#define SRT_TRAV_ONE_TRI_PER_STEP 0
-#endif
-// Closest-hit steps: the lanes of a warp that entered a step wait for each
-// other before the node visit (__syncwarp), so that it runs with all of them
-// at once instead of in the groups in which they left the triangle loop and
-// the stack pop (measured on bounce 1 of config 2: 0.75M warp node visits
-// with 21.8 lanes each instead of 1.09M with 15.0; closest-hit 3.29 vs
-// 3.37 ms per frame).  Any-hit steps use pooled triangle tests instead
-// (pool_tris); the two together measured slower than either alone.
-#ifndef SRT_TRAV_WARPSYNC
-#define SRT_TRAV_WARPSYNC 1
-#endif
-
-// The top entry of the traversal stack in registers (SRT_TRAV_REG_TOP): a
-// push keeps the new group in `top` and moves the previous top to shared
-// memory; a pop takes `top` if there is one.  A group pushed at a node visit
-// and popped when that node's subtree is done never touches shared memory.
-#ifndef SRT_TRAV_REG_TOP
-#define SRT_TRAV_REG_TOP 0
-#endif
-constexpr uint32_t AXES_HAS_TOP = 1u << 16;  // TravState.axes: `top` holds an entry
-
+// step = the pending triangle tests of the warp's last node visits (pool_tris)
+// + one node visit per lane (trav_step).
 struct TravState {
     float3 o, idir;
     float tmin, tbest;
     float sx, sy, sz;
-    uint32_t axes;  // kx | ky << 2 | kz << 4 | oct << 8 (| AXES_HAS_TOP)
+    uint32_t axes;  // kx | ky << 2 | kz << 4 | oct << 8
     uint2 g, tg;
     int sp;
     uint32_t best;
     float bu, bv;
-#if SRT_TRAV_REG_TOP
-    uint2 top;
-#endif
 };
-
-// Pops the next node group into T.g; false when the stack is empty.
-SRT_DEV bool trav_pop(TravState& T, const uint2* stack, int stride) {
-#if SRT_TRAV_REG_TOP
-    if (T.axes & AXES_HAS_TOP) {
-        T.g = T.top;
-        T.axes &= ~AXES_HAS_TOP;
-        return true;
-    }
-#endif
-    if (T.sp == 0) return false;
-    --T.sp;
-    T.g = stack[T.sp * stride];
-    return true;
-}
-// Pushes T.g; false when STACK shared-memory entries are in use (overflow).
-template <int STACK>
-SRT_DEV bool trav_push(TravState& T, uint2* stack, int stride) {
-#if SRT_TRAV_REG_TOP
-    if (T.axes & AXES_HAS_TOP) {
-        if (T.sp >= STACK) return false;
-        stack[T.sp * stride] = T.top;
-        ++T.sp;
-    }
-    T.top = T.g;
-    T.axes |= AXES_HAS_TOP;
-    return true;
-#else
-    if (T.sp >= STACK) return false;
-    stack[T.sp * stride] = T.g;
-    ++T.sp;
-    return true;
-#endif
-}
 
 // Returns false when the ray cannot hit anything (finished at once).
 SRT_DEV bool trav_init(TravState& T, const DevScene& S, float3 o, float3 d, float tmin, float tmax) {
@@ -927,34 +829,35 @@ SRT_DEV bool trav_init(TravState& T, const DevScene& S, float3 o, float3 d, floa
     return true;
 }
 
-// Pooled triangle tests (SRT_TRAV_POOL), called by all 32 lanes of a warp
+// Pooled triangle tests, called by all 32 lanes of a warp
 // at once: the triangles pending at the lanes' last node visits (T.tg of the
 // lanes with `live` set) are numbered across the warp by a prefix sum and
 // dealt out one per lane per round, so a round tests up to 32 triangles
 // whatever lanes they belong to (idle lanes work too), instead of each lane
-// looping over its own with the others waiting.  A lane fetches its task's
-// ray from the owning lane (shuffles), tests it with the same tri_test, and
-// a segmented minimum over the lanes of one owner (tasks of a lane are
-// consecutive) gives the owner the lexicographic minimum of (t, id) and its
-// (u, v); the owner keeps it if it beats its best.  The closest hit does not
-// depend on the order of the tests, so results are unchanged; any-hit rays
-// stop at their first hit (T.best != MISS afterwards).  Leaves T.tg empty.
-// Used by the persistent any-hit kernel (SRT_TRAV_POOL): the triangle loop of
-// bounce-1 closest-hit steps ran 2.15M warp iterations per config-2 frame
-// with 4.45 of 32 lanes busy; pooled, the shadow rays of bounces 1-4 take
-// 1.57 instead of 1.94 ms per frame.  Closest-hit steps measured no gain
-// alone and 1.6x slower with the closest-hit warp sync (SRT_TRAV_POOL=2
-// pools them too).
-#ifndef SRT_TRAV_POOL
-#define SRT_TRAV_POOL 1
-#endif
+// looping over its own with the others waiting.  The owners list a round's
+// tasks in `tasks` (32 words of shared memory per warp); a lane fetches its
+// task's ray from the owner (shuffles) and tests it with the same tri_test; the
+// owner then reads the hits of its tasks (consecutive lanes of a ballot) and
+// keeps the lexicographic minimum of (t, id).  The closest hit does not depend
+// on the order of the tests, so results are unchanged; any-hit rays stop at
+// their first hit (T.best != MISS afterwards).  Leaves T.tg empty.
+// Looping over its own triangles kept 4.45 of 32 lanes busy on bounce 1 of
+// config 2; with pooled tests in both forms and 8 blocks per SM (lists instead
+// of a search and an __fns per task, hits read from the ballot instead of a
+// segmented minimum): closest hits 3.13 -> 2.99 ms and shadow rays 1.83 -> 1.79
+// ms per config-2 frame, Cornell 640x480 0.68 -> 0.68 and 0.41 -> 0.40, a seeded
+// scene of 812k triangles 0.97 -> 0.94 and 0.52 -> 0.53, caustic slab 1.30 -> 1.34
+// and 0.77 -> 0.76 (its nodes hold few triangles; testing one per lane directly
+// where no lane has more: 1.35).
 // MULTI: the lanes trace rays of different scenes (the batched renderer's
 // persistent launch), so a task reads the triangles of its owner's scene.
 template <bool ANY, bool MULTI = false>
-SRT_DEV void pool_tris(const DevScene& S, TravState& T, bool live, uint32_t& n_tris) {
+SRT_DEV void pool_tris(const DevScene& S, TravState& T, bool live, uint32_t* tasks, uint32_t& n_tris) {
     constexpr uint32_t FULL = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t cnt = live ? (uint32_t)__popc(T.tg.y) : 0u;
+    uint32_t bits = live ? T.tg.y : 0u;
+    if (!__any_sync(FULL, bits != 0u)) return;
+    const uint32_t cnt = (uint32_t)__popc(bits);
     uint32_t incl = cnt;
 #pragma unroll
     for (uint32_t d = 1; d < 32u; d <<= 1) {
@@ -962,218 +865,93 @@ SRT_DEV void pool_tris(const DevScene& S, TravState& T, bool live, uint32_t& n_t
         if (lane >= d) incl += v;
     }
     const uint32_t total = __shfl_sync(FULL, incl, 31);
-    if (total == 0u) return;
     const uint32_t excl = incl - cnt;
+    uint32_t pos = excl;
     for (uint32_t base = 0; base < total; base += 32u) {
-        const uint32_t task = base + lane;
-        const bool have = task < total;
-        // owner = the number of lanes whose tasks end at or before this one
-        uint32_t o = 0;
-#pragma unroll
-        for (uint32_t step = 16; step >= 1u; step >>= 1) {
-            const uint32_t v = __shfl_sync(FULL, incl, (int)(o + step - 1u));
-            if (v <= task) o += step;
+        while (bits != 0u && pos < base + 32u) {
+            tasks[pos - base] = lane | ((uint32_t)(__ffs(bits) - 1) << 8);
+            bits &= bits - 1u;
+            ++pos;
         }
-        o = have ? o : 31u;
-        const uint32_t o_excl = __shfl_sync(FULL, excl, (int)o);
-        const uint32_t gx = __shfl_sync(FULL, T.tg.x, (int)o), gy = __shfl_sync(FULL, T.tg.y, (int)o);
-        const float ox = __shfl_sync(FULL, T.o.x, (int)o), oy = __shfl_sync(FULL, T.o.y, (int)o),
-                    oz = __shfl_sync(FULL, T.o.z, (int)o);
-        const float sx = __shfl_sync(FULL, T.sx, (int)o), sy = __shfl_sync(FULL, T.sy, (int)o),
-                    sz = __shfl_sync(FULL, T.sz, (int)o);
-        const float tmin = __shfl_sync(FULL, T.tmin, (int)o), tmax = __shfl_sync(FULL, T.tbest, (int)o);
-        const uint32_t axes = __shfl_sync(FULL, T.axes, (int)o);
-        uint32_t klo = 0xFFFFFFFFu, khi = 0xFFFFFFFFu;  // (t bits, id) of a hit, else all ones
-        float hu = 0.f, hv = 0.f;
+        __syncwarp();
+        const bool have = base + lane < total;
+        const uint32_t task = have ? tasks[lane] : lane;
+        __syncwarp();  // the next round's tasks go into the same words
+        const int o = (int)(task & 31u);
+        const uint32_t gx = __shfl_sync(FULL, T.tg.x, o);
+        const float ox = __shfl_sync(FULL, T.o.x, o), oy = __shfl_sync(FULL, T.o.y, o), oz = __shfl_sync(FULL, T.o.z, o);
+        const float sx = __shfl_sync(FULL, T.sx, o), sy = __shfl_sync(FULL, T.sy, o), sz = __shfl_sync(FULL, T.sz, o);
+        const float tmin = __shfl_sync(FULL, T.tmin, o), tmax = __shfl_sync(FULL, T.tbest, o);
+        const uint32_t axes = __shfl_sync(FULL, T.axes, o);
         const TriSlot* tris = S.tris;
         if (MULTI)
             tris = reinterpret_cast<const TriSlot*>(
-                __shfl_sync(FULL, reinterpret_cast<unsigned long long>(S.tris), (int)o));
+                __shfl_sync(FULL, reinterpret_cast<unsigned long long>(S.tris), o));
+        bool hit = false;
+        float t = 0.f, u = 0.f, v = 0.f;
+        uint32_t id = 0u;
         if (have) {
-            const uint32_t bit = __fns(gy, 0u, (int)(task - o_excl + 1u)) & 31u;  // always found: task < incl[o]
-            const TriSlot* ts = tris + gx + bit;
+            const TriSlot* ts = tris + gx + (task >> 8);
             const float4 a0 = __ldg(&ts->v0), a1 = __ldg(&ts->v1), a2 = __ldg(&ts->v2);
             ++n_tris;
-            float t, u, v;
-            if (tri_test(xyz(a0), xyz(a1), xyz(a2), f3(ox, oy, oz), axes & 3u, (axes >> 2) & 3u, (axes >> 4) & 3u, sx,
-                         sy, sz, tmin, tmax, t, u, v)) {
-                khi = __float_as_uint(t);  // t >= tmin > 0: the bits order like the values
-                klo = __float_as_uint(a0.w);
-                hu = u;
-                hv = v;
-            }
+            id = __float_as_uint(a0.w);
+            hit = tri_test(xyz(a0), xyz(a1), xyz(a2), f3(ox, oy, oz), axes & 3u, (axes >> 2) & 3u, (axes >> 4) & 3u, sx,
+                           sy, sz, tmin, tmax, t, u, v);
         }
-        // segmented minimum over the lanes of one owner (consecutive lanes)
-        const uint32_t own = have ? o : 32u;
-#pragma unroll
-        for (uint32_t d = 1; d < 32u; d <<= 1) {
-            const uint32_t olo = __shfl_down_sync(FULL, klo, d), ohi = __shfl_down_sync(FULL, khi, d);
-            const float ou = __shfl_down_sync(FULL, hu, d), ov = __shfl_down_sync(FULL, hv, d);
-            const uint32_t oo = __shfl_down_sync(FULL, own, d);
-            if (lane + d < 32u && oo == own && (ohi < khi || (ohi == khi && olo < klo))) {
-                khi = ohi;
-                klo = olo;
-                hu = ou;
-                hv = ov;
-            }
+        // the hits of this lane's tasks: lanes [lo, hi) of the round
+        uint32_t hits = __ballot_sync(FULL, hit);
+        if (hits == 0u) continue;
+        const uint32_t lo = max(excl, base) - base, hi = min(incl, base + 32u) - base;
+        if (cnt == 0u || incl <= base || excl >= base + 32u) hits = 0u;
+        else hits &= (hi - lo >= 32u ? FULL : ((1u << (hi - lo)) - 1u)) << lo;
+        if (ANY) {
+            if (hits != 0u) T.best = 0u;
+            continue;
         }
-        // each owner reads the minimum at the first lane of its segment
-        const bool mine = cnt > 0u && incl > base && excl < base + 32u;
-        const uint32_t first = mine ? (excl > base ? excl - base : 0u) : lane;
-        const uint32_t rlo = __shfl_sync(FULL, klo, (int)first), rhi = __shfl_sync(FULL, khi, (int)first);
-        const float ru = __shfl_sync(FULL, hu, (int)first), rv = __shfl_sync(FULL, hv, (int)first);
-        if (mine && rhi != 0xFFFFFFFFu) {
-            if (ANY) {
-                if (T.best == MISS) {
-                    T.best = rlo;
-                    T.tbest = __uint_as_float(rhi);
-                }
-            } else {
-                const uint32_t chi = __float_as_uint(T.tbest);
-                if (rhi < chi || (rhi == chi && rlo < T.best)) {
-                    T.tbest = __uint_as_float(rhi);
-                    T.best = rlo;
-                    T.bu = ru;
-                    T.bv = rv;
-                }
+        while (__any_sync(FULL, hits != 0u)) {
+            const int src = hits != 0u ? __ffs(hits) - 1 : (int)lane;
+            const float ht = __shfl_sync(FULL, t, src), hu = __shfl_sync(FULL, u, src), hv = __shfl_sync(FULL, v, src);
+            const uint32_t hid = __shfl_sync(FULL, id, src);
+            if (hits != 0u && (ht < T.tbest || (ht == T.tbest && hid < T.best))) {
+                T.tbest = ht;
+                T.best = hid;
+                T.bu = hu;
+                T.bv = hv;
             }
+            hits &= hits - 1u;
         }
     }
     if (live) T.tg.y = 0u;
 }
 
-// Returns true when the ray is finished (for ANY: T.best != MISS on a hit).
-template <bool ANY, int STACK, bool PF = false>
-SRT_DEV bool trav_step(const DevScene& S, TravState& T, uint2* stack, int stride, uint32_t* err, uint32_t& n_nodes,
-                       uint32_t& n_tris, uint4* nbuf = nullptr) {
-    const uint32_t kx = T.axes & 3u, ky = (T.axes >> 2) & 3u, kz = (T.axes >> 4) & 3u, oct = (T.axes >> 8) & 7u;
-    // `entered`: the lanes converged at the step's start.  Every one of them
-    // reaches the __syncwarp below (nothing before it returns), so the sync is
-    // well formed.  Syncing the ballot of all lanes that take the step instead
-    // (a stronger wait) measured slower: closest-hit 3.40 vs 3.30 ms per frame.
-    constexpr bool kSync = SRT_TRAV_WARPSYNC && !ANY && !PF && !SRT_TRAV_ONE_TRI_PER_STEP;
-    const uint32_t entered = kSync ? __activemask() : 0u;
-    bool any_hit = false;
-    bool have = true;
-    if (PF) {
-        // pick the next node and start fetching it; the triangle tests below
-        // run while the copy is in flight (same visiting order)
-        if ((T.g.y & 0xFF000000u) == 0u) {
-            if (T.sp == 0) have = false;
-            else {
-                --T.sp;
-                T.g = stack[T.sp * stride];
-            }
-        }
-        if (have) {
-            int bit = 31 - __clz(T.g.y & 0xFF000000u);
-            T.g.y &= ~(1u << bit);
-            uint32_t slot = (uint32_t)(bit - 24) ^ (oct ^ 7u);
-            uint32_t idx = T.g.x + __popc(T.g.y & ((1u << slot) - 1u) & 0xFFu);
-            if (T.g.y & 0xFF000000u) {
-                if (T.sp >= STACK) {
-                    atomicOr(err, ERR_STACK_OVERFLOW);
-                    return true;
-                }
-                stack[T.sp * stride] = T.g;
-                ++T.sp;
-            }
-            if (idx >= S.n_nodes) {
-                atomicOr(err, ERR_BAD_INDEX);
-                return true;
-            }
-            fetch_node_async(S, idx, nbuf, stride);
-        }
+// One node visit of this lane's ray, after pool_tris; true when the ray is
+// finished.
+template <int STACK>
+SRT_DEV bool trav_step(const DevScene& S, TravState& T, uint2* stack, int stride, uint32_t* err, uint32_t& n_nodes) {
+    const uint32_t oct = (T.axes >> 8) & 7u;
+    if ((T.g.y & 0xFF000000u) == 0u) {
+        if (T.sp == 0) return true;
+        --T.sp;
+        T.g = stack[T.sp * stride];
     }
-#if SRT_TRAV_ONE_TRI_PER_STEP
-    // one item per step: a triangle if one is pending, else a node, so a lane
-    // with a long triangle list does not hold up the lanes visiting nodes
-    const bool tri_step = T.tg.y != 0u;
-    for (int once = 0; once < 1 && T.tg.y != 0u; ++once) {
-#else
-    while (T.tg.y != 0u) {
-#endif
-        int b = __ffs(T.tg.y) - 1;
-        T.tg.y &= T.tg.y - 1u;
-        const TriSlot* ts = S.tris + T.tg.x + (uint32_t)b;
-        float4 a0 = __ldg(&ts->v0), a1 = __ldg(&ts->v1), a2 = __ldg(&ts->v2);
-        ++n_tris;
-        float t, tu, tv;
-        if (!tri_test(xyz(a0), xyz(a1), xyz(a2), T.o, kx, ky, kz, T.sx, T.sy, T.sz, T.tmin, T.tbest, t, tu, tv))
-            continue;
-        uint32_t id = __float_as_uint(a0.w);
-        if (ANY) {
-            if (PF && have) cp_async_wait_all();  // no copy into the slot outlives the ray
-            T.best = id;
-            T.tbest = t;
-            if (!kSync) return true;
-            any_hit = true;
-            break;
-        }
-        if (t < T.tbest || id < T.best) {  // (t, id) lexicographic; t <= tbest holds here
-            T.tbest = t;
-            T.best = id;
-            T.bu = tu;
-            T.bv = tv;
-        }
-    }
-
-#if SRT_TRAV_ONE_TRI_PER_STEP
-    if (tri_step) return false;
-#endif
-    if (PF) {
-        if (!have) return true;
-        cp_async_wait_all();
-        ++n_nodes;
-        node_children(nbuf[0], nbuf[stride], nbuf[2 * stride], nbuf[3 * stride], nbuf[4 * stride], T.o, T.idir, oct,
-                      T.tmin, T.tbest, T.g, T.tg);
-        return false;
-    }
-    if constexpr (kSync) {
-        // the same steps with every exit (an any-hit, the end of the tree, an
-        // error) deferred past one __syncwarp, which every lane that entered
-        // the step reaches (nothing above returns), so that the node fetch and
-        // slab tests run with all lanes still tracing at once
-        bool fin = ANY && any_hit;
-        uint32_t idx = 0u;
-        if (!fin && (T.g.y & 0xFF000000u) == 0u) fin = !trav_pop(T, stack, stride);
-        if (!fin) {
-            const int bit = 31 - __clz(T.g.y & 0xFF000000u);
-            T.g.y &= ~(1u << bit);
-            const uint32_t slot = (uint32_t)(bit - 24) ^ (oct ^ 7u);
-            idx = T.g.x + __popc(T.g.y & ((1u << slot) - 1u) & 0xFFu);
-            if ((T.g.y & 0xFF000000u) && !trav_push<STACK>(T, stack, stride)) {
-                atomicOr(err, ERR_STACK_OVERFLOW);
-                fin = true;
-            }
-            if (!fin && idx >= S.n_nodes) {
-                atomicOr(err, ERR_BAD_INDEX);
-                fin = true;
-            }
-        }
-        __syncwarp(entered);
-        if (fin) return true;
-        const uint4* np = reinterpret_cast<const uint4*>(S.nodes + idx);
-        uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
-        ++n_nodes;
-        node_children(w0, w1, w2, w3, w4, T.o, T.idir, oct, T.tmin, T.tbest, T.g, T.tg);
-        return false;
-    }
-    if ((T.g.y & 0xFF000000u) == 0u && !trav_pop(T, stack, stride)) return true;
-    int bit = 31 - __clz(T.g.y & 0xFF000000u);
+    const int bit = 31 - __clz(T.g.y & 0xFF000000u);
     T.g.y &= ~(1u << bit);
-    uint32_t slot = (uint32_t)(bit - 24) ^ (oct ^ 7u);
-    uint32_t idx = T.g.x + __popc(T.g.y & ((1u << slot) - 1u) & 0xFFu);
-    if ((T.g.y & 0xFF000000u) && !trav_push<STACK>(T, stack, stride)) {
-        atomicOr(err, ERR_STACK_OVERFLOW);
-        return true;
+    const uint32_t slot = (uint32_t)(bit - 24) ^ (oct ^ 7u);
+    const uint32_t idx = T.g.x + __popc(T.g.y & ((1u << slot) - 1u) & 0xFFu);
+    if (T.g.y & 0xFF000000u) {
+        if (T.sp >= STACK) {
+            atomicOr(err, ERR_STACK_OVERFLOW);
+            return true;
+        }
+        stack[T.sp * stride] = T.g;
+        ++T.sp;
     }
     if (idx >= S.n_nodes) {
         atomicOr(err, ERR_BAD_INDEX);
         return true;
     }
     const uint4* np = reinterpret_cast<const uint4*>(S.nodes + idx);
-    uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
+    const uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
     ++n_nodes;
     node_children(w0, w1, w2, w3, w4, T.o, T.idir, oct, T.tmin, T.tbest, T.g, T.tg);
     return false;

@@ -26,14 +26,13 @@
 #ifndef SRT_TRACE_MULTI_BLOCKS
 #define SRT_TRACE_MULTI_BLOCKS SRT_TRACE_MIN_BLOCKS
 #endif
-// resident blocks of the persistent kernel (k_trace_pt) per SM: 9 caps it at
-// 56 registers without spills of the closest-hit form (a 4-byte spill in the
-// any-hit form); config-2 frame 9.16 vs 9.43 ms with 8 (closest-hit bounces
-// 1-4 6 % faster, photon pass 2.45 vs 2.54 ms).  The one-ray-per-thread
-// kernel stays at 8 (bounce 0 0.44 vs 0.42 ms with 9); 10 blocks (48
-// registers) spill: 9.43 ms.
+// resident blocks of the persistent kernel (k_trace_pt) per SM.  With pooled
+// triangle tests in both forms, 9 / 8 / 7 (56 / 64 / 72 registers): config-2
+// closest hits 3.06 / 2.99 / 3.05 ms, caustic slab 1.36 / 1.34 / 1.35, Cornell
+// 640x480 0.72 / 0.68 / 0.65, config 1 frame - / 0.682 / 0.661; frames of config 2
+// - / 6.64 / 6.78 ms, caustic slab - / 3.86 / 3.89.
 #ifndef SRT_TRACE_PT_BLOCKS
-#define SRT_TRACE_PT_BLOCKS 9
+#define SRT_TRACE_PT_BLOCKS 8
 #endif
 // idle lanes that trigger a refill of the warp: closest-hit and any-hit
 // kernels (config-2 frame, refill at 4 / 6 / 8 / 12 / 16 / 20 idle lanes for
@@ -46,7 +45,7 @@
 #define SRT_TRACE_REFILL_ANY 12
 #endif
 // k_trace_pt traces a ray on eight lanes (trace_groups) when the launch has at
-// most this many rays per group of its resident warps (2: 42,624 rays).  Such a
+// most this many rays per group of its resident warps (2: 37,888 rays).  Such a
 // launch lasts as long as its longest rays: one ray per lane took 53 us for 44
 // photon rays and 0.13-0.16 ms for 1k-59k camera rays of config 2.  Frames
 // without the tail kernel, at 0 / 1 / 2 / 4 / 8 / 16 rays per group: prism
@@ -74,35 +73,20 @@
 #ifndef SRT_PRIMARY_PERSISTENT
 #define SRT_PRIMARY_PERSISTENT 0
 #endif
-// photon rays in persistent warps (k_trace_pt) instead of one per thread:
-// with the warp-synchronous node visits the refill pays (photon pass 2.53 vs
-// 2.62 ms per config-2 frame; before it, 3.35 vs 3.15)
+// photon rays in persistent warps (k_trace_pt) instead of one per thread: the
+// refill pays (photon pass 2.53 vs 2.62 ms per config-2 frame)
 #ifndef SRT_PHOTON_PERSISTENT
 #define SRT_PHOTON_PERSISTENT 1
-#endif
-
-// Fetch the next node with cp.async into shared memory while the pending
-// triangle tests run (k_trace and k_trace_pt).
-#ifndef SRT_TRAV_PREFETCH
-#define SRT_TRAV_PREFETCH 0
 #endif
 
 namespace srt {
 
 namespace {
 
-constexpr bool kPrefetch = SRT_TRAV_PREFETCH != 0;
-constexpr bool kPool = SRT_TRAV_POOL != 0 && !kPrefetch;
-
-// Dynamic shared memory of a traversal block: the stacks, then (prefetch)
-// 5 x uint4 node slots per thread.
+// Dynamic shared memory of a traversal block: the stacks.
 template <int STACK>
 constexpr size_t trace_smem() {
-    return sizeof(uint2) * STACK * TRACE_BLOCK + (kPrefetch ? sizeof(uint4) * 5 * TRACE_BLOCK : 0);
-}
-template <int STACK>
-SRT_DEV uint4* node_slots(uint2* smem) {
-    return reinterpret_cast<uint4*>(smem + STACK * TRACE_BLOCK) + threadIdx.x;
+    return sizeof(uint2) * STACK * TRACE_BLOCK;
 }
 
 // One ray per thread, one launch over the whole queue.
@@ -122,8 +106,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, SRT_TRACE_MIN_BLOCKS)
     float t = 0.f, u = 0.f, v = 0.f;
     uint32_t prim;
     TravCounters tc{&stats->nodes_bounce[kind][bounce], &stats->tris_bounce[kind][bounce]};
-    bool h = traverse<ANY, COUNT, STACK, kPrefetch>(S, ray, stack_smem + threadIdx.x, TRACE_BLOCK, t, prim, u, v, err,
-                                                    tc, kPrefetch ? node_slots<STACK>(stack_smem) : nullptr);
+    bool h = traverse<ANY, COUNT, STACK>(S, ray, stack_smem + threadIdx.x, TRACE_BLOCK, t, prim, u, v, err, tc);
     if (ANY) {
         // shadow ray: unoccluded -> add its contribution (shader.wgsl:659-669)
         if (!h) {
@@ -215,6 +198,8 @@ __global__ void __launch_bounds__(TRACE_BLOCK, SRT_TRACE_PT_BLOCKS)
     }
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt = (1u << lane) - 1u;
+    __shared__ uint32_t pool_tasks[TRACE_BLOCK];
+    uint32_t* tasks = pool_tasks + (threadIdx.x & ~31u);
     TravState T;
     bool active = false, exhausted = false;
     uint32_t q = 0, id = 0, n_nodes = 0, n_tris = 0;
@@ -249,13 +234,10 @@ __global__ void __launch_bounds__(TRACE_BLOCK, SRT_TRACE_PT_BLOCKS)
             if (exhausted) break;
             continue;
         }
-        if (kPool && (ANY || SRT_TRAV_POOL >= 2)) {
-            // the triangles of the lanes' last node visits, dealt out over the warp
-            pool_tris<ANY>(S, T, active, n_tris);
-            if (ANY && active && T.best != MISS) active = false;  // occluded: nothing to add
-        }
-        if (active && trav_step<ANY, STACK, kPrefetch>(S, T, stack, TRACE_BLOCK, err, n_nodes, n_tris,
-                                                       kPrefetch ? node_slots<STACK>(stack_smem) : nullptr)) {
+        // the triangles of the lanes' last node visits, dealt out over the warp
+        pool_tris<ANY>(S, T, active, tasks, n_tris);
+        if (ANY && active && T.best != MISS) active = false;  // occluded: nothing to add
+        if (active && trav_step<STACK>(S, T, stack, TRACE_BLOCK, err, n_nodes)) {
             active = false;
             if (ANY) {
                 if (T.best == MISS) {
@@ -351,9 +333,8 @@ __global__ void __launch_bounds__(TRACE_BLOCK, SRT_TRACE_MIN_BLOCKS)
 // Persistent form of the batch's traversal (SRT_BATCH_TRACE_PT): the lanes
 // of a warp take rays from one virtual queue over every item's rays (no
 // padding) and keep their own scene, so a finished lane takes the next ray
-// whatever scene it belongs to; the steps are those of k_trace_pt (closest
-// hits with the warp-synchronous node visit, any-hit rays with pooled
-// triangle tests that read the owner's scene).
+// whatever scene it belongs to; the steps are those of k_trace_pt, with
+// pooled triangle tests that read the owner's scene.
 template <bool ANY, int STACK>
 __global__ void __launch_bounds__(TRACE_BLOCK, SRT_TRACE_MULTI_BLOCKS)
     k_trace_multi_pt(const MultiTraceItem* __restrict__ items, int n_items, uint32_t* __restrict__ fetch) {
@@ -373,6 +354,8 @@ __global__ void __launch_bounds__(TRACE_BLOCK, SRT_TRACE_MULTI_BLOCKS)
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt = (1u << lane) - 1u;
     uint2* stack = stack_smem + threadIdx.x;
+    __shared__ uint32_t pool_tasks[TRACE_BLOCK];
+    uint32_t* tasks = pool_tasks + (threadIdx.x & ~31u);
     DevScene S;  // this lane's scene: the fields traversal reads
     S.nodes = nullptr;
     S.tris = nullptr;
@@ -429,11 +412,9 @@ __global__ void __launch_bounds__(TRACE_BLOCK, SRT_TRACE_MULTI_BLOCKS)
             if (exhausted) break;
             continue;
         }
-        if (kPool && (ANY || SRT_TRAV_POOL >= 2)) {
-            pool_tris<ANY, true>(S, T, active, n_tris);
-            if (ANY && active && T.best != MISS) active = false;  // occluded: nothing to add
-        }
-        if (active && trav_step<ANY, STACK>(S, T, stack, TRACE_BLOCK, items[s].err, n_nodes, n_tris)) {
+        pool_tris<ANY, true>(S, T, active, tasks, n_tris);
+        if (ANY && active && T.best != MISS) active = false;  // occluded: nothing to add
+        if (active && trav_step<STACK>(S, T, stack, TRACE_BLOCK, items[s].err, n_nodes)) {
             active = false;
             finish(items[s]);
         }
