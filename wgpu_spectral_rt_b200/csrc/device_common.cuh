@@ -414,24 +414,24 @@ SRT_DEV uint32_t grid_hash(float3 p, float3 j, float cell, uint32_t hash_bits) {
 }
 
 // ------------------------------------------------------------------ camera ray (shader.wgsl:713-728)
-SRT_DEV void camera_ray(const srt_camera_uniform& cam, uint32_t x, uint32_t y, uint32_t w, uint32_t h,
-                        uint32_t& s, float3& o, float3& d) {
+// Element (r, c) of view_inv * proj_inv.
+SRT_DEV float camera_elem(const srt_camera_uniform& cam, uint32_t r, uint32_t c) {
     const float* vi = cam.view_inverse;
     const float* pi = cam.proj_inverse;
+    return vi[r] * pi[4u * c] + vi[4u + r] * pi[4u * c + 1u] + vi[8u + r] * pi[4u * c + 2u] +
+           vi[12u + r] * pi[4u * c + 3u];
+}
+// m: camera_elem(r, c) at m[4 r + c].
+SRT_DEV void camera_ray(const srt_camera_uniform& cam, const float* m, uint32_t x, uint32_t y, uint32_t w, uint32_t h,
+                        uint32_t& s, float3& o, float3& d) {
+    const float* vi = cam.view_inverse;
     float jx = rng_next(s);
     float jy = rng_next(s);
     float nx = ((float)x + jx) / (float)w * 2.0f - 1.0f;
     float ny = ((float)y + jy) / (float)h * 2.0f - 1.0f;
     float t[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        // row r of (view_inv * proj_inv), then times (nx, ny, 1, 1)
-        float m0 = vi[r] * pi[0] + vi[4 + r] * pi[1] + vi[8 + r] * pi[2] + vi[12 + r] * pi[3];
-        float m1 = vi[r] * pi[4] + vi[4 + r] * pi[5] + vi[8 + r] * pi[6] + vi[12 + r] * pi[7];
-        float m2 = vi[r] * pi[8] + vi[4 + r] * pi[9] + vi[8 + r] * pi[10] + vi[12 + r] * pi[11];
-        float m3 = vi[r] * pi[12] + vi[4 + r] * pi[13] + vi[8 + r] * pi[14] + vi[12 + r] * pi[15];
-        t[r] = m0 * nx + m1 * ny + m2 + m3;
-    }
+    for (int r = 0; r < 4; ++r) t[r] = m[4 * r] * nx + m[4 * r + 1] * ny + m[4 * r + 2] + m[4 * r + 3];
     o = f3(vi[12], vi[13], vi[14]);
     d = normalize(f3(t[0] / t[3], t[1] / t[3], t[2] / t[3]) - o);
 }

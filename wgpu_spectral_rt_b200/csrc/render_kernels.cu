@@ -559,8 +559,13 @@ SRT_DEV void tile_pixel(uint32_t q, uint32_t w, uint32_t h, uint32_t& x, uint32_
 __global__ void k_raygen(FrameArgs a) {
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t n = a.width * a.height;
-    if (q >= n) return;
     const srt_camera_uniform& cam = *a.cam;
+    // the frame's matrix, once per block instead of per pixel (1080p 47 -> 39 us;
+    // 31 us to write the paths' state)
+    __shared__ float m[16];
+    if (threadIdx.x < 16u) m[threadIdx.x] = camera_elem(cam, threadIdx.x >> 2, threadIdx.x & 3u);
+    __syncthreads();
+    if (q >= n) return;
     uint32_t x, y;
     if (SRT_RAYGEN_TILE) tile_pixel(q, a.width, a.height, x, y);
     else {
@@ -570,7 +575,7 @@ __global__ void k_raygen(FrameArgs a) {
     const uint32_t p = x + y * a.width;
     uint32_t s = pcg_hash(x + y * a.width + cam.frame_count * 927163u + a.seed);
     float3 o, d;
-    camera_ray(cam, x, y, a.width, a.height, s, o, d);
+    camera_ray(cam, m, x, y, a.width, a.height, s, o, d);
     float4 wl = sample_hero(s);
     a.pb.ray_o[p] = f4(o.x, o.y, o.z, 0.0001f);
     a.pb.ray_d[p] = f4(d.x, d.y, d.z, 100.0f);
@@ -776,21 +781,41 @@ template <bool GUIDE>
 SRT_DEV void shade_slot(const FrameArgs& a, uint32_t bounce, uint32_t id, bool valid) {
     VertexOut v;
     if (valid) v = shade_vertex<GUIDE, false>(a, id, bounce);
-    uint32_t slot = warp_push(v.alive, &a.counters->paths[bounce + 1]);
+    // the warp's places in its queues: one atomic instruction, a lane per queue
+    // (one after the other each waited for the last one's answer; config-2
+    // shading 1.331 -> 1.313 ms per frame)
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    const uint32_t m_alive = __ballot_sync(FULL, v.alive), m_shadow = __ballot_sync(FULL, v.shadow),
+                   m_dark = __ballot_sync(FULL, v.dark), m_guided = GUIDE ? __ballot_sync(FULL, v.guided) : 0u;
+    uint32_t* counter = &a.counters->paths[bounce + 1];
+    uint32_t add = m_alive;
+    if (lane == 1u) {
+        counter = &a.counters->shadow[bounce];
+        add = m_shadow;
+    } else if (lane == 2u) {
+        counter = &a.counters->dark[bounce];
+        add = m_dark;
+    } else if (GUIDE && lane == 3u) {
+        counter = &a.guide.gc->verts[bounce];
+        add = m_guided;
+    }
+    uint32_t base = 0u;
+    if (lane < (GUIDE ? 4u : 3u) && add != 0u) base = atomicAdd(counter, (uint32_t)__popc(add));
+    const uint32_t slot = __shfl_sync(FULL, base, 0) + __popc(m_alive & lt);
     if (v.alive) {
         a.pb.queue[(bounce + 1) & 1][slot] = id;
         if (a.ray_sort) a.pb.sort_keys[slot] = v.key;
     }
-    uint32_t sslot = warp_push(v.shadow, &a.counters->shadow[bounce]);
+    const uint32_t sslot = __shfl_sync(FULL, base, 1) + __popc(m_shadow & lt);
     if (v.shadow) {
         a.pb.sh_o[sslot] = f4(v.sh_o.x, v.sh_o.y, v.sh_o.z, 0.001f);
         a.pb.sh_d[sslot] = f4(v.sh_d.x, v.sh_d.y, v.sh_d.z, v.sh_tmax);
         a.pb.sh_c[sslot] = v.sh_c;
         a.pb.sh_id[sslot] = id;
     }
-    warp_push(v.dark, &a.counters->dark[bounce]);
     if (GUIDE) {
-        uint32_t gslot = warp_push(v.guided, &a.guide.gc->verts[bounce]);
+        const uint32_t gslot = __shfl_sync(FULL, base, 3) + __popc(m_guided & lt);
         if (v.guided) {
             a.guide.gv.p[gslot] = v.g_p;
             a.guide.gv.n[gslot] = v.g_n;
@@ -1184,7 +1209,10 @@ __global__ void k_test_math(int op, uint32_t n, const void* __restrict__ in, voi
             const uint32_t* p = ui + 5 * i;
             uint32_t s = p[4];
             float3 o, d;
-            camera_ray(*(const srt_camera_uniform*)aux, p[0], p[1], p[2], p[3], s, o, d);
+            const srt_camera_uniform& cam = *(const srt_camera_uniform*)aux;
+            float m[16];
+            for (uint32_t e = 0; e < 16u; ++e) m[e] = camera_elem(cam, e >> 2, e & 3u);
+            camera_ray(cam, m, p[0], p[1], p[2], p[3], s, o, d);
             float* r = fo + 7 * i;
             r[0] = o.x;
             r[1] = o.y;
