@@ -13,8 +13,8 @@
 // tile does once (ranking, look-back of 256 digits) at 1.7 tiles per SM for 1M
 // pairs.  Against three kernels per pass (tile histograms, a scan of every
 // digit's row, a scatter straight from registers), the whole device-resident
-// grid of 1,000,003 / 300,000 / 20,000 / 300 photons: 99 -> 89, 68 -> 61, 62 -> 45
-// and 54 -> 35 us; the photon pass of config 1 0.330 -> 0.305 ms.  Tiles of 2048 /
+// grid of 1,000,003 / 300,000 / 20,000 / 300 photons: 99 -> 81, 68 -> 58, 62 -> 46
+// and 54 -> 36 us; the photon pass of config 1 0.330 -> 0.305 ms.  Tiles of 2048 /
 // 8192 items kept in registers: 96, 96 us for the first.
 //
 // Tiles take their numbers from a counter in the order in which they start, so
@@ -107,8 +107,12 @@ __device__ __forceinline__ uint32_t rs_block_exclusive(uint32_t v, uint32_t* war
 // Items of this thread's status column before tile `tile`: look-back over the
 // words status[t * stride], t < tile, RS_WINDOW of them loaded at once (a load
 // takes an L2 round trip, and the prefix is many tiles away when all start
-// together).
-constexpr uint32_t RS_WINDOW = 16;
+// together; loads beyond it are wasted, and 256 digits of 245 tiles of them are
+// what a pass of 1M pairs waits for).  Windows of 2 / 3 / 4 / 5 / 6 / 8 / 16 / 32:
+// the device-resident grid of 1,000,003 photons 87.3 / 81.2 / 81.3 / 81.4 / 81.6 /
+// 86.5 / 89.0 / 97.2 us, of 300,000 62.2 / 58.3 / 58.5 / 57.9 / 58.0 / 58.8 / 61.4 /
+// 61.5, of 2^20 with 24-bit keys 132 / 129 / 129 / 128 / 130 / 132 / 139 / 147.
+constexpr uint32_t RS_WINDOW = 5;
 __device__ __forceinline__ uint32_t rs_look_back(const uint32_t* status, uint32_t stride, uint32_t tile,
                                                  uint32_t* gave_up) {
     uint32_t before = 0u;
