@@ -519,11 +519,12 @@ __global__ void __launch_bounds__(32 * SAH_SPLIT_WARPS)
     const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
     const uint32_t ti = blockIdx.x * SAH_SPLIT_WARPS + w;
     const bool valid = ti < n_tasks;
-    SahTask& T = tasks[valid ? ti : 0u];
-    const uint32_t first = T.first, count = valid ? T.count : 2u, split = T.split, node = T.node;
+    SahTask& T = tasks[valid ? ti : 0u];  // (read and written by valid warps only)
+    const uint32_t first = valid ? T.first : 0u, count = valid ? T.count : 2u, split = valid ? T.split : SAH_MEDIAN,
+                   node = valid ? T.node : 0u;
     uint32_t left = count / 2;  // median by position
     float3 clo[2] = {f3(0.f, 0.f, 0.f), f3(0.f, 0.f, 0.f)}, chi[2] = {f3(0.f, 0.f, 0.f), f3(0.f, 0.f, 0.f)};
-    bool median = !valid || split == SAH_MEDIAN;
+    bool median = split == SAH_MEDIAN;
     int bk = -1, bax = -1;
     if (!median) {
         const int NB = (int)T.nbins;  // the bin arrays' stride per axis
