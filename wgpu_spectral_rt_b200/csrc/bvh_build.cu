@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "bvh_build.h"
+#include "bvh_collapse.h"
 #include "dev_arena.h"
 #include "radix_sort.cuh"
 
@@ -133,31 +134,10 @@ struct Bvh2 {
     uint2* choice;     // internal: what attains them, a byte each
 };
 
-// Which binary nodes become wide ones, by the cost recurrence of Ylitie, Karras
-// and Laine (HPG 2017, section 3.1): cost[i] is the least surface-area cost of
-// the subtree as a forest of at most i roots, each a leaf (area x triangles x
-// COLLAPSE_TRI) or a wide node (area x COLLAPSE_NODE + its children's forest of
-// `width` roots).  choice byte i (i = 2 .. width): roots given to the left
-// child, 0: the same forest as i - 1; byte 0: 1 if the node alone is a leaf.
-// Against opening the child of largest area until a node is full, everywhere
-// (k_collapse still does at the top): config 2 186k instead of 267k nodes, closest
-// hits 3.26 -> 3.22 ms, shadow rays 1.95 -> 1.87; Cornell 640x480 0.73 -> 0.70 and
-// 0.47 -> 0.42, photon pass of the animated scene 0.94 -> 0.89.
-// Weight of a triangle 0.15 / 0.3 / 0.5 / 0.8 of a node: config 2 closest hits
-// 3.29 / 3.26 / 3.26 / 3.24 ms, shadow rays 1.93 / 1.95 / 1.96 / 1.99; animated
-// 1.01 / 1.00 / 1.00 / 1.00 and 0.54 / 0.54 / 0.57 / 0.57.
-#ifndef SRT_COLLAPSE_TRI
-#define SRT_COLLAPSE_TRI 0.3f
-#endif
-constexpr float COLLAPSE_NODE = 1.0f, COLLAPSE_TRI = SRT_COLLAPSE_TRI;
-
-__device__ __forceinline__ float box_area(float4 lo, float4 hi) {
-    const float x = hi.x - lo.x, y = hi.y - lo.y, z = hi.z - lo.z;
-    return x * y + y * z + z * x;
-}
+// Which binary nodes become wide ones (bvh_collapse.h).
 __device__ __forceinline__ void child_costs(const Bvh2& b, uint32_t ref, float4 lo, float4 hi, float* c) {
     if (ref & LEAF) {
-        const float l = box_area(lo, hi) * COLLAPSE_TRI;
+        const float l = collapse_area(hi.x - lo.x, hi.y - lo.y, hi.z - lo.z) * COLLAPSE_TRI;
         for (int i = 0; i < 7; ++i) c[i] = l;
     } else {
         const float4 p = __ldcg(&b.cost[2 * ref]), q = __ldcg(&b.cost[2 * ref + 1]);
@@ -172,48 +152,14 @@ __device__ __forceinline__ void child_costs(const Bvh2& b, uint32_t ref, float4 
 }
 __device__ void collapse_costs(const Bvh2& b, uint32_t node, uint4 nd, float4 a0, float4 a1, float4 c0, float4 c1,
                                float4 lo, float4 hi, int width, uint32_t leaf_max) {
-    float l[7], r[7], best[9];
+    float l[7], r[7], cost[7];
+    uint32_t byte[8];
     child_costs(b, nd.x, a0, a1, l);
     child_costs(b, nd.y, c0, c1, r);
-    uint32_t pick[9] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-#pragma unroll
-    for (int i = 2; i <= 8; ++i) {
-        best[i] = 3.4e38f;
-#pragma unroll
-        for (int k = 1; k < i; ++k) {
-            if (k > 7 || i - k > 7) continue;
-            const float c = l[k - 1] + r[i - k - 1];
-            if (c < best[i]) {
-                best[i] = c;
-                pick[i] = (uint32_t)k;
-            }
-        }
-    }
-    const float area = box_area(lo, hi);
-    const uint32_t count = nd.w - nd.z + 1u;
-    float wide = best[8];
-#pragma unroll
-    for (int i = 2; i < 8; ++i)
-        if (i == width) wide = best[i];
-    best[1] = area * COLLAPSE_NODE + wide;
-    uint32_t leaf = 0u;
-    if (count <= leaf_max && area * (float)count * COLLAPSE_TRI <= best[1]) {
-        best[1] = area * (float)count * COLLAPSE_TRI;
-        leaf = 1u;
-    }
-    // the wide node's own distribution is kept even where fewer roots cost as little
-    uint32_t byte[8];
-    byte[0] = leaf;
-#pragma unroll
-    for (int i = 2; i <= 8; ++i) {
-        byte[i - 1] = pick[i];
-        if (i < 8 && i < width && !(best[i] < best[i - 1])) {
-            best[i] = best[i - 1];
-            byte[i - 1] = 0u;
-        }
-    }
-    b.cost[2 * node] = make_float4(best[1], best[2], best[3], best[4]);
-    b.cost[2 * node + 1] = make_float4(best[5], best[6], best[7], 0.f);
+    collapse_choose(l, r, collapse_area(hi.x - lo.x, hi.y - lo.y, hi.z - lo.z), nd.w - nd.z + 1u, width, leaf_max, cost,
+                    byte);
+    b.cost[2 * node] = make_float4(cost[0], cost[1], cost[2], cost[3]);
+    b.cost[2 * node + 1] = make_float4(cost[4], cost[5], cost[6], 0.f);
     b.choice[node] = make_uint2(byte[0] | (byte[1] << 8) | (byte[2] << 16) | (byte[3] << 24),
                                 byte[4] | (byte[5] << 8) | (byte[6] << 16) | (byte[7] << 24));
 }
@@ -221,6 +167,13 @@ __device__ __forceinline__ uint32_t choice_of(const Bvh2& b, uint32_t ref, int i
     const uint2 c = b.choice[ref];
     return ((i <= 4 ? c.x >> (8 * (i - 1)) : c.y >> (8 * (i - 5)))) & 0xFFu;
 }
+struct Bvh2Tree {  // the binary tree as collapse_expand reads it
+    const Bvh2& b;
+    __device__ __forceinline__ bool leaf(uint32_t ref) const { return (ref & LEAF) != 0u; }
+    __device__ __forceinline__ uint32_t left(uint32_t ref) const { return b.inode[ref].x; }
+    __device__ __forceinline__ uint32_t right(uint32_t ref) const { return b.inode[ref].y; }
+    __device__ __forceinline__ uint32_t choice(uint32_t ref, int i) const { return choice_of(b, ref, i); }
+};
 
 __global__ void k_karras(const uint32_t* __restrict__ keys, int n, Bvh2 b) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -945,10 +898,8 @@ __global__ void k_collapse(Bvh2 b, const uint2* __restrict__ qin, uint32_t n_in,
     if (e >= n_in) return;
     uint2 q = qin[e];
     uint32_t refs[8];
-    int roots[8];  // how many roots refs[c] may become
     int nc = 1;
     refs[0] = q.x;
-    roots[0] = 1;
     const uint32_t below = (q.x & LEAF) ? 1u : b.inode[q.x].w - b.inode[q.x].z + 1u;
     if (!(q.x & LEAF) && below > tri_cap / 2u) {
         // a node over more than half of the triangles: the child of largest
@@ -982,30 +933,9 @@ __global__ void k_collapse(Bvh2 b, const uint2* __restrict__ qin, uint32_t n_in,
             refs[nc++] = nd.y;
         }
     } else if (!(q.x & LEAF)) {
-        // the forest of `width` roots that collapse_costs chose
-        const uint4 nd = b.inode[q.x];
-        const int k = (int)choice_of(b, q.x, width);
-        refs[0] = nd.x;
-        roots[0] = k;
-        refs[1] = nd.y;
-        roots[1] = width - k;
-        nc = 2;
-        for (int c = 0; c < nc;) {
-            if (roots[c] == 1 || (refs[c] & LEAF)) {
-                ++c;
-                continue;
-            }
-            const int k = (int)choice_of(b, refs[c], roots[c]);
-            if (k == 0) {
-                --roots[c];
-                continue;
-            }
-            const uint4 nd = b.inode[refs[c]];
-            refs[nc] = nd.y;
-            roots[nc++] = roots[c] - k;
-            refs[c] = nd.x;
-            roots[c] = k;
-        }
+        bool ok = true;
+        nc = collapse_expand(Bvh2Tree{b}, q.x, width, refs, ok);
+        if (!ok) atomicOr(err, ERR_BAD_INDEX);
     }
     // children boxes, counts and node box
     float3 clo[8], chi[8];
