@@ -1,7 +1,7 @@
-"""The two functions that pick the wide tree's nodes (bvh_collapse.h), compiled
-for the host: over boxes of any size, infinite and NaN ones included, every
-choice is a split of its roots, no node gets more than `width` children, and
-the wide nodes cover every leaf exactly once."""
+"""The functions that pick the wide tree's nodes (bvh_collapse.h), compiled for
+the host: over boxes of any size, infinite and NaN ones included, every choice
+is a split of its roots, no node gets more than `width` children, the wide
+nodes cover every leaf exactly once, and every child has a slot of its own."""
 from __future__ import annotations
 
 import ctypes as C
@@ -103,16 +103,22 @@ extern "C" int collapse_tree(const float* leaves, uint32_t n, int split, int wid
         return 0;
     } catch (const std::out_of_range&) { return 3; } catch (const std::logic_error&) { return 4; }
 }
+extern "C" void slots(int nc, const float* d, int* child_in) { collapse_slots(nc, (const float (*)[3])d, child_in); }
 """
 
 
 @pytest.fixture(scope="module")
-def collapse(tmp_path_factory):
+def library(tmp_path_factory):
     d = tmp_path_factory.mktemp("collapse")
     (d / "collapse.cpp").write_text(SOURCE)
     subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", f"-I{ROOT}/wgpu_spectral_rt_b200/csrc",
                     str(d / "collapse.cpp"), "-o", str(d / "collapse.so")], check=True, timeout=120)
-    fn = C.CDLL(str(d / "collapse.so")).collapse_tree
+    return C.CDLL(str(d / "collapse.so"))
+
+
+@pytest.fixture(scope="module")
+def collapse(library):
+    fn = library.collapse_tree
 
     def run(boxes, split=0, width=8, leaf_max=2):
         n = len(boxes)
@@ -157,3 +163,20 @@ def test_all_boxes_beyond_the_largest_area(collapse):
     err, seen, out = collapse(boxes)
     assert err == 0 and np.all(seen == 1)
     assert out[1] <= 6  # full nodes: 8^4 > 600 leaves
+
+
+@pytest.mark.parametrize("value", [0.0, 1.0, 3e38, -3.4e38, np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("nc", [1, 2, 7, 8])
+def test_every_child_gets_a_slot_of_its_own(library, nc, value):
+    for where in ("one", "axis", "all"):
+        d = np.random.default_rng(nc).normal(size=(8, 3)).astype(np.float32)
+        if where == "one":
+            d[nc - 1] = value
+        elif where == "axis":
+            d[:, 1] = value
+        else:
+            d[:] = value
+        child_in = np.zeros(8, np.int32)
+        library.slots(nc, d.ctypes.data_as(C.c_void_p), child_in.ctypes.data_as(C.c_void_p))
+        assert sorted(child_in[child_in >= 0]) == list(range(nc))
+        assert np.count_nonzero(child_in < 0) == 8 - nc

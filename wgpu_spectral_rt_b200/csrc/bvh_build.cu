@@ -958,33 +958,16 @@ __global__ void k_collapse(Bvh2 b, const uint2* __restrict__ qin, uint32_t n_in,
         atomicOr(err, ERR_QUEUE_OVERFLOW);
         return;
     }
-    // slot assignment: slot s is visited first by rays whose octant is s
-    // (bit set = negative direction), which want the child lying farthest
-    // along +x/+y/+z for set bits; greedy on the best (child, slot) score.
-    float3 pc = (nlo + nhi) * 0.5f;
-    int slot_of[8];
+    const float3 pc = (nlo + nhi) * 0.5f;
+    float from_centre[8][3];
     int child_in[8];
-    for (int s = 0; s < 8; ++s) child_in[s] = -1;
-    for (int c = 0; c < nc; ++c) slot_of[c] = -1;
-    for (int it = 0; it < nc; ++it) {
-        float bs = -3.4e38f;
-        int bc = -1, bsl = -1;
-        for (int c = 0; c < nc; ++c) {
-            if (slot_of[c] >= 0) continue;
-            float3 d = (clo[c] + chi[c]) * 0.5f - pc;
-            for (int s = 0; s < 8; ++s) {
-                if (child_in[s] >= 0) continue;
-                float sc = ((s & 1) ? d.x : -d.x) + ((s & 2) ? d.y : -d.y) + ((s & 4) ? d.z : -d.z);
-                if (sc > bs) {
-                    bs = sc;
-                    bc = c;
-                    bsl = s;
-                }
-            }
-        }
-        slot_of[bc] = bsl;
-        child_in[bsl] = bc;
+    for (int c = 0; c < nc; ++c) {
+        const float3 d = (clo[c] + chi[c]) * 0.5f - pc;
+        from_centre[c][0] = d.x;
+        from_centre[c][1] = d.y;
+        from_centre[c][2] = d.z;
     }
+    collapse_slots(nc, from_centre, child_in);
     uint32_t meta[2] = {0u, 0u};
     uint32_t imask = 0u, int_rank = 0u, tri_off = 0u, used = 0u;
     float3 slo[8], shi[8];

@@ -118,4 +118,33 @@ SRT_HD int collapse_expand(const TREE& tree, uint32_t ref, int width, uint32_t* 
     return nc;
 }
 
+// Slots of a node's nc children, d[c]: the child's centre from the node's.  Slot s
+// is visited first by rays whose octant is s (bit set = negative direction), which
+// want the child lying farthest along +x/+y/+z for set bits; greedy on the best
+// (child, slot) score.  child_in[s]: the child in slot s, or -1.  Every child gets
+// a slot of its own whatever the scores are (a box without a centre scores NaN).
+SRT_HD void collapse_slots(int nc, const float (*d)[3], int* child_in) {
+    uint32_t placed = 0u;
+    for (int s = 0; s < 8; ++s) child_in[s] = -1;
+    for (int it = 0; it < nc; ++it) {
+        float bs = -3.4e38f;
+        int bc = -1, bsl = -1;
+        for (int c = 0; c < nc; ++c) {
+            if ((placed >> c) & 1u) continue;
+            for (int s = 0; s < 8; ++s) {
+                if (child_in[s] >= 0) continue;
+                const float sc = ((s & 1) ? d[c][0] : -d[c][0]) + ((s & 2) ? d[c][1] : -d[c][1]) +
+                                 ((s & 4) ? d[c][2] : -d[c][2]);
+                if (bc < 0 || sc > bs) {
+                    bs = sc;
+                    bc = c;
+                    bsl = s;
+                }
+            }
+        }
+        placed |= 1u << bc;
+        child_in[bsl] = bc;
+    }
+}
+
 }  // namespace srt
