@@ -739,7 +739,9 @@ __device__ void quantize_node(float3 nlo, float3 nhi, const float3* slo, const f
         scale[a] = __uint_as_float(ebyte[a] << 23);
         double lo_exact = (double)nlov[a];
         nlov[a] = (float)(lo_exact - 2.0 * (double)scale[a]);
-        while ((double)nlov[a] > lo_exact - 2.0 * (double)scale[a]) nlov[a] = nextafterf(nlov[a], -3.4e38f);
+        // (to -infinity: towards a finite end a corner near -3.4e38 would move away from it for good)
+        while ((double)nlov[a] > lo_exact - 2.0 * (double)scale[a])
+            nlov[a] = nextafterf(nlov[a], __int_as_float(0xFF800000));
     }
     uint32_t qlo[3][2] = {{0u, 0u}, {0u, 0u}, {0u, 0u}}, qhi[3][2] = {{0u, 0u}, {0u, 0u}, {0u, 0u}};
     for (int s = 0; s < 8; ++s) {
@@ -748,10 +750,8 @@ __device__ void quantize_node(float3 nlo, float3 nhi, const float3* slo, const f
         for (int a = 0; a < 3; ++a) {
             double sc = (double)scale[a];
             // one quantum of padding on each side
-            int ql = (int)floor(((double)lo3[a] - (double)nlov[a]) / sc) - 1;
-            int qh = (int)ceil(((double)hi3[a] - (double)nlov[a]) / sc) + 1;
-            ql = min(max(ql, 0), 255);
-            qh = min(max(qh, 0), 255);
+            int ql = (int)fmin(fmax(floor(((double)lo3[a] - (double)nlov[a]) / sc) - 1.0, 0.0), 255.0);
+            int qh = (int)fmin(fmax(ceil(((double)hi3[a] - (double)nlov[a]) / sc) + 1.0, 0.0), 255.0);
             while (ql > 0 && (double)nlov[a] + ql * sc > (double)lo3[a] - sc) --ql;
             while (qh < 255 && (double)nlov[a] + qh * sc < (double)hi3[a] + sc) ++qh;
             if ((double)nlov[a] + ql * sc > (double)lo3[a] - sc || (double)nlov[a] + qh * sc < (double)hi3[a] + sc)
