@@ -180,3 +180,17 @@ def test_every_child_gets_a_slot_of_its_own(library, nc, value):
         library.slots(nc, d.ctypes.data_as(C.c_void_p), child_in.ctypes.data_as(C.c_void_p))
         assert sorted(child_in[child_in >= 0]) == list(range(nc))
         assert np.count_nonzero(child_in < 0) == 8 - nc
+
+
+@pytest.mark.parametrize("kind", ["points", "line", "tiny"])
+def test_boxes_without_area_fill_their_nodes(collapse, kind):
+    boxes = np.zeros((200, 6), np.float32)
+    if kind == "line":
+        boxes[:, 0] = np.arange(200)
+        boxes[:, 3] = boxes[:, 0] + 0.5
+    elif kind == "tiny":
+        boxes = _boxes(200) * np.float32(1e-24)
+    for split, levels in ((0, 3), (1, 30)):  # 8^3 > 200; 7 more leaves per node of a chain, as it is opened from its end
+        err, seen, out = collapse(boxes, split)
+        assert err == 0 and np.all(seen == 1)
+        assert out[1] <= levels

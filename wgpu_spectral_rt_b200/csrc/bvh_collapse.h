@@ -32,12 +32,14 @@ namespace srt {
 constexpr float COLLAPSE_NODE = 1.0f, COLLAPSE_TRI = SRT_COLLAPSE_TRI;
 // Areas are clamped, so that the costs are finite and ordered whatever the
 // boxes are (a corner at 1e20 has an infinite area, a NaN one none): the cost of
-// 2^30 triangles stays below 1.4e37.
-constexpr float COLLAPSE_AREA_MAX = 1e28f;
+// 2^30 triangles stays below 1.4e37.  No area is zero: where all boxes are points
+// or lines along an axis, every forest would cost the same, wide nodes would get
+// two children, and a chain of 40 splits a tree too deep for traversal.
+constexpr float COLLAPSE_AREA_MIN = 1e-36f, COLLAPSE_AREA_MAX = 1e28f;
 
-// Half the surface of a box of extents x, y, z, clamped; NaN counts as 0.
+// Half the surface of a box of extents x, y, z, clamped; NaN counts as the least.
 SRT_HD float collapse_area(float x, float y, float z) {
-    return fminf(fmaxf(x * y + y * z + z * x, 0.0f), COLLAPSE_AREA_MAX);
+    return fminf(fmaxf(x * y + y * z + z * x, COLLAPSE_AREA_MIN), COLLAPSE_AREA_MAX);
 }
 
 // From the children's costs l[0..6] and r[0..6] (1 .. 7 roots): the node's
