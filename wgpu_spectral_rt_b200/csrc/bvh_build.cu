@@ -889,11 +889,12 @@ __global__ void k_expand_lights(const LightInst* __restrict__ li, const uint8_t*
 }
 
 // One thread per 8-wide node of this level: queue entries (bvh2 ref, node).
+// Nodes over more than `open_above` triangles open their largest children.
 __global__ void k_collapse(Bvh2 b, const uint2* __restrict__ qin, uint32_t n_in, uint2* __restrict__ qout,
                            uint32_t* __restrict__ n_out, Node8* __restrict__ nodes, uint32_t* __restrict__ node_alloc,
                            uint32_t node_cap, TriSlot* __restrict__ tris_out, uint32_t* __restrict__ tri_alloc,
                            uint32_t tri_cap, const TriSlot* __restrict__ flat, const uint32_t* __restrict__ sorted_tri,
-                           uint32_t* __restrict__ err, int width, uint32_t leaf_max) {
+                           uint32_t* __restrict__ err, int width, uint32_t leaf_max, uint32_t open_above) {
     uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n_in) return;
     uint2 q = qin[e];
@@ -901,9 +902,9 @@ __global__ void k_collapse(Bvh2 b, const uint2* __restrict__ qin, uint32_t n_in,
     int nc = 1;
     refs[0] = q.x;
     const uint32_t below = (q.x & LEAF) ? 1u : b.inode[q.x].w - b.inode[q.x].z + 1u;
-    if (!(q.x & LEAF) && below > tri_cap / 2u) {
-        // a node over more than half of the triangles: the child of largest
-        // area opened until it is full.  The recurrence would make the big flat
+    if (!(q.x & LEAF) && below > open_above) {
+        // the child of largest area opened until the node is full: a node over
+        // more than half of the triangles, or every one (build_bvh8).  The recurrence would make the big flat
         // leaves (walls) its children, where the quanta are coarsest and every
         // ray that starts on a wall meets its box: with it at the root too,
         // bounce 0 of config 2 0.342 vs 0.325 ms, its shadow rays 1.94 vs 1.87 ms
@@ -948,7 +949,8 @@ __global__ void k_collapse(Bvh2 b, const uint2* __restrict__ qin, uint32_t n_in,
         ref_range(b, refs[c], cfirst[c], ccount[c]);
         nlo = f3(fminf(nlo.x, clo[c].x), fminf(nlo.y, clo[c].y), fminf(nlo.z, clo[c].z));
         nhi = f3(fmaxf(nhi.x, chi[c].x), fmaxf(nhi.y, chi[c].y), fmaxf(nhi.z, chi[c].z));
-        is_leaf[c] = (refs[c] & LEAF) || (ccount[c] <= leaf_max && choice_of(b, refs[c], 1) != 0u);
+        is_leaf[c] = (refs[c] & LEAF) ||
+                     (ccount[c] <= leaf_max && (open_above == 0u || choice_of(b, refs[c], 1) != 0u));
         if (is_leaf[c]) n_tri += ccount[c];
         else ++n_int;
     }
@@ -1132,36 +1134,41 @@ cudaError_t build_bvh8(const BvhInputs& in, cudaStream_t st, BvhOutputs* out, st
         k_refit<<<grid, B, 0, st>>>(flat, sv, (int)n, b, width, leaf_max);
         ++out->kernel_launches;
         CK(cudaGetLastError());
-        // collapse, level by level; node 0 is the root
-        uint2 root = make_uint2(n > 1 ? 0u : LEAF, 0u);
-        uint32_t init_counts[4] = {1u, 0u, 0u, 0u};  // node alloc, tri alloc, queue out count, pad
-        CK(cudaMemcpyAsync(qa, &root, sizeof(root), cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(counters, init_counts, sizeof(init_counts), cudaMemcpyHostToDevice, st));
-        uint32_t n_in = 1;
+        // collapse, level by level; node 0 is the root.  The recurrence is not
+        // bound to shallow trees (scenes of triangles whose sizes fall off
+        // geometrically: up to 1.3 times the levels); one too deep for
+        // traversal is collapsed again by opening the largest child everywhere.
         uint32_t depth = 0;
-        out->level_start[0] = 0u;
-        out->level_start[1] = 1u;
-        while (n_in > 0) {
-            CK(cudaMemsetAsync(counters + 2, 0, 4, st));
-            k_collapse<<<(n_in + 127) / 128, 128, 0, st>>>(b, qa, n_in, qb, counters + 2, out->nodes, counters,
-                                                           node_cap, out->tris, counters + 1, n, flat, sv, err,
-                                                           width, leaf_max);
-            ++out->kernel_launches;
-            ++depth;
-            CK(cudaGetLastError());
-            uint32_t hc3[3];
-            CK(cudaMemcpyAsync(hc3, counters, sizeof(hc3), cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-            n_in = hc3[2];
-            if (depth < 65) out->level_start[depth + 1] = hc3[0];  // nodes of the next level end here
-            uint2* t = qa;
-            qa = qb;
-            qb = t;
-            if (depth > 64) {
-                if (msg) *msg = "BVH8 collapse exceeded 64 levels";
-                e = cudaErrorUnknown;
-                goto done;
+        for (uint32_t open_above : {n / 2u, 0u}) {
+            const uint2 root = make_uint2(n > 1 ? 0u : LEAF, 0u);
+            const uint32_t init_counts[4] = {1u, 0u, 0u, 0u};  // node alloc, tri alloc, queue out count, pad
+            CK(cudaMemcpyAsync(qa, &root, sizeof(root), cudaMemcpyHostToDevice, st));
+            CK(cudaMemcpyAsync(counters, init_counts, sizeof(init_counts), cudaMemcpyHostToDevice, st));
+            uint32_t n_in = 1;
+            depth = 0;
+            out->level_start[0] = 0u;
+            out->level_start[1] = 1u;
+            while (n_in > 0 && depth <= 64) {
+                CK(cudaMemsetAsync(counters + 2, 0, 4, st));
+                k_collapse<<<(n_in + 127) / 128, 128, 0, st>>>(b, qa, n_in, qb, counters + 2, out->nodes, counters,
+                                                               node_cap, out->tris, counters + 1, n, flat, sv, err,
+                                                               width, leaf_max, open_above);
+                ++out->kernel_launches;
+                ++depth;
+                CK(cudaGetLastError());
+                uint32_t hc3[3];
+                CK(cudaMemcpyAsync(hc3, counters, sizeof(hc3), cudaMemcpyDeviceToHost, st));
+                CK(cudaStreamSynchronize(st));
+                n_in = hc3[2];
+                if (depth < 65) out->level_start[depth + 1] = hc3[0];  // nodes of the next level end here
+                std::swap(qa, qb);
             }
+            if (depth <= (uint32_t)TRAV_STACK) break;
+        }
+        if (depth > 64) {
+            if (msg) *msg = "BVH8 collapse exceeded 64 levels";
+            e = cudaErrorUnknown;
+            goto done;
         }
         uint32_t hc[4], herr = 0;
         CK(cudaMemcpyAsync(hc, counters, sizeof(hc), cudaMemcpyDeviceToHost, st));
