@@ -524,6 +524,15 @@ srt_status srt_renderer_guide_set_weights(srt_renderer* r, const float* w, uint3
  * kernels' bounded waits; returns SRT_ERR_TIMEOUT, and the context stays
  * usable. */
 srt_status srt_test_wait_timeout(srt_ctx* ctx, uint32_t polls);
+/* The stable radix sort of (key, value) pairs by bits [0, end_bit) that the
+ * photon grid, the LBVH builder and the ray sort use (n = 1..2^24, host
+ * buffers).  Failure-path test: with first_tile > 0 the first pass's tile
+ * numbers start there, as if another sort had drawn the ones before; its
+ * bounded waits run out, blocks past the last tile leave, SRT_ERR_TIMEOUT is
+ * returned and the outputs mean nothing.  SRT_ERR_DEVICE_ASSERT if a word
+ * behind the sort's arrays was written. */
+srt_status srt_test_sort(srt_ctx* ctx, const uint32_t* keys, const uint32_t* vals, uint32_t n, int end_bit,
+                         uint32_t first_tile, uint32_t* keys_out, uint32_t* vals_out);
 srt_status srt_renderer_guide_get_state(srt_renderer* r, float* params, float* adam_m, float* adam_v,
                                         uint32_t* adam_step);
 srt_status srt_renderer_guide_set_state(srt_renderer* r, const float* params, const float* adam_m,

@@ -1,0 +1,38 @@
+"""The radix sort by itself (srt_test_sort): stable over whole tiles of 4096, at
+their edges and at more tiles than two look-back windows of 5, up to the
+largest photon grid; and where its tile numbers were drawn by another launch it
+reports that and writes nothing past its arrays."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TILE = 4096
+
+
+def _pairs(n, bits):
+    g = np.random.default_rng(n + bits)
+    return g.integers(0, 1 << bits, n, dtype=np.uint32), np.arange(n, dtype=np.uint32)
+
+
+@pytest.mark.parametrize("n", [1, TILE - 1, TILE, TILE + 1, 5 * TILE, 5 * TILE + 1, 10 * TILE + 1, 1 << 20])
+@pytest.mark.parametrize("bits", [5, 23, 32])
+def test_sort_is_stable(srt, ctx, n, bits):
+    keys, vals = _pairs(n, bits)
+    k, v = srt.sort_check(ctx, keys, vals, bits)
+    order = np.argsort(keys, kind="stable")
+    np.testing.assert_array_equal(k, keys[order])
+    np.testing.assert_array_equal(v, vals[order])
+
+
+@pytest.mark.parametrize("n,first", [(TILE, 1), (5 * TILE, 1), (5 * TILE, 3), (5 * TILE, 5), (10 * TILE + 1, 4),
+                                     (10 * TILE + 1, 11), (10 * TILE + 1, 245), (TILE, 0x7FFFFFFF)])
+def test_tile_numbers_of_another_launch(srt, ctx, n, first):
+    keys, vals = _pairs(n, 23)
+    with pytest.raises(srt.SrtError) as e:
+        srt.sort_check(ctx, keys, vals, 23, first)
+    assert e.value.status == 4  # SRT_ERR_TIMEOUT
+    k, _ = srt.sort_check(ctx, keys, vals, 23)
+    np.testing.assert_array_equal(k, np.sort(keys))

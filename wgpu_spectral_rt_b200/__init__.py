@@ -234,6 +234,7 @@ SIGNATURES = {
     "srt_renderer_guide_set_state": (_I, [_P, _P, _P, _P, _U32]),
     "srt_write_accum_f64": (_I, [_P, _P]),
     "srt_test_wait_timeout": (_I, [_P, _U32]),
+    "srt_test_sort": (_I, [_P, _P, _P, _U32, _I, _U32, _P, _P]),
     "srt_guide_test_train": (_I, [_P, _P, _P, _P, _U32, _F, _P, _P, _P, _P, _U32, _P, _P, _P, _P]),
     "srt_guide_test_train_tc": (_I, [_P, _P, _P, _P, _U32, _F, _P, _P, _P, _P, _U32, _P, _P, _P, _P]),
 }
@@ -741,6 +742,15 @@ def guide_default_weights(seed: int = 1) -> np.ndarray:
 def wait_timeout_check(ctx: Context, polls: int = 1000) -> None:
     """Runs a device wait that cannot complete (bounded by `polls`); raises SrtError with SRT_ERR_TIMEOUT."""
     _check(lib().srt_test_wait_timeout(ctx.h, polls), ctx.h)
+
+
+def sort_check(ctx: Context, keys: np.ndarray, vals: np.ndarray, end_bit: int = 32, first_tile: int = 0):
+    """The device radix sort over host arrays (srt_test_sort): sorted keys and values; with first_tile > 0 a sort
+    that another one disturbs, which raises SrtError with SRT_ERR_TIMEOUT."""
+    k, v = np.ascontiguousarray(keys, np.uint32), np.ascontiguousarray(vals, np.uint32)
+    ko, vo = np.empty_like(k), np.empty_like(v)
+    _check(lib().srt_test_sort(ctx.h, ptr(k), ptr(v), len(k), end_bit, first_tile, ptr(ko), ptr(vo)), ctx.h)
+    return ko, vo
 
 
 def guide_forward(ctx: Context, params: np.ndarray, x: np.ndarray, tcgen05: bool = False) -> np.ndarray:

@@ -1878,6 +1878,45 @@ extern "C" srt_status srt_test_wait_timeout(srt_ctx* c, uint32_t polls) {
     return check_device_error(c, c->d_err);
 }
 
+extern "C" srt_status srt_test_sort(srt_ctx* c, const uint32_t* keys, const uint32_t* vals, uint32_t n, int end_bit,
+                                    uint32_t first_tile, uint32_t* keys_out, uint32_t* vals_out) {
+    if (!c || !keys || !vals || !keys_out || !vals_out || n == 0 || n > (1u << 24) || end_bit < 1 || end_bit > 32)
+        return SRT_ERR_INVALID_ARG;
+    cudaSetDevice(c->device);
+    // every array is followed by words that nothing may write
+    constexpr size_t GUARD = 1u << 16;
+    constexpr uint32_t MARK = 0xA5A5A5A5u;
+    const size_t words = radix_scratch_words(n);
+    uint32_t *d[4] = {}, *scratch = nullptr, *sk = nullptr, *sv = nullptr, flag = 0;
+    DevArena mem;
+    for (uint32_t*& p : d) mem.add(&p, n + GUARD);
+    mem.add(&scratch, words + GUARD);
+    CUDA_TRY(c, dev_commit(mem));
+    for (uint32_t* p : d) CUDA_TRY(c, cudaMemsetAsync(p + n, MARK & 0xFF, 4 * GUARD, c->stream));
+    CUDA_TRY(c, cudaMemsetAsync(scratch + words, MARK & 0xFF, 4 * GUARD, c->stream));
+    CUDA_TRY(c, cudaMemcpyAsync(d[0], keys, 4ull * n, cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(c, cudaMemcpyAsync(d[1], vals, 4ull * n, cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(c, cudaMemsetAsync(scratch, 0, RS_HEAD * sizeof(uint32_t), c->stream));
+    const int passes = rs_passes(0, end_bit);
+    k_rs_count<<<std::min(rs_tiles(n), 592u), RS_THREADS, 0, c->stream>>>(d[0], nullptr, n, 0, passes, scratch);
+    // the first pass hands out tile numbers from first_tile on
+    CUDA_TRY(c, cudaMemcpyAsync(scratch + RS_TICKET, &first_tile, 4, cudaMemcpyHostToDevice, c->stream));
+    sort_passes(d[0], d[1], d[2], d[3], n, nullptr, 0, end_bit, scratch, c->stream, &sk, &sv);
+    CUDA_TRY(c, cudaGetLastError());
+    CUDA_TRY(c, cudaMemcpyAsync(&flag, scratch + RS_GAVE_UP, 4, cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(c, cudaMemcpyAsync(keys_out, sk, 4ull * n, cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(c, cudaMemcpyAsync(vals_out, sv, 4ull * n, cudaMemcpyDeviceToHost, c->stream));
+    std::vector<uint32_t> guard(GUARD);
+    for (int k = 0; k < 5; ++k) {
+        CUDA_TRY(c, cudaMemcpyAsync(guard.data(), k < 4 ? d[k] + n : scratch + words, 4 * GUARD, cudaMemcpyDeviceToHost,
+                                    c->stream));
+        CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+        for (uint32_t w : guard)
+            if (w != MARK) return fail(c, SRT_ERR_DEVICE_ASSERT, "the sort wrote past its arrays");
+    }
+    return flag ? fail(c, SRT_ERR_TIMEOUT, "the sort's bounded wait gave up") : SRT_OK;
+}
+
 extern "C" srt_status srt_renderer_guide_get_state(srt_renderer* r, float* params, float* adam_m, float* adam_v,
                                                    uint32_t* adam_step) {
     if (!r || !params || !adam_m || !adam_v || !adam_step) return SRT_ERR_INVALID_ARG;

@@ -19,7 +19,9 @@
 //
 // Tiles take their numbers from a counter in the order in which they start, so
 // the tiles a look-back waits for are running; its polls are bounded all the
-// same (RS_POLLS), and a tile that gives up sets RS_GAVE_UP in the scratch.
+// same (RS_POLLS), and a tile that gives up sets RS_GAVE_UP in the scratch, as
+// does a block whose number is none of a tile's (launches that share a scratch
+// overlap): the result is then to be dropped.
 // The element count may live in device memory (n_dev), so the same launches
 // serve a count produced on the GPU and can be captured in a CUDA graph; tiles
 // at or beyond the count exit at once.
@@ -163,6 +165,10 @@ static __global__ void __launch_bounds__(RS_THREADS) k_rs_pass(const uint32_t* _
     for (uint32_t d = tid; d < RS_WARPS * 128u; d += RS_THREADS) reinterpret_cast<uint32_t*>(&cnt[0][0])[d] = 0u;
     __syncthreads();
     const uint32_t tile = ticket;
+    if (tile >= tiles) {  // another launch drew from the same counter (calls that share a scratch overlap)
+        if (tid == 0) atomicOr(&scratch[RS_GAVE_UP], 1u);
+        return;
+    }
     const uint32_t tile_base = tile * (uint32_t)RS_TILE, items = min((uint32_t)RS_TILE, n - tile_base);
     // threads 0 .. 255: one digit each
     const bool digit = tid < 256u;

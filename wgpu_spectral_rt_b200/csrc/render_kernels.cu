@@ -424,6 +424,10 @@ __global__ void __launch_bounds__(RS_THREADS) k_deposit(FrameArgs a) {
     if (threadIdx.x == 0) ticket = atomicAdd(&a.ph.deposit[0], 1u);
     __syncthreads();
     const uint32_t tile = ticket, tiles = deposit_tiles(a.photons_per_frame);
+    if (tile >= tiles) {  // (one block per tile: its counter was not cleared)
+        if (threadIdx.x == 0) atomicOr(a.err, ERR_BAD_INDEX);
+        return;
+    }
     const uint32_t first = tile * DEPOSIT_TILE + threadIdx.x * 16u;
     const uint4 f = *reinterpret_cast<const uint4*>(a.ph.flags + first);  // (flags past the last emitter are clear)
     uint32_t stored = 0u;
