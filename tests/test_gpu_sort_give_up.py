@@ -1,7 +1,8 @@
 """The radix sort by itself (srt_test_sort): stable over whole tiles of 4096, at
 their edges and at more tiles than two look-back windows of 5, up to the
 largest photon grid; and where its tile numbers were drawn by another launch it
-reports that and writes nothing past its arrays."""
+reports that and writes nothing past its arrays.  What sorts reports a sort that
+gave up instead of using its result."""
 from __future__ import annotations
 
 import numpy as np
@@ -36,3 +37,22 @@ def test_tile_numbers_of_another_launch(srt, ctx, n, first):
     assert e.value.status == 4  # SRT_ERR_TIMEOUT
     k, _ = srt.sort_check(ctx, keys, vals, 23)
     np.testing.assert_array_equal(k, np.sort(keys))
+
+
+def test_lbvh_build_reports_a_sort_that_gave_up(srt, ctx, monkeypatch):
+    b = srt.SceneBuilder()
+    b.add_preset(srt.PRESET_CORNELL_BOX)
+    ctx.set_bvh_builder(srt.BVH_LBVH)
+    try:
+        scene = b.build(ctx)
+        monkeypatch.setenv("SRT_FAULT", "sort")
+        for build in (lambda: b.build(ctx), lambda: scene.rebuild_bvh(8)):
+            with pytest.raises(srt.SrtError) as e:
+                build()
+            assert e.value.status == 4  # SRT_ERR_TIMEOUT
+        monkeypatch.delenv("SRT_FAULT")
+        scene.rebuild_bvh(8)
+        b.build(ctx).close()
+        scene.close()
+    finally:
+        ctx.set_bvh_builder(srt.BVH_SAH)

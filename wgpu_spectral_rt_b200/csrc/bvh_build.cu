@@ -1085,6 +1085,14 @@ cudaError_t build_bvh8(const BvhInputs& in, cudaStream_t st, BvhOutputs* out, st
             ++out->kernel_launches;
             uint32_t* sk;
             out->kernel_launches += sort_pairs(keys, vals, keys2, vals2, n, nullptr, 0, 30, scratch, st, &sk, &sv);
+            uint32_t gave_up = 0;
+            CK(cudaMemcpyAsync(&gave_up, scratch + RS_GAVE_UP, 4, cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+            if (gave_up) {  // sk and sv may hold anything
+                if (msg) *msg = "the sort's bounded wait gave up";
+                e = cudaErrorTimeout;
+                goto done;
+            }
             if (n > 1) {
                 k_karras<<<(n - 1 + B - 1) / B, B, 0, st>>>(sk, (int)n, b);
                 ++out->kernel_launches;

@@ -28,7 +28,7 @@ namespace {
 std::string g_last_create_error;
 
 bool env_fault(const char* what) {
-    // Host-side fault injection for the error paths: SRT_FAULT=alloc|launch
+    // Host-side fault injection for the error paths: SRT_FAULT=alloc|launch (and sort: sort_fault)
     const char* f = std::getenv("SRT_FAULT");
     return f && std::strcmp(f, what) == 0;
 }
@@ -93,6 +93,11 @@ srt_status cuda_fail(srt_ctx* c, cudaError_t e, const char* where) {
         cudaError_t _e = (expr);                           \
         if (_e != cudaSuccess) return cuda_fail(ctx, _e, #expr); \
     } while (0)
+
+// Status of a failed tree build.
+srt_status build_status(cudaError_t e) {
+    return e == cudaErrorMemoryAllocation ? SRT_ERR_OOM : e == cudaErrorTimeout ? SRT_ERR_TIMEOUT : SRT_ERR_CUDA;
+}
 
 cudaError_t dev_commit(DevArena& a) {
     if (env_fault("alloc")) return cudaErrorMemoryAllocation;
@@ -515,7 +520,7 @@ srt_status scene_build_impl(srt_ctx* c, const srt_scene_arrays* a,
     s->n_inst = a->n_instances;
     std::string msg;
     cudaError_t e = build_bvh8(bi, st, &s->bvh, &msg);
-    if (e != cudaSuccess) return fail(c, e == cudaErrorMemoryAllocation ? SRT_ERR_OOM : SRT_ERR_CUDA, "BVH build: " + msg);
+    if (e != cudaSuccess) return fail(c, build_status(e), "BVH build: " + msg);
     if (s->bvh.depth > (uint32_t)TRAV_STACK)
         return fail(c, SRT_ERR_UNSUPPORTED, "BVH deeper than the traversal stack");
     launch_scatter_masks(s->bvh, s->inst, s->materials, s->bvh.scatter, st);
@@ -717,7 +722,7 @@ extern "C" srt_status srt_scene_rebuild_bvh(srt_scene* s, uint32_t width) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         cudaFree(nb.mem);
-        return fail(c, e == cudaErrorMemoryAllocation ? SRT_ERR_OOM : SRT_ERR_CUDA, "BVH rebuild: " + msg);
+        return fail(c, build_status(e), "BVH rebuild: " + msg);
     }
     cudaFree(s->bvh.mem);
     s->bvh = nb;

@@ -29,6 +29,8 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <cstdlib>
+#include <cstring>
 #include <cuda_runtime.h>
 
 namespace srt {
@@ -248,6 +250,13 @@ static __global__ void __launch_bounds__(RS_THREADS) k_rs_pass(const uint32_t* _
     }
 }
 
+// Host-side fault injection: with SRT_FAULT=sort every sort_pairs counts as one
+// whose bounded wait gave up.
+inline bool sort_fault() {
+    const char* f = std::getenv("SRT_FAULT");
+    return f && std::strcmp(f, "sort") == 0;
+}
+
 // Digit passes of a sort of bits [begin_bit, end_bit).
 constexpr int rs_passes(int begin_bit, int end_bit) { return (end_bit - begin_bit + 7) / 8; }
 
@@ -272,7 +281,8 @@ inline int sort_passes(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint3
 
 // Sorts bits [begin_bit, end_bit) of (keys, vals), ping-ponging with the
 // alternate buffers.  max_n (< 2^30) bounds the count for the launch grid;
-// n_dev (optional) holds the actual count.
+// n_dev (optional) holds the actual count.  The caller looks at
+// scratch[RS_GAVE_UP] before it uses the result.
 inline int sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint32_t max_n,
                       const uint32_t* n_dev, int begin_bit, int end_bit, uint32_t* scratch, cudaStream_t st,
                       uint32_t** out_keys, uint32_t** out_vals) {
@@ -282,6 +292,7 @@ inline int sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32
         k_rs_count<<<std::min(rs_tiles(max_n), 592u), RS_THREADS, 0, st>>>(keys, n_dev, max_n, begin_bit,
                                                                          rs_passes(begin_bit, end_bit), scratch);
         ++launches;
+        if (sort_fault()) cudaMemsetAsync(scratch + RS_GAVE_UP, 1, sizeof(uint32_t), st);
     }
     return launches + sort_passes(keys, vals, keys_alt, vals_alt, max_n, n_dev, begin_bit, end_bit, scratch, st, out_keys,
                                   out_vals);
