@@ -56,3 +56,37 @@ def test_lbvh_build_reports_a_sort_that_gave_up(srt, ctx, monkeypatch):
         scene.close()
     finally:
         ctx.set_bvh_builder(srt.BVH_SAH)
+
+
+def _frames(srt, ctx, scene, cam, w, h, flags, n=2):
+    r = srt.Renderer(ctx, scene, w, h, srt.default_params(max_depth=6, photons_per_frame=1 << 14, flags=flags))
+    try:
+        for f in range(n):
+            r.render(cam.build_uniform(w / h, f))
+        return r.read_accum()
+    finally:
+        r.close()
+
+
+@pytest.mark.parametrize("size", [(63, 65), (64, 64), (17, 241), (8193, 1)])  # 4095, 4096, 4097, 8193 paths
+def test_ray_sort_changes_no_image(srt, ctx, size):
+    b = srt.SceneBuilder()
+    cam = srt.CameraController(*b.add_preset(srt.PRESET_CORNELL_BOX))
+    scene = b.build(ctx)
+    plain = _frames(srt, ctx, scene, cam, *size, 0)
+    assert np.array_equal(_frames(srt, ctx, scene, cam, *size, srt.FLAG_RAY_SORT), plain)
+    scene.close()
+
+
+def test_frame_reports_a_ray_sort_that_gave_up(srt, ctx, monkeypatch):
+    b = srt.SceneBuilder()
+    cam = srt.CameraController(*b.add_preset(srt.PRESET_CORNELL_BOX))
+    scene = b.build(ctx)
+    plain = _frames(srt, ctx, scene, cam, 64, 48, 0)
+    monkeypatch.setenv("SRT_FAULT", "sort")
+    with pytest.raises(srt.SrtError) as e:
+        _frames(srt, ctx, scene, cam, 64, 48, srt.FLAG_RAY_SORT)
+    assert e.value.status == 4  # SRT_ERR_TIMEOUT
+    monkeypatch.delenv("SRT_FAULT")
+    assert np.array_equal(_frames(srt, ctx, scene, cam, 64, 48, srt.FLAG_RAY_SORT), plain)
+    scene.close()

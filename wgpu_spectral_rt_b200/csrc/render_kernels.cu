@@ -1108,6 +1108,14 @@ __global__ void k_finalize(FrameArgs a) {
                            (unsigned char)__float2uint_rn(clampf(fc.z, 0.f, 1.f) * 255.0f), 255);
 }
 
+// After the ray sort of the paths entering bounce + 1: where its bounded wait
+// gave up the queue may hold anything, so no path goes on and the frame reports it.
+__global__ void k_check_sort(FrameArgs a, uint32_t bounce) {
+    if (threadIdx.x != 0 || a.pb.sort_scratch[RS_GAVE_UP] == 0u || a.counters->paths[bounce + 1] == 0u) return;
+    a.counters->paths[bounce + 1] = 0u;
+    atomicOr(a.err, ERR_WAIT_TIMEOUT);
+}
+
 // One lane per bounce (a chain of loads per bounce on one thread took 6 us at
 // the end of every frame).
 __global__ void k_frame_stats(FrameArgs a) {
@@ -1311,6 +1319,8 @@ int launch_bounce(const FrameArgs& a, uint32_t bounce, cudaStream_t st, int stag
             launches += sort_pairs(a.pb.sort_keys, a.pb.queue[(bounce + 1) & 1], a.pb.sort_keys_alt,
                                    a.pb.sort_vals_alt, a.width * a.height, &a.counters->paths[bounce + 1], 0, 32,
                                    a.pb.sort_scratch, st, &sk, &sv);
+            k_check_sort<<<1, 32, 0, st>>>(a, bounce);
+            ++launches;
         }
     }
     if (stage == 3) launches += launch_trace_shadow(a, bounce, st);
