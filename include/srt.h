@@ -499,6 +499,7 @@ srt_status srt_photon_gather(srt_ctx* ctx, const srt_photon* photons, uint32_t n
  *  7 grid hash(position[3], frame bits, cell)     in f32[5] -> out u32[1]
  *  8 camera ray(cam uniform from `aux`, pixel x, y, width, height as bits, rng seed) in u32[5]
  *    -> out f32[7] origin[3] dir[3] rng out (bits)
+ *  9 every |f| below a bound (what shading may skip) in f32[5] = f[4], bound -> out u32[1] (0/1)
  * in/out strides are the per-op sizes above; n records. */
 srt_status srt_test_device_math(srt_ctx* ctx, int op, uint32_t n, const void* in, void* out, const void* aux);
 

@@ -713,7 +713,7 @@ def photon_gather(ctx: Context, photons: np.ndarray, queries: np.ndarray, frame:
 
 
 MATH_SIZES = {0: (4, 4), 1: (4, 12), 2: (8, 4), 3: (28, 16), 4: (36, 16), 5: (4, 20), 6: (96, 40), 7: (20, 4),
-              8: (20, 28)}
+              8: (20, 28), 9: (20, 4)}
 
 
 def device_math(ctx: Context, op: int, inp: np.ndarray, aux: CameraUniform | None = None) -> np.ndarray:
@@ -721,7 +721,7 @@ def device_math(ctx: Context, op: int, inp: np.ndarray, aux: CameraUniform | Non
     isz, osz = MATH_SIZES[op]
     a = np.ascontiguousarray(inp)
     n = a.nbytes // isz
-    out = np.zeros(n * osz // 4, np.uint32 if op in (0, 7) else np.float32)
+    out = np.zeros(n * osz // 4, np.uint32 if op in (0, 7, 9) else np.float32)
     _check(lib().srt_test_device_math(ctx.h, op, n, ptr(a), ptr(out), C.byref(aux) if aux is not None else None), ctx.h)
     return out.reshape(n, osz // 4)
 

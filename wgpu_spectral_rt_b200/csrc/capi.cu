@@ -1807,9 +1807,9 @@ extern "C" srt_status srt_trace_rays(srt_scene* s, const srt_ray* rays, uint32_t
 }
 
 extern "C" srt_status srt_test_device_math(srt_ctx* c, int op, uint32_t n, const void* in, void* out, const void* aux) {
-    static const size_t in_sz[9] = {4, 4, 8, 28, 36, 4, 96, 20, 20};
-    static const size_t out_sz[9] = {4, 12, 4, 16, 16, 20, 40, 4, 28};
-    if (!c || op < 0 || op > 8 || (n && (!in || !out)) || (op == 8 && !aux)) return SRT_ERR_INVALID_ARG;
+    static const size_t in_sz[10] = {4, 4, 8, 28, 36, 4, 96, 20, 20, 20};
+    static const size_t out_sz[10] = {4, 12, 4, 16, 16, 20, 40, 4, 28, 4};
+    if (!c || op < 0 || op > 9 || (n && (!in || !out)) || (op == 8 && !aux)) return SRT_ERR_INVALID_ARG;
     cudaSetDevice(c->device);
     if (n == 0) return SRT_OK;
     void *din = nullptr, *dout = nullptr, *daux = nullptr;

@@ -111,6 +111,11 @@ SRT_DEV float4 operator/(float4 a, float4 b) { return f4(a.x / b.x, a.y / b.y, a
 SRT_DEV float4 operator*(float4 a, float s) { return f4(a.x * s, a.y * s, a.z * s, a.w * s); }
 SRT_DEV float4 operator/(float4 a, float s) { return f4(a.x / s, a.y / s, a.z / s, a.w / s); }
 SRT_DEV float max4(float4 a) { return fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)); }
+// Every component lies within (-bound, bound); a NaN among them does not
+// (max4 drops one beside a number).
+SRT_DEV bool within4(float4 a, float bound) {
+    return fabsf(a.x) < bound && fabsf(a.y) < bound && fabsf(a.z) < bound && fabsf(a.w) < bound;
+}
 SRT_DEV float clampf(float x, float lo, float hi) { return fminf(fmaxf(x, lo), hi); }
 SRT_DEV float sq(float x) { return x * x; }
 SRT_DEV float signf(float x) { return x > 0.f ? 1.f : (x < 0.f ? -1.f : 0.f); }

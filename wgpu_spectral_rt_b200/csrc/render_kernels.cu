@@ -701,7 +701,7 @@ SRT_DEV VertexOut shade_vertex(const FrameArgs& a, uint32_t id, uint32_t bounce)
             const float4 f = thr * (spec / PI);
             const float inf = __int_as_float(0x7F800000);
             // an empty range adds zeros (unless a factor is not finite)
-            if (rg.y > rg.x || !(max4(f) < inf) || !(fabsf(k.density) < inf)) {
+            if (rg.y > rg.x || !within4(f, inf) || !(fabsf(k.density) < inf)) {
                 if (TAIL) {
                     out.gather = true;
                     out.ga_range = rg;
@@ -731,7 +731,7 @@ SRT_DEV VertexOut shade_vertex(const FrameArgs& a, uint32_t id, uint32_t bounce)
             // every factor of its contribution finite).  Config 2: shadow rays
             // 2.33 -> 1.96 ms per frame, the frame 7.84 -> 7.52 ms; animated
             // 512x384 shadow rays 0.66 -> 0.60 ms.
-            out.dark = ct == 0.0f && max4(f) < 1e15f && ls.pdf > 1e-30f && ls.emission.x >= 1.0f &&
+            out.dark = ct == 0.0f && within4(f, 1e15f) && ls.pdf > 1e-30f && ls.emission.x >= 1.0f &&
                        ls.emission.x <= 1e6f && fabsf(ls.emission.y) < 1e15f;
             if (!out.dark) {
                 float bpdf = ct / PI;
@@ -1233,6 +1233,10 @@ __global__ void k_test_math(int op, uint32_t n, const void* __restrict__ in, voi
             r[4] = d.y;
             r[5] = d.z;
             r[6] = __uint_as_float(s);
+        } break;
+        case 9: {
+            const float* p = fi + 5 * i;
+            uo[i] = within4(f4(p[0], p[1], p[2], p[3]), p[4]) ? 1u : 0u;
         } break;
         default:
             break;
