@@ -8,7 +8,7 @@
 // temporary storage from one file-scope __device__ array of fixed size, and
 // works only on buffers the caller already owns.
 //
-// The array (GRID_NOALLOC_SCRATCH_WORDS 32-bit words, 17 MiB) lives in
+// The array (GRID_NOALLOC_SCRATCH_WORDS 32-bit words, 16.5 MiB) lives in
 // every GPU that loads this library until the process exits.  Every call
 // shares it, so calls that overlap on the GPU (concurrent streams, or several
 // host threads) race on it and must be serialised by the caller.  Each call
@@ -30,6 +30,7 @@ constexpr uint32_t GRID_NOALLOC_MAX_PHOTONS = 1u << 20;
 // keys, values and their ping-pong copies (4 words per photon) + the sort's scratch
 constexpr size_t GRID_NOALLOC_SCRATCH_WORDS =
     4ull * GRID_NOALLOC_MAX_PHOTONS + radix_scratch_words(GRID_NOALLOC_MAX_PHOTONS);
+static_assert(4 * GRID_NOALLOC_SCRATCH_WORDS / 1024 == 16900, "16.5 MiB, as srt.h says");
 
 static __device__ __align__(256) uint32_t g_grid_noalloc_scratch[GRID_NOALLOC_SCRATCH_WORDS];
 
@@ -40,7 +41,7 @@ namespace {
 __global__ void k_noalloc_ranges(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals, uint32_t n,
                                  uint32_t hash_bits, unsigned long long* __restrict__ keys_out,
                                  uint2* __restrict__ ranges, const uint32_t* __restrict__ sort_scratch) {
-    if (sort_scratch[RS_GAVE_UP] != 0u) return;  // the sort's bounded wait gave up (calls overlapped): empty ranges
+    if (sort_scratch[RS_GAVE_UP] != 0u) return;  // calls overlapped and the sort noticed: empty ranges, keys_out as it was
     uint32_t sentinel = 1u << hash_bits;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t h = keys[i];
