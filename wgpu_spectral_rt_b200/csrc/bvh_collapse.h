@@ -126,17 +126,18 @@ SRT_HD int collapse_expand(const TREE& tree, uint32_t ref, int width, uint32_t* 
 // (child, slot) score.  child_in[s]: the child in slot s, or -1.  Every child gets
 // a slot of its own whatever the scores are (a box without a centre scores NaN).
 SRT_HD void collapse_slots(int nc, const float (*d)[3], int* child_in) {
-    uint32_t placed = 0u;
+    uint32_t placed = 0u, taken = 0u;  // children with a slot, slots with a child
     for (int s = 0; s < 8; ++s) child_in[s] = -1;
     for (int it = 0; it < nc; ++it) {
         float bs = -3.4e38f;
         int bc = -1, bsl = -1;
         for (int c = 0; c < nc; ++c) {
             if ((placed >> c) & 1u) continue;
+            const float x = d[c][0], y = d[c][1], z = d[c][2];
+#pragma unroll
             for (int s = 0; s < 8; ++s) {
-                if (child_in[s] >= 0) continue;
-                const float sc = ((s & 1) ? d[c][0] : -d[c][0]) + ((s & 2) ? d[c][1] : -d[c][1]) +
-                                 ((s & 4) ? d[c][2] : -d[c][2]);
+                if ((taken >> s) & 1u) continue;
+                const float sc = ((s & 1) ? x : -x) + ((s & 2) ? y : -y) + ((s & 4) ? z : -z);
                 if (bc < 0 || sc > bs) {
                     bs = sc;
                     bc = c;
@@ -145,6 +146,7 @@ SRT_HD void collapse_slots(int nc, const float (*d)[3], int* child_in) {
             }
         }
         placed |= 1u << bc;
+        taken |= 1u << bsl;
         child_in[bsl] = bc;
     }
 }
