@@ -175,8 +175,15 @@ struct Bvh2Tree {  // the binary tree as collapse_expand reads it
     __device__ __forceinline__ uint32_t choice(uint32_t ref, int i) const { return choice_of(b, ref, i); }
 };
 
-__global__ void k_karras(const uint32_t* __restrict__ keys, int n, Bvh2 b) {
+// Also looks at the sort that ordered the codes: where it gave up, keys and
+// triangles may be anything, and nothing is built from them (ERR_WAIT_TIMEOUT).
+__global__ void k_karras(const uint32_t* __restrict__ keys, int n, Bvh2 b, const uint32_t* __restrict__ sort_scratch,
+                         uint32_t* __restrict__ err) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (sort_scratch[RS_GAVE_UP] != 0u) {
+        if (i == 0) atomicOr(err, ERR_WAIT_TIMEOUT);
+        return;
+    }
     if (i >= n - 1) return;
     int d = (delta(keys, n, i, i + 1) - delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
     int dmin = delta(keys, n, i, i - d);
@@ -205,9 +212,9 @@ __global__ void k_karras(const uint32_t* __restrict__ keys, int n, Bvh2 b) {
 }
 
 __global__ void k_refit(const TriSlot* __restrict__ flat, const uint32_t* __restrict__ sorted_tri, int n, Bvh2 b,
-                        int width, uint32_t leaf_max) {
+                        int width, uint32_t leaf_max, const uint32_t* __restrict__ err) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= n || (*err & ERR_WAIT_TIMEOUT)) return;
     TriSlot s = flat[sorted_tri[i]];
     float3 lo = f3(fminf(fminf(s.v0.x, s.v1.x), s.v2.x), fminf(fminf(s.v0.y, s.v1.y), s.v2.y),
                    fminf(fminf(s.v0.z, s.v1.z), s.v2.z));
@@ -896,7 +903,7 @@ __global__ void k_collapse(Bvh2 b, const uint2* __restrict__ qin, uint32_t n_in,
                            uint32_t tri_cap, const TriSlot* __restrict__ flat, const uint32_t* __restrict__ sorted_tri,
                            uint32_t* __restrict__ err, int width, uint32_t leaf_max, uint32_t open_above) {
     uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_in) return;
+    if (e >= n_in || (*(volatile uint32_t*)err & ERR_WAIT_TIMEOUT)) return;
     uint2 q = qin[e];
     uint32_t refs[8];
     int nc = 1;
@@ -1085,16 +1092,8 @@ cudaError_t build_bvh8(const BvhInputs& in, cudaStream_t st, BvhOutputs* out, st
             ++out->kernel_launches;
             uint32_t* sk;
             out->kernel_launches += sort_pairs(keys, vals, keys2, vals2, n, nullptr, 0, 30, scratch, st, &sk, &sv);
-            uint32_t gave_up = 0;
-            CK(cudaMemcpyAsync(&gave_up, scratch + RS_GAVE_UP, 4, cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-            if (gave_up) {  // sk and sv may hold anything
-                if (msg) *msg = "the sort's bounded wait gave up";
-                e = cudaErrorTimeout;
-                goto done;
-            }
             if (n > 1) {
-                k_karras<<<(n - 1 + B - 1) / B, B, 0, st>>>(sk, (int)n, b);
+                k_karras<<<(n - 1 + B - 1) / B, B, 0, st>>>(sk, (int)n, b, scratch, err);
                 ++out->kernel_launches;
             }
         } else {
@@ -1139,7 +1138,7 @@ cudaError_t build_bvh8(const BvhInputs& in, cudaStream_t st, BvhOutputs* out, st
         }
         const int width = in.width < 2 ? 2 : (in.width > 8 ? 8 : in.width);
         const uint32_t leaf_max = in.leaf_max < 1u ? 1u : (in.leaf_max > LEAF_MAX_LIMIT ? LEAF_MAX_LIMIT : in.leaf_max);
-        k_refit<<<grid, B, 0, st>>>(flat, sv, (int)n, b, width, leaf_max);
+        k_refit<<<grid, B, 0, st>>>(flat, sv, (int)n, b, width, leaf_max, err);
         ++out->kernel_launches;
         CK(cudaGetLastError());
         // collapse, level by level; node 0 is the root.  The recurrence is not
@@ -1182,6 +1181,11 @@ cudaError_t build_bvh8(const BvhInputs& in, cudaStream_t st, BvhOutputs* out, st
         CK(cudaMemcpyAsync(hc, counters, sizeof(hc), cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        if (herr & ERR_WAIT_TIMEOUT) {
+            if (msg) *msg = "the sort's bounded wait gave up";
+            e = cudaErrorTimeout;
+            goto done;
+        }
         if (herr != 0u || hc[1] != n) {
             if (msg) *msg = "BVH8 collapse produced an inconsistent tree";
             e = cudaErrorUnknown;

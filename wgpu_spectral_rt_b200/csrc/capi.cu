@@ -525,7 +525,6 @@ srt_status scene_build_impl(srt_ctx* c, const srt_scene_arrays* a,
         return fail(c, SRT_ERR_UNSUPPORTED, "BVH deeper than the traversal stack");
     launch_scatter_masks(s->bvh, s->inst, s->materials, s->bvh.scatter, st);
     CUDA_TRY(c, cudaGetLastError());
-    CUDA_TRY(c, cudaStreamSynchronize(st));
     s->n_tris = total;
     s->n_lights = a->n_lights;
     DevScene& d = s->dev;
