@@ -567,6 +567,7 @@ def main(argv=None):
     ms_max, paths_all = replica_reduce(ms, w * h * args.steps, dist, f"cuda:{local_rank}")
     value = paths_all / (ms_max * 1e-3) / 1e6
     photons_all = photons * args.steps * world
+    # rays answered: photon rays that cannot scatter and light samples that add zeros count, but are not traced
     rays_all = (st["rays_closest"] + st["rays_shadow"] + st["rays_photon"]) * world
 
     # ---- end to end through the C ABI with host buffers: the camera uniform goes
@@ -690,6 +691,8 @@ def main(argv=None):
                        "parallelism": f"replicas x{world}", "bvh_nodes": info["nodes"], "bvh_depth": info["depth"]},
             "mphotons_per_s": round(photons_all / (ms_max * 1e-3) / 1e6, 2),
             "mrays_per_s": round(rays_all / (ms_max * 1e-3) / 1e6, 2),
+            "mrays_counts": "rays answered; photon rays that cannot scatter and light samples behind the surface are "
+                            "not traced",
             "rays_per_path": round((st["rays_closest"] + st["rays_shadow"]) / max(1, st["paths"]), 3),
             "photons_stored_per_frame": round(st["photons_stored"] / max(1, st["frames"])),
             "e2e": {"value": round(e2e_value, 3), "unit": "Mpaths/s", "h2d_bytes_per_step": 272,

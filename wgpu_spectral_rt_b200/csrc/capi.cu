@@ -38,7 +38,7 @@ struct srt_ctx {
     // One workspace kept between calls that bring their own data
     // (srt_trace_rays), up to WORK_KEEP bytes; a call takes it out while it runs,
     // so that a second thread's call finds none and allocates its own (250k ray
-    // queries from host arrays 2.55 -> 1.2 ms).
+    // queries from host arrays 2.5-2.8 -> 1.2-1.6 ms, with the host's copy speed).
     static constexpr size_t WORK_KEEP = 64ull << 20;
     struct Work {
         void* p = nullptr;

@@ -2,8 +2,8 @@
 //
 // One kernel per 8-bit digit pass, after one that counts the digits of every
 // pass (k_rs_count, or the kernel that makes the keys: rs_count_key).  A pass
-// reads its tile once: it ranks the tile's items among equal digits (warp
-// match_any per 32-item round, per-warp counters in shared memory), learns how
+// reads its tile once: it ranks the tile's items among equal digits (a ballot per
+// bit of the digit per 32-item round, per-warp counters in shared memory), learns how
 // many of each digit the tiles before it hold by decoupled look-back (Merrill
 // and Garland, "Single-pass Parallel Prefix Scan with Decoupled Look-back",
 // 2016; one thread per digit), and writes the items, ordered by digit in shared
